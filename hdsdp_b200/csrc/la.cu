@@ -381,7 +381,32 @@ __global__ void __launch_bounds__(GT) gemm_grouped_kernel(const GemmP *__restric
     if ((int) blockIdx.x * BM >= p.M || (int) blockIdx.y * BN >= p.N) return;
     gemm_tile(p, blockIdx.x, blockIdx.y);
 }
+
+// GEMM z of a strided group: operands at A + z sa, B + z sb, C + z sc; with kstep set, the
+// K range [z kstep, (z + 1) kstep) of one product (sa and sb then move along K)
+__global__ void __launch_bounds__(GT) gemm_strided_kernel(GemmP p, long sa, long sb, long sc, int kstep) {
+    const int z = blockIdx.z;
+    p.A += z * sa;
+    p.B += z * sb;
+    p.C += z * sc;
+    if (kstep > 0) p.K = min(kstep, p.K - z * kstep);
+    gemm_tile(p, blockIdx.x, blockIdx.y);
+}
 }  // namespace
+
+void gemm_strided(cudaStream_t s, const GemmDesc &d, long sa, long sb, long sc, int count, int kstep) {
+    if (count <= 0 || d.M <= 0 || d.N <= 0) return;
+    for (int z0 = 0; z0 < count; z0 += 65535) {
+        GemmP p = d;
+        p.A += z0 * sa;
+        p.B += z0 * sb;
+        p.C += z0 * sc;
+        if (kstep > 0) p.K -= z0 * kstep;
+        dim3 grid((d.M + BM - 1) / BM, (d.N + BN - 1) / BN, std::min(65535, count - z0));
+        gemm_strided_kernel<<<hb::counted(grid), GT, 0, s>>>(p, sa, sb, sc, kstep);
+        HB_CUDA(cudaGetLastError());
+    }
+}
 
 void gemm_grouped(cudaStream_t s, const GemmDesc *d_desc, int count, int maxM, int maxN) {
     if (count <= 0 || maxM <= 0 || maxN <= 0) return;

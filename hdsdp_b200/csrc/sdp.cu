@@ -34,6 +34,9 @@ T *upload_vec(const std::vector<T> &h, cudaStream_t s) {
 // of rows r and c. Launched on a grid of (row blocks, columns c); rows below c return.
 __device__ __forceinline__ long long r1map_pos(int n, int r, int c) { return (long long) (2LL * n - c - 1) * c / 2 + r; }
 
+// Scratch for the products with the dense coefficient matrices (bytes for each of the two sets).
+constexpr size_t kDrScratch = 256u << 20;
+
 // Lists longer than this leave the sliced layout for the warp-per-position one.
 constexpr int kLongList = 64;
 
@@ -239,15 +242,71 @@ __global__ void r1d_weights_kernel(int k, const int *id, const double *sign, con
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < k; a += gridDim.x * blockDim.x) d[a] = dA * sign[a] * w[id[a]];
 }
 
-__global__ void axpy_mat_devscale_kernel(int n, const double *A, long lda, const double *w, int j, double dA,
-                                         double *S, long lds) {
-    const double a = dA * w[j];
-    if (a == 0.0) return;
-    const long total = (long) n * n;
+// ---- dense coefficient matrices (class DR): all of them in one launch each --------------
+// These kernels stream the slab of ndr matrices (8 ld n ndr bytes) once. One launch per matrix
+// and per inner product was bound by launches: order 80 with 40 matrices took 7,600 of them and
+// 35.2 ms for two dual-scaling iterations, now about 240 and 3.4 ms.
+
+// S += dA sum_i w[id[i]] A_i, in the order of i; one thread per entry, so the loads of a warp
+// are contiguous in every matrix
+__global__ void dr_axpy_kernel(int n, int ndr, const int *__restrict__ id, const double *__restrict__ A, long lda,
+                               const double *__restrict__ w, double dA, double *S, long lds) {
+    const long total = (long) n * n, step = lda * n;
     for (long idx = blockIdx.x * (long) blockDim.x + threadIdx.x; idx < total; idx += (long) gridDim.x * blockDim.x) {
-        int r = (int) (idx % n), c = (int) (idx / n);
-        S[(size_t) r + (size_t) c * lds] += a * A[(size_t) r + (size_t) c * lda];
+        const int r = (int) (idx % n), c = (int) (idx / n);
+        const double *a = A + (size_t) r + (size_t) c * lda;
+        double acc = S[(size_t) r + (size_t) c * lds];
+#pragma unroll 8
+        for (int i = 0; i < ndr; ++i) acc += dA * w[id[i]] * a[i * step];
+        S[(size_t) r + (size_t) c * lds] = acc;
     }
+}
+
+// part[j gridDim.x + b] = block b's share of <A_j, Z> (columns b, b + gridDim.x, ...), or the
+// whole of it into out[id[j]] when one block takes a matrix
+__global__ void dr_inner_kernel(int n, const int *__restrict__ id, const double *__restrict__ A, long lda,
+                                const double *__restrict__ Z, long ldz, double *part, double *out) {
+    __shared__ double red[32];
+    const int j = blockIdx.y;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const double *a = A + (size_t) j * lda * n;
+    double acc = 0.0;
+    for (int c = blockIdx.x * nw + warp; c < n; c += gridDim.x * nw) {
+        const double *ac = a + (size_t) c * lda, *zc = Z + (size_t) c * ldz;
+        for (int r = lane; r < n; r += 32) acc += ac[r] * zc[r];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) red[warp] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int q = 0; q < nw; ++q) t += red[q];
+        if (gridDim.x == 1) out[id[j]] = t;
+        else part[(size_t) j * gridDim.x + blockIdx.x] = t;
+    }
+}
+
+// out[id[j]] = sum_b part[j nb + b] in order
+__global__ void dr_sum_kernel(int ndr, int nb, const int *__restrict__ id, const double *__restrict__ part, double *out) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= ndr) return;
+    double t = 0.0;
+    for (int b = 0; b < nb; ++b) t += part[(size_t) j * nb + b];
+    out[id[j]] = t;
+}
+
+// M(id_i, id_j) = sum_s part_s(j, i - i0), in order, for the chunk's columns i and every j <= i
+// (part_s: ndr x nc, the inner products over one range of the entries)
+__global__ void dr_schur_kernel(int ndr, int i0, int nc, int ns, const int *__restrict__ id,
+                                const double *__restrict__ part, double *M, long ldm) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x, i = i0 + blockIdx.y;
+    if (j > i) return;
+    double t = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < ns; ++q) t += part[(size_t) q * ndr * nc + (size_t) (i - i0) * ndr + j];
+    const int a = id[i], b = id[j];
+    M[(size_t) max(a, b) + (size_t) min(a, b) * ldm] = t;
 }
 
 // ---- Schur pair kernels -------------------------------------------------------------
@@ -679,7 +738,7 @@ void SdpDevice::upload(int n_, int m_, const HostCoeff &C, const std::vector<Hos
             r1did.push_back(j);
             r1dsg.push_back(a.sign);
         } else if (a.cls == CLS_DR) {
-            dr_id.push_back(j);
+            dr_host_id.push_back(j);
         }
     }
 
@@ -721,21 +780,38 @@ void SdpDevice::upload(int n_, int m_, const HostCoeff &C, const std::vector<Hos
     if (nr1d > 0) HB_CUDA(hb::cmalloc(&Vt, sizeof(double) * ld * nr1d));
     if (nr1s > 0 && nsp > 0) HB_CUDA(hb::cmalloc(&Vs, sizeof(double) * ld * nr1s));
 
-    ndr = (int) dr_id.size();
-    for (int i = 0; i < ndr; ++i) {
-        const HostCoeff &c = A[dr_id[i]];
-        double *mat = nullptr;
-        HB_CUDA(hb::cmalloc(&mat, sizeof(double) * ld * n));
-        HB_CUDA(cudaMemsetAsync(mat, 0, sizeof(double) * ld * n, s));
-        int *dr = upload_vec(c.r, s), *dc = upload_vec(c.c, s);
-        double *dv = upload_vec(c.v, s);
-        if (!c.r.empty())
-            scatter_sym_kernel<<<hb::counted(grid1((long) c.r.size())), 256, 0, s>>>((int) c.r.size(), dr, dc, dv, mat, ld);
-        HB_CUDA(cudaStreamSynchronize(s));
-        hb::cache_free(dr);
-        hb::cache_free(dc);
-        hb::cache_free(dv);
-        dr_mat.push_back(mat);
+    ndr = (int) dr_host_id.size();
+    if (ndr > 0) {
+        const size_t mat = (size_t) ld * n;
+        dr_id = upload_vec(dr_host_id, s);
+        HB_CUDA(hb::cmalloc(&dr_slab, sizeof(double) * mat * ndr));
+        HB_CUDA(cudaMemsetAsync(dr_slab, 0, sizeof(double) * mat * ndr, s));
+        for (int i = 0; i < ndr; ++i) {
+            const HostCoeff &c = A[dr_host_id[i]];
+            int *dr = upload_vec(c.r, s), *dc = upload_vec(c.c, s);
+            double *dv = upload_vec(c.v, s);
+            if (!c.r.empty())
+                scatter_sym_kernel<<<hb::counted(grid1((long) c.r.size())), 256, 0, s>>>((int) c.r.size(), dr, dc, dv,
+                                                                                        dr_slab + i * mat, ld);
+            HB_CUDA(cudaStreamSynchronize(s));
+            hb::cache_free(dr);
+            hb::cache_free(dc);
+            hb::cache_free(dv);
+        }
+        // as many products at a time as fit kDrScratch; the inner products split along the
+        // entries until their 64 x 64 tiles give the SMs two blocks each (at least 128 entries)
+        dr_chunk = (int) std::max<size_t>(1, std::min<size_t>(ndr, kDrScratch / (sizeof(double) * mat)));
+        const long tiles = (long) ((ndr + 63) / 64) * ((dr_chunk + 63) / 64);
+        const long want = std::max(1L, 296 / tiles);
+        const long entries = ld * n;
+        dr_kstep = (int) std::max(128L, ((entries + want - 1) / want + 15) / 16 * 16);
+        dr_split = (int) ((entries + dr_kstep - 1) / dr_kstep);
+        dr_dsplit = (int) std::max(1, std::min((n + 7) / 8, 296 / ndr));
+        HB_CUDA(hb::cmalloc(&dr_t1, sizeof(double) * mat * dr_chunk));
+        HB_CUDA(hb::cmalloc(&dr_t2, sizeof(double) * mat * dr_chunk));
+        HB_CUDA(cudaMemsetAsync(dr_t2, 0, sizeof(double) * mat * dr_chunk, s));   // rows beyond n stay zero
+        HB_CUDA(hb::cmalloc(&dr_part, sizeof(double) * std::max((size_t) dr_split * ndr * dr_chunk,
+                                                                (size_t) ndr * dr_dsplit)));
     }
 
     // S-assembly gather map
@@ -901,8 +977,11 @@ void SdpDevice::release() {
     f(sp_id); f(sp_ptr); f(sp_r); f(sp_c); f(sp_v);
     f(r1s_id); f(r1s_ptr); f(r1s_p); f(r1s_a); f(r1s_sign);
     f(r1d_id); f(r1d_sign); f(A1); f(G); f(V); f(Vt); f(Vs);
-    for (double *p : dr_mat) f(p);
-    dr_mat.clear();
+    f(dr_id); f(dr_slab); f(dr_t1); f(dr_t2); f(dr_part);
+    dr_id = nullptr;
+    dr_slab = dr_t1 = dr_t2 = dr_part = nullptr;
+    dr_host_id.clear();
+    ndr = 0;
     f(pos_r); f(pos_c); f(pos_ptr); f(ent_j); f(ent_v);
     f(pos2_r); f(pos2_c); f(pos2_cnt); f(pos2_ptr); f(ent2_j); f(ent2_v);
     pos2_r = pos2_c = pos2_cnt = ent2_j = nullptr;
@@ -944,8 +1023,9 @@ void SdpDevice::assemble(double dC, double dA, const double *d_wvec, double dEye
             scale_columns(s, n, nr1d, A1, ld, d_w, V, ld);
             gemm(s, n, n, nr1d, 1.0, V, ld, 0, A1, ld, 1, 1.0, S, ldS, 0);
         }
-        for (int i = 0; i < ndr; ++i)
-            axpy_mat_devscale_kernel<<<hb::counted(grid1((long) n * n)), 256, 0, s>>>(n, dr_mat[i], ld, d_wvec, dr_id[i], dA, S, ldS);
+        if (ndr > 0)
+            dr_axpy_kernel<<<hb::counted((int) std::min<long>(((long) n * n + 63) / 64, 148L * 32)), 64, 0, s>>>(
+                n, ndr, dr_id, dr_slab, ld, d_wvec, dA, S, ldS);
     }
     HB_CUDA(cudaGetLastError());
 }
@@ -1018,14 +1098,35 @@ void SdpDevice::schur_matrix(const double *W, long ldW, double *M, long ldM, con
         schur_r1_sp_kernel<<<hb::counted(g3), blk, 0, s>>>(nr1s, r1s_id, r1s_sign, Vs, ld, nsp, sp_id, sp_ptr, sp_r, sp_c, sp_v,
                                               M, ldM);
     }
-    for (int i = 0; i < ndr; ++i) {
-        // B_i = W A_i W, then M_ij = <A_j, B_i>
-        gemm(s, n, n, n, 1.0, dr_mat[i], ld, 0, W, ldW, 0, 0.0, T1, ld, 0);
-        gemm(s, n, n, n, 1.0, W, ldW, 0, T1, ld, 0, 0.0, T2, ld, 0);
-        symmetrize_avg(s, n, T2, ld);
-        inner_all(T2, ld, vecbuf);
-        scatter_row_kernel<<<hb::counted(grid1(m)), 256, 0, s>>>(m, dr_id[i], vecbuf, M, ldM);
+    // dense coefficients, a chunk at a time: B_i = W A_i W as one product with the slab and one
+    // strided group, then M_ij = <A_j, B_i> as the products of the slab's columns with the
+    // chunk's, split along the entries
+    for (int i0 = 0; i0 < ndr; i0 += dr_chunk) {
+        const int nc = std::min(dr_chunk, ndr - i0);
+        const long mat = ld * n;
+        gemm(s, n, n * nc, n, 1.0, W, ldW, 0, dr_slab + i0 * mat, ld, 0, 0.0, dr_t1, ld, 0);
+        gemm_strided(s, GemmDesc{n, n, n, 1.0, 0.0, dr_t1, ld, 0, W, ldW, 0, dr_t2, ld, 0, nullptr}, mat, 0, mat, nc);
+        for (int i = 0; i < nc && ndr < m; ++i) {
+            // the products with the other classes
+            double *B = dr_t2 + i * mat;
+            symmetrize_avg(s, n, B, ld);
+            inner_all(B, ld, vecbuf);
+            scatter_row_kernel<<<hb::counted(grid1(m)), 256, 0, s>>>(m, dr_host_id[i0 + i], vecbuf, M, ldM);
+        }
+        gemm_strided(s, GemmDesc{ndr, nc, (int) mat, 1.0, 0.0, dr_slab, mat, 1, dr_t2, mat, 0, dr_part, ndr, 0, nullptr},
+                     dr_kstep, dr_kstep, (long) ndr * nc, dr_split, dr_kstep);
+        const dim3 g((i0 + nc + 63) / 64, nc);
+        dr_schur_kernel<<<hb::counted(g), 64, 0, s>>>(ndr, i0, nc, dr_split, dr_id, dr_part, M, ldM);
     }
+    HB_CUDA(cudaGetLastError());
+}
+
+void SdpDevice::dr_inner(const double *Z, long ldZ, double *out) {
+    if (ndr == 0) return;
+    const dim3 grid(dr_dsplit, ndr);
+    dr_inner_kernel<<<hb::counted(grid), 256, 0, stream>>>(n, dr_id, dr_slab, ld, Z, ldZ, dr_part, out);
+    if (dr_dsplit > 1)
+        dr_sum_kernel<<<hb::counted((ndr + 63) / 64), 64, 0, stream>>>(ndr, dr_dsplit, dr_id, dr_part, out);
     HB_CUDA(cudaGetLastError());
 }
 
@@ -1060,7 +1161,7 @@ void SdpDevice::inner_all(const double *Z, long ldZ, double *out, bool reuse_v) 
         const double *Vz = reuse_v ? V : Vt;
         coldot_pair_kernel<<<hb::counted((nr1d * 32 + 255) / 256), 256, 0, s>>>(n, nr1d, r1d_id, r1d_sign, A1, ld, Vz, ld, out);
     }
-    for (int i = 0; i < ndr; ++i) frob_dot(s, n, dr_mat[i], ld, Z, ldZ, out + dr_id[i]);
+    dr_inner(Z, ldZ, out);
     HB_CUDA(cudaGetLastError());
 }
 
@@ -1093,9 +1194,9 @@ void SdpDevice::inner_all_sq(const double *W, long ldW, double *out, bool reuse_
         const double *Vw = reuse_v ? V : Vt;
         coldot_pair_kernel<<<hb::counted((nr1d * 32 + 255) / 256), 256, 0, s>>>(n, nr1d, r1d_id, r1d_sign, Vw, ld, Vw, ld, out);
     }
-    for (int i = 0; i < ndr; ++i) {
-        gemm(s, n, n, n, 1.0, dr_mat[i], ld, 0, W, ldW, 0, 0.0, T1, ld, 0);
-        frob_dot(s, n, T1, ld, W, ldW, out + dr_id[i]);
+    if (ndr > 0) {
+        gemm(s, n, n, n, 1.0, W, ldW, 0, W, ldW, 0, 0.0, T1, ld, 0);   // W^2
+        dr_inner(T1, ld, out);
     }
     HB_CUDA(cudaGetLastError());
 }

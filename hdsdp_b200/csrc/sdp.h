@@ -61,10 +61,18 @@ struct SdpDevice {
     int *r1d_id = nullptr;
     double *r1d_sign = nullptr;
     double *A1 = nullptr;
-    // DR class: full n x n matrices
+    // DR class: full n x n matrices one after the other in one slab (matrix i at dr_slab +
+    // i ld n, so the slab is also an n x (n ndr) matrix), rows beyond n zero
     int ndr = 0;
-    std::vector<int> dr_id;
-    std::vector<double *> dr_mat;
+    int *dr_id = nullptr;
+    double *dr_slab = nullptr;
+    // scratch of its products: W A_i and W A_i W of dr_chunk matrices at a time, the partial
+    // sums of their inner products with the slab (dr_split of them along n ld)
+    int dr_chunk = 0, dr_split = 0, dr_kstep = 0, dr_dsplit = 0;
+    std::vector<int> dr_host_id;
+    double *dr_t1 = nullptr, *dr_t2 = nullptr, *dr_part = nullptr;
+    // out[id_j] = <A_j, Z> over the DR class
+    void dr_inner(const double *Z, long ldZ, double *out);
     // S assembly gather map over SP and R1S lower entries
     int npos = 0;
     int *pos_r = nullptr, *pos_c = nullptr, *pos_ptr = nullptr, *ent_j = nullptr;
