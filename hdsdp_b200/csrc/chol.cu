@@ -91,145 +91,152 @@ __device__ __forceinline__ void dmma_c(double &d0, double &d1, double a, double 
 
 
 // ---------------------------------------------------------------------------------
-// Diagonal-block factorisation: four 16-column sub-panels. Warp 0 factors and inverts
-// each 16 x 16 pivot block in registers; the panel below, the trailing update and the
-// off-diagonal blocks of the 64 x 64 inverse are DMMA products in shared memory with
-// the other warps.
+// Diagonal-block factorisation: eight 8-column sweeps over the 64 x 64 block T stacked on the
+// identity. The same elimination that turns T into L turns the identity below it into
+// E = L^-T, so the inverse costs no pass of its own.
+//
+// What bounds it is the chain of 64 pivots, each a reciprocal square root (50 cycles), a
+// product and a fused multiply-add (8.5 each). So warp 0 does nothing but the 8 x 8 pivot
+// blocks, every lane factoring the block for itself in registers, without shuffles or shared
+// memory between the pivots. Warps 1-7 keep one 8-row block each in DMMA accumulators for the
+// whole factorisation (warp j the block row T_j until sweep j - 1, then E_(j-1), which comes to
+// life with that sweep) and bring it up to date while warp 0 is in the next sweep. A block with
+// its update by the previous panel takes 7.3 us (13,000 cycles, of which 740 a
+// sweep are warp 0's arithmetic); 16.3 us with 16-column sweeps by shuffles and a separate
+// inverse. Order 1000: 0.394 -> 0.235 ms, with K = L^-1 0.408 -> 0.290 ms.
 // ---------------------------------------------------------------------------------
-constexpr unsigned FULL = 0xffffffffu;
 
-// Factor T[off.., off..] (16 x 16, lower, pitch TP) in place and write its inverse to
-// X[off.., off..]. Executed by one whole warp with two lane roles: lane r < 16 holds row
-// r of the block, lane 16 + k holds column k of the inverse (starting as e_k). For each
-// column c one set of broadcasts of L(q, c), q > c, drives both the trailing update
-// A(r, q) -= L(r, c) L(q, c) and the forward elimination X(q, k) -= L(q, c) X(c, k):
-// the two are the same instruction, v[q] -= v[c] L(q, c), on every lane (a lane of the
-// second role is never masked by the row test). The broadcasts of a column are issued
-// before their uses so that their latencies overlap.
-__device__ __forceinline__ bool warp_chol_inv16(double *T, double *X, int off, int lane) {
-    const bool row_role = lane < 16;
-    double v[16];
+// c += -(A B^T) over 64 columns for operand fragments na = -A and the 8-row block B in shared
+// memory (pitch TP), two chains of products
+__device__ __forceinline__ void mma8_64(double (&c)[2], const double (&na)[16], const double *B) {
+    const int at = ((threadIdx.x & 31) >> 2) + (threadIdx.x & 3) * TP;
+    double b[16], d[2] = {};
 #pragma unroll
-    for (int q = 0; q < 16; ++q)
-        v[q] = row_role ? ((q <= lane) ? T[(off + lane) + (off + q) * TP] : 0.0) : ((q == lane - 16) ? 1.0 : 0.0);
-    // one reciprocal square root per column: L_cc = p rsqrt(p), the column below scales
-    // by rsqrt(p), and so does row c of the inverse. The pivot of column c + 1 only
-    // needs L(c + 1, c), so it is formed first and its reciprocal square root runs
-    // while the rest of column c is applied.
-    double p = __shfl_sync(FULL, v[0], 0);
-    bool bad = !(p > 0.0);
-    double rs = rsqrt(p);
-    // fixed trip counts keep v[] and lq[] in registers (the loops unroll completely)
+    for (int k = 0; k < 16; ++k) b[k] = B[at + 4 * k * TP];
 #pragma unroll
-    for (int c = 0; c < 16; ++c) {
-        v[c] = (lane == c) ? p * rs : v[c] * rs;
-        double pn = 1.0, rn = 1.0;
-        if (c + 1 < 16) {
-            // lane c + 1 holds L(c + 1, c) itself: it forms the next pivot without waiting
-            // for the broadcast that the other lanes' update of column c + 1 needs (the same
-            // fused multiply-add, so the same value as that update gives)
-            const double own = v[c + 1] - v[c] * v[c];
-            pn = __shfl_sync(FULL, own, c + 1);
-            const double l1 = __shfl_sync(FULL, v[c], c + 1);
-            if (lane >= c + 1) v[c + 1] -= v[c] * l1;
-            if (!(pn > 0.0)) bad = true;
-            rn = rsqrt(pn);
-        }
-        double lq[16];
-#pragma unroll
-        for (int q = c + 2; q < 16; ++q) lq[q] = __shfl_sync(FULL, v[c], q);
-#pragma unroll
-        for (int q = c + 2; q < 16; ++q)
-            if (lane >= q) v[q] -= v[c] * lq[q];
-        p = pn;
-        rs = rn;
+    for (int k = 0; k < 16; k += 2) {
+        dmma_c(c[0], c[1], na[k], b[k]);
+        dmma_c(d[0], d[1], na[k + 1], b[k + 1]);
     }
-    if (row_role) {
-#pragma unroll
-        for (int q = 0; q < 16; ++q)
-            if (q <= lane) T[(off + lane) + (off + q) * TP] = v[q];
-    } else {
-        const int k = lane - 16;
-#pragma unroll
-        for (int q = 0; q < 16; ++q)
-            if (q >= k) X[(off + q) + (off + k) * TP] = v[q];
-    }
-    return !bad;
+    c[0] += d[0];
+    c[1] += d[1];
 }
 
-// C (rows x cols, multiples of 8) = / += alpha * A (rows x K) * op(B), K a multiple of 4,
-// in shared memory (pitch TP) on the DMMA path; 8 x 8 tiles dealt to the warps starting
-// at warp `w0`. A(r, k) = Ab[r + k*TP]; op(B)(k, c) = bt ? Bb[c + k*TP] : Bb[k + c*TP].
-// With lower set, tiles strictly above the diagonal are skipped.
-// With nwarp set, only warps w0 .. w0 + nwarp - 1 take part (and all of them must call).
-__device__ __forceinline__ void smem_mma(double *Cb, const double *Ab, const double *Bb, int bt, int rows, int cols,
-                                         int K, double alpha, bool accumulate, bool lower, int w0 = 0,
-                                         int nwarp = 0) {
-    const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) - w0;
-    const int nw = nwarp ? nwarp : (int) (blockDim.x >> 5);
-    const int tr = rows >> 3, ntile = tr * (cols >> 3);
-    for (int t = w; t < ntile; t += nw) {
-        const int ti = t % tr, tj = t / tr;
-        if (lower && ti < tj) continue;
-        double c0 = 0.0, c1 = 0.0;
-        for (int k0 = 0; k0 < K; k0 += 4) {
-            const int kk = k0 + (lane & 3);
-            const double av = Ab[(ti * 8 + (lane >> 2)) + kk * TP];
-            const int cc = tj * 8 + (lane >> 2);
-            const double bv = bt ? Bb[cc + kk * TP] : Bb[kk + cc * TP];
-            dmma_c(c0, c1, av, bv);
+// 1 / sqrt(p) for positive normal p: the hardware's approximation (rsqrt.approx, about 20 bits)
+// and one step of Householder's third-order iteration y (1 + e/2 + 3 e^2 / 8), e = 1 - p y^2.
+// Straight-line code, so that the other work of a column is scheduled under it (rsqrt() ends in
+// a branch for its special cases); within 2 ulp of rsqrt() over the normal range.
+__device__ __forceinline__ double rsqrt_normal(double p) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(p));
+    const double e = fma(-(p * y), y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// The lower part of the 8 x 8 block d (pitch TP, 16-byte aligned) in every lane's registers.
+__device__ __forceinline__ void load8(const double *d, double (&a)[8][8]) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int r = c & ~1; r < 8; r += 2) {
+            const double2 v = *reinterpret_cast<const double2 *>(d + r + c * TP);
+            a[r][c] = v.x;
+            a[r + 1][c] = v.y;
         }
-        const int r = ti * 8 + (lane >> 2), c = tj * 8 + (lane & 3) * 2;
-        if (accumulate) {
-            Cb[r + c * TP] += alpha * c0;
-            Cb[r + (c + 1) * TP] += alpha * c1;
-        } else {
-            Cb[r + c * TP] = alpha * c0;
-            Cb[r + (c + 1) * TP] = alpha * c1;
+}
+
+// One sweep by one warp over the 8 x 8 pivot block a: every lane factors it for itself and
+// carries its row x along, x <- x L^-T. Two columns at a time: with the 2 x 2 pivot p11, p21,
+// p22 and its determinant, 1/L_22 = sqrt(p11) / sqrt(det), so both reciprocal square roots run
+// at once (46 cycles of latency a column instead of 66). False when a pivot is not a positive number whose
+// products with its neighbour stay in the normal range (sweep8_any then takes the block).
+__device__ __forceinline__ bool sweep8(double (&a)[8][8], double (&x)[8]) {
+    bool fine = true;
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+        const double p11 = a[c][c], p21 = a[c + 1][c], p22 = a[c + 1][c + 1];
+        const double det = fma(p11, p22, -(p21 * p21));
+        // high words: p11 and p22 between 2^-500 and 2^500, det at least 2^-1020
+        fine = fine && (unsigned) __double2hiint(p11) - 0x20b00000u < 0x3e800000u &&
+               (unsigned) __double2hiint(p22) - 0x20b00000u < 0x3e800000u &&
+               (unsigned) __double2hiint(det) - 0x00300000u < 0x7fb00000u;
+        const double r1 = rsqrt_normal(p11), rd = rsqrt_normal(det);
+        const double l21 = p21 * r1, r2 = rd * (p11 * r1);
+        x[c] *= r1;
+        x[c + 1] = (x[c + 1] - x[c] * l21) * r2;
+#pragma unroll
+        for (int r = c + 2; r < 8; ++r) {
+            a[r][c] *= r1;
+            a[r][c + 1] = (a[r][c + 1] - a[r][c] * l21) * r2;
+        }
+#pragma unroll
+        for (int q = c + 2; q < 8; ++q) {
+#pragma unroll
+            for (int r = q; r < 8; ++r) a[r][q] = a[r][q] - a[r][c] * a[q][c] - a[r][c + 1] * a[q][c + 1];
+            x[q] = x[q] - x[c] * a[q][c] - x[c + 1] * a[q][c + 1];
         }
     }
+    return fine;
+}
+
+// The same for any pivots, a column at a time with rsqrt(); returns the first column whose
+// pivot is not positive, or 8.
+__device__ __noinline__ int sweep8_any(const double *d, double (&x)[8]) {
+    double a[8][8];
+    load8(d, a);
+    int bad = 8;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const double p = a[c][c];
+        if (!(p > 0.0) && bad == 8) bad = c;
+        const double rs = rsqrt(p);
+        x[c] *= rs;
+#pragma unroll
+        for (int r = c + 1; r < 8; ++r) a[r][c] *= rs;
+#pragma unroll
+        for (int q = c + 1; q < 8; ++q) {
+#pragma unroll
+            for (int r = q; r < 8; ++r) a[r][q] -= a[r][c] * a[q][c];
+            x[q] -= x[c] * a[q][c];
+        }
+    }
+    return bad;
 }
 
 // Shared-memory regions of the factorisation kernel (64 x TP doubles each): tile
 // products use regions 0 and 1; the diagonal-block factorisation keeps its block in
-// region 3, the previous panel's rows in region 2 and the inverse in region 1.
+// region 3, the previous panel's rows in region 2 and its exchange buffers in region 1.
 constexpr int R_X = 1, R_P = 2, R_T = 3;
-__device__ __forceinline__ double *region(double *sm, int r) { return sm + (size_t) r * 64 * TP; }
+// (addressed through the array itself, not a pointer argument, so that every access is known to
+// be to shared memory)
+extern __shared__ double dyn_smem[];
+__device__ __forceinline__ double *region(int r) { return dyn_smem + r * 64 * TP; }
 
-// Block row i of the inverse of the 64 x 64 diagonal block, off the diagonal:
-// X_ij = -X_ii sum_{k=j}^{i-1} L_ik X_kj for j < i (16 x 16 blocks), by warps
-// w0 .. w0 + nwarp - 1 (nwarp 0: all warps); `bar` synchronises exactly those warps
-// between the two products. Scratch: rows 0-15, columns 16-63 of P.
-template <typename Bar>
-__device__ __forceinline__ void inverse_block_row(const double *T, double *X, double *P, int i, int w0, int nwarp,
-                                                  Bar bar) {
-    for (int j = 0; j < i; ++j)
-        smem_mma(P + 16 * (j + 1) * TP, T + 16 * i + 16 * j * TP, X + 16 * j + 16 * j * TP, 0, 16, 16, 16 * (i - j),
-                 1.0, false, false, w0, nwarp);
-    bar();
-    for (int j = 0; j < i; ++j)
-        smem_mma(X + 16 * i + 16 * j * TP, X + 16 * i + 16 * i * TP, P + 16 * (j + 1) * TP, 0, 16, 16, 16, -1.0,
-                 false, false, w0, nwarp);
-}
-
-// Factor the nb x nb diagonal block at (j0, j0) and write its inverse to Dinv (64
-// columns, zero padded). The block is first updated in shared memory by the previous
-// panel's rows, A_jj -= P P^T, when they are given: `staged` (block and rows already in
-// regions 3 and 2, copies possibly still in flight) or Pp (nb x 64 rows, pitch ldp,
-// staged here). Executed by one block. Returns false (and sets *info) on a failed
-// pivot. The strictly upper part of the diagonal block in L holds zeros (copy_lower_k
-// and every later write keep it so), which lets whole column segments be staged.
-__device__ bool potf2_dev(double *L, long ld, int j0, int nb, double *Dinv, long ldd, int *info, double *sm,
-                          const double *Pp = nullptr, long ldp = 0, bool staged = false) {
-    double *T = region(sm, R_T), *X = region(sm, R_X), *P = region(sm, R_P);
+// Factor the nb x nb diagonal block at (j0, j0) and write its inverse to Dinv (lower part; the
+// rest of Dinv is zero from the allocation on). With `staged` the block and the previous
+// panel's 64 rows P are in regions 3 and 2 (copies possibly still in flight) and the block is
+// first updated, A_jj -= P P^T. Executed by one block of 256 threads. Returns false (and sets
+// *info) on a failed pivot. The strictly upper part of the diagonal block in L holds zeros
+// (copy_lower_k and every later write keep it so), which lets whole column segments be staged.
+//
+// Sweep s turns column block s. Warp 0 factors the pivot block and publishes E_ss = L_ss^-T
+// (barrier 1). Every row block multiplies its tile of column s by E_ss; those of T are published
+// as operands (barrier 2, without warp 0), and each row block is updated with them. The owner
+// of row s + 1 updates the next pivot block before all else and hands it to warp 0 (barrier 3).
+__device__ bool potf2_dev(double *L, long ld, int j0, int nb, double *Dinv, long ldd, int *info, bool staged = false) {
+    double *T = region(R_T), *P = region(R_P);
+    // E_ss and L_ss of alternate sweeps (8 columns, pitch PU), the published tiles of column s
+    // (pitch PB). An 8 x 8 tile held as accumulators serves as a DMMA operand as it is: register h
+    // of a lane is column 2 (lane % 4) + h, so product h takes those columns of both operands. The
+    // pitches keep the reads of the other operand free of bank conflicts in that order.
+    constexpr int PU = 72, PB = 66;
+    double *U = region(R_X), *Ls = U + 16 * PU, *B = U + 32 * PU;
     __shared__ int fail;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double *Ljj = L + (size_t) j0 + (size_t) j0 * ld;
-    if (!staged) {
-        stage_tile(T, Ljj, ld, nb, nb, 64);
-        if (Pp) stage_tile(P, Pp, ldp, nb, 64, 64);
-    }
-    for (int idx = tid; idx < 64 * 64; idx += blockDim.x) X[(idx & 63) + (idx >> 6) * TP] = 0.0;
+    double *Dj = Dinv + j0;
+    const bool vec = ((((size_t) Dj) & 15) == 0) && ((ldd & 1) == 0);   // two rows of Dinv a store
+    if (!staged) stage_tile(T, Ljj, ld, nb, nb, 64);
     cpa_wait_all();
     if (tid == 0) fail = 0;
     for (int r = nb + tid; r < 64; r += blockDim.x) T[r + r * TP] = 1.0;  // pad with the identity
@@ -237,98 +244,145 @@ __device__ bool potf2_dev(double *L, long ld, int j0, int nb, double *Dinv, long
     const int sb = 4096 + (j0 / 64) * 32;
     (void) sb;
     CHOL_STAMP(sb);
-    const int nwork = (int) (blockDim.x >> 5) - 1;
-    auto bar_workers = [nwork]() { asm volatile("bar.sync 1, %0;\n" ::"r"(32 * nwork) : "memory"); };
-    // The update A_jj -= P P^T by the previous panel's rows: warp 0 updates the first 16 x 16
-    // diagonal block and starts factoring it while the other warps update the rest (the
-    // padded rows of P are zero, so the identity padding survives).
-    if (staged || Pp) {
-        if (warp == 0) {
-            smem_mma(T, P, P, 1, 16, 16, 64, -1.0, true, true, 0, 1);
+    const int nq = (nb + 7) / 8;               // column blocks (the padding beyond them is the identity)
+    const int fr = lane >> 2, fc = lane & 3;   // row, and column or column pair, of a fragment's entry
+    double na[16];                             // -P_j as operand fragments
+    if (staged && warp < nq)
+#pragma unroll
+        for (int k = 0; k < 16; ++k) na[k] = -P[8 * warp + fr + (4 * k + fc) * TP];
+    if (warp == 0) {
+        if (staged) {
+            double *c = T + fr + 2 * fc * TP, acc[2] = {c[0], c[TP]};
+            mma8_64(acc, na, P);
+            c[0] = acc[0];
+            c[TP] = acc[1];
             __syncwarp();
-        } else {
-            smem_mma(T + 16, P + 16, P, 1, 48, 16, 64, -1.0, true, false, 1, nwork);
-            smem_mma(T + 16 + 16 * TP, P + 16, P + 16, 1, 48, 48, 64, -1.0, true, true, 1, nwork);
         }
-    }
-    // Four 16-column sweeps with a one-block look-ahead: after sweep s and the panel below
-    // it, warp 0 updates only the next diagonal block and goes on to factor it, while the
-    // other warps apply the rest of the trailing update (and a block row of the inverse);
-    // sweep s + 1 touches only the next diagonal block of T and of X.
-    for (int s0 = 0; s0 < 64; s0 += 16) {
-        if (warp == 0) {
-            const bool ok = warp_chol_inv16(T, X, s0, lane);
-            if (lane == 0 && !ok) fail = s0 + 1;
-        } else if (s0 >= 32) {
-            // block row s0/16 - 1 of the inverse while warp 0 factors block s0/16
-            inverse_block_row(T, X, P, s0 / 16 - 1, 1, nwork, bar_workers);
+        for (int s = 0; s < nq; ++s) {
+            const int o = 8 * s;
+            const double *d = T + o + o * TP;
+            if (s > 0) asm volatile("bar.sync 3, 64;" ::: "memory");
+            // lanes 8-15 carry the pivot block's rows (L_ss), lanes 0-7 the identity's (E_ss);
+            // the upper half warp repeats them
+            double a[8][8], x[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const double t = d[(lane & 7) + c * TP];
+                x[c] = (lane & 8) ? t : ((lane & 7) == c ? 1.0 : 0.0);
+            }
+            load8(d, a);
+            int bad = 8;
+            if (!sweep8(a, x)) {
+                for (int c = 0; c < 8; ++c) x[c] = (lane & 8) ? d[(lane & 7) + c * TP] : ((lane & 7) == c ? 1.0 : 0.0);
+                bad = sweep8_any(d, x);
+            }
+            double *out = ((lane & 8) ? Ls : U) + (s & 1) * 8 * PU + (lane & 7);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) out[c * PU] = x[c];
+            if (bad < 8) fail = o + bad + 1;
+            asm volatile("bar.arrive 1, 256;" ::: "memory");
+            CHOL_STAMP(sb + 1 + s);
+            if (bad < 8) break;
         }
-        __syncthreads();
-        CHOL_STAMP(sb + 1 + (s0 >> 4) * 2);
-        if (fail) break;
-        const int rem = 64 - s0 - 16;
-        if (rem > 0) {
-            // panel below: P = T_below X_ss^T (all warps)
-            smem_mma(P + s0 + 16, T + (s0 + 16) + s0 * TP, X + s0 + s0 * TP, 1, rem, 16, 16, 1.0, false, false);
-            __syncthreads();
-            if (warp == 0) {
-                // the next diagonal block and its rows of the panel
-                const int r0 = s0 + 16;
-                smem_mma(T + r0 + r0 * TP, P + r0, P + r0, 1, 16, 16, 16, -1.0, true, true, 0, 1);
-                for (int idx = lane; idx < 256; idx += 32) {
-                    const int r = r0 + (idx & 15), c = idx >> 4;
-                    T[r + (s0 + c) * TP] = P[r + c * TP];
-                }
-                __syncwarp();
-            } else if (rem > 16) {
-                // rows below the next diagonal block: T[r1.., r0..] -= P_rest [P_next; P_rest]^T
-                const int r0 = s0 + 16, r1 = s0 + 32, rr = rem - 16;
-                smem_mma(T + r1 + r0 * TP, P + r1, P + r0, 1, rr, 16, 16, -1.0, true, false, 1, nwork);
-                smem_mma(T + r1 + r1 * TP, P + r1, P + r1, 1, rr, rr, 16, -1.0, true, true, 1, nwork);
-                for (int idx = tid - 32; idx < rr * 16; idx += 32 * nwork) {
-                    const int r = r1 + (idx & 15) + 16 * (idx >> 8), c = (idx >> 4) & 15;
-                    T[r + (s0 + c) * TP] = P[r + c * TP];
+    } else {
+        const int j = warp;
+        const bool live = j < nq;
+        // acc[r]: the row block's tile of column block s + r (a row of T has j - s + 1 of them)
+        double acc[8][2];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const double *c = T + 8 * j + fr + (8 * q + 2 * fc) * TP;
+            acc[q][0] = c[0];
+            acc[q][1] = c[TP];
+        }
+        if (staged && live) {
+            mma8_64(acc[0], na, P);
+            mma8_64(acc[1], na, P + 8);
+        }
+        for (int s = 0; s < nq; ++s) {
+            const double *Us = U + (s & 1) * 8 * PU;
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            const double2 u = *reinterpret_cast<const double2 *>(Us + 2 * fc + fr * PU);
+            const int failed = *(volatile int *) &fail;
+            const bool low = j > s;
+            // the tile of column s times E_ss
+            double c[2] = {}, f[2] = {};
+            dmma_c(c[0], c[1], acc[0][0], u.x);
+            dmma_c(f[0], f[1], acc[0][1], u.y);
+            c[0] += f[0];
+            c[1] += f[1];
+            if (failed) break;
+            if (live && (low || j - 1 < s)) {
+                if (low) {
+                    if (j == s + 1) {
+                        double *t = T + 8 * j + fr + (8 * j + 2 * fc) * TP;
+                        dmma_c(acc[1][0], acc[1][1], -c[0], c[0]);
+                        dmma_c(acc[1][0], acc[1][1], -c[1], c[1]);
+                        t[0] = acc[1][0];
+                        t[TP] = acc[1][1];
+                        asm volatile("bar.arrive 3, 64;" ::: "memory");
+                    }
+                    double *b = B + 8 * j + fr + 2 * fc * PB;
+                    b[0] = c[0];
+                    b[PB] = c[1];
+                    if (8 * j + fr < nb) {
+                        double *g = Ljj + (size_t) (8 * j + fr) + (size_t) (8 * s + 2 * fc) * ld;
+                        g[0] = c[0];
+                        g[ld] = c[1];
+                    }
+                } else {
+                    const int r = 8 * s + 2 * fc;
+                    double *g = Dj + (size_t) r + (size_t) (8 * (j - 1) + fr) * ldd;
+                    if (r + 1 < nb && vec) {
+                        *reinterpret_cast<double2 *>(g) = make_double2(c[0], c[1]);
+                    } else {
+                        if (r < nb) g[0] = c[0];
+                        if (r + 1 < nb) g[1] = c[1];
+                    }
                 }
             }
-        }
-        CHOL_STAMP(sb + 2 + (s0 >> 4) * 2);
-    }
-    if (fail) {
-        if (tid == 0) *info = j0 + fail;
-        return false;
-    }
-    // the last block row of the inverse, with all warps
-    inverse_block_row(T, X, P, 3, 0, 0, []() { __syncthreads(); });
-    __syncthreads();
-    CHOL_STAMP(sb + 10);
-    // write L (lower part only) and Dinv (zero beyond column nb), two rows per store
-    const bool vl = ((((size_t) Ljj) & 15) == 0) && ((ld & 1) == 0);
-    const bool vd = ((((size_t) (Dinv + j0)) & 15) == 0) && ((ldd & 1) == 0);
-    for (int idx = tid; idx < 32 * 64; idx += blockDim.x) {
-        const int r = (idx & 31) * 2, cc = idx >> 5;
-        if (r >= nb) continue;
-        const bool two = r + 1 < nb;
-        if (cc < nb && r + 1 >= cc) {
-            double *dst = Ljj + (size_t) r + (size_t) cc * ld;
-            if (two && r >= cc && vl) {
-                *reinterpret_cast<double2 *>(dst) = make_double2(T[r + cc * TP], T[r + 1 + cc * TP]);
-            } else {
-                if (r >= cc) dst[0] = T[r + cc * TP];
-                if (two) dst[1] = T[r + 1 + cc * TP];
+            asm volatile("bar.sync 2, 224;" ::: "memory");
+            if (live) {
+                if (j == s + 1) {
+                    // from here on row block s of E: E_ss, and -E_ss T(q, s)^T to its right
+#pragma unroll
+                    for (int r = 1; r < 8; ++r) acc[r][0] = acc[r][1] = 0.0;
+                    c[0] = Us[fr + 2 * fc * PU];
+                    c[1] = Us[fr + (2 * fc + 1) * PU];
+                }
+                const int last = (j > s + 1) ? j - s : (j <= s + 1 ? nq - 1 - s : 0);
+#pragma unroll
+                for (int r = 1; r < 8; ++r) {
+                    if (r > last) break;
+                    const double *b = B + 8 * (s + r) + fr + 2 * fc * PB;
+                    dmma_c(acc[r][0], acc[r][1], -c[0], b[0]);
+                    dmma_c(acc[r][0], acc[r][1], -c[1], b[PB]);
+                }
+                if (staged && j > s + 1) mma8_64(acc[2], na, P + 8 * (s + 2));
+#pragma unroll
+                for (int r = 0; r < 7; ++r) {
+                    acc[r][0] = acc[r + 1][0];
+                    acc[r][1] = acc[r + 1][1];
+                }
             }
-        }
-        const double d0 = (cc < nb) ? X[r + cc * TP] : 0.0;
-        const double d1 = (cc < nb) ? X[r + 1 + cc * TP] : 0.0;
-        double *dd = Dinv + (size_t) (j0 + r) + (size_t) cc * ldd;
-        if (two && vd) {
-            *reinterpret_cast<double2 *>(dd) = make_double2(d0, d1);
-        } else {
-            dd[0] = d0;
-            if (two) dd[1] = d1;
+            if (j == 1) {
+                // the pivot block of L and of Dinv
+                const double *l = Ls + (s & 1) * 8 * PU;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int r = lane & 7, c = (lane >> 3) + 4 * h, gr = 8 * s + r, gc = 8 * s + c;
+                    if (gr < nb && r >= c) Ljj[(size_t) gr + (size_t) gc * ld] = l[r + c * PU];
+                    if (gr < nb && r >= c) Dj[(size_t) gr + (size_t) gc * ldd] = Us[c + r * PU];
+                }
+            }
         }
     }
     __syncthreads();
     CHOL_STAMP(sb + 11);
+    if (fail) {
+        if (tid == 0) *info = j0 + fail;
+        return false;
+    }
     return true;
 }
 
@@ -366,10 +420,18 @@ __device__ __forceinline__ void stage_job(const TileJob &J, double *As, double *
     }
 }
 
+// The 32 x 16 part of the 64 x 64 tile that this warp computes. Warps w and w + 4 share an SM
+// sub-partition: they take opposite rows and columns (0 and 3, 1 and 2 of the four column
+// parts), so that a triangular operand leaves every sub-partition the same work.
+__device__ __forceinline__ int warp_row() { return (((threadIdx.x >> 5) & 1) ^ (threadIdx.x >> 7)) * 32; }
+__device__ __forceinline__ int warp_col() {
+    const int w = threadIdx.x >> 5;
+    return ((w < 4) ? (w >> 1) : 3 - ((w - 4) >> 1)) * 16;
+}
+
 // This thread's C entries of a mode-0 job (zero otherwise), in fragment order.
 __device__ __forceinline__ void load_c(const TileJob &J, double (&cv)[4][2][2]) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int wm = (w & 1) * 32, wn = (w >> 1) * 16;
+    const int lane = threadIdx.x & 31, wm = warp_row(), wn = warp_col();
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -383,14 +445,17 @@ __device__ __forceinline__ void load_c(const TileJob &J, double (&cv)[4][2][2]) 
             }
 }
 
-// acc = As * Bs^T over k < kp (8 warps: a 32 x 16 block of 8 x 8 DMMA tiles each).
-__device__ __forceinline__ void dmma_tile(const double *As, const double *Bs, int kp, double (&acc)[4][2][2]) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int wm = (w & 1) * 32, wn = (w >> 1) * 16;
+// acc = As * Bs^T over k < kp (8 warps: a 32 x 16 block of 8 x 8 DMMA tiles each). tri 1: Bs is
+// lower triangular (Bs(c, k) = 0 for k > c), tri 2: As is; the zero part is skipped.
+__device__ __forceinline__ void dmma_tile(const double *As, const double *Bs, int kp, double (&acc)[4][2][2],
+                                          int tri = 0) {
+    const int lane = threadIdx.x & 31, wm = warp_row(), wn = warp_col();
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    if (tri == 1) kp = min(kp, wn + 16);
+    if (tri == 2) kp = min(kp, wm + 32);
     for (int k = 0; k < kp; k += 4) {
         const int kk = k + (lane & 3);
         double a[4], b[2];
@@ -409,8 +474,7 @@ __device__ __forceinline__ void dmma_tile(const double *As, const double *Bs, in
 // into shared memory (pitch TP, zeros outside the written entries).
 __device__ __forceinline__ void store_tile(const TileJob &J, const double (&cv)[4][2][2],
                                            const double (&acc)[4][2][2], double *Ct, long ldct, double *Csm) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int wm = (w & 1) * 32, wn = (w >> 1) * 16;
+    const int lane = threadIdx.x & 31, wm = warp_row(), wn = warp_col();
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int r = wm + i * 8 + (lane >> 2);
@@ -434,17 +498,17 @@ __device__ __forceinline__ void store_tile(const TileJob &J, const double (&cv)[
 // One tile product with its operands staged in regions 0 and 1. Operands are staged
 // first, so C may alias A or B (in-place panel solves).
 __device__ void tile_mma_dev(double *Cb, long ldc, int mr, int nc, const double *Ab, long lda, int ar,
-                             const double *Bb, long ldb, int bt, int bc, int nb, bool diag, int mode, double *sm,
-                             double *Ct = nullptr, long ldct = 0, double *Csm = nullptr) {
+                             const double *Bb, long ldb, int bt, int bc, int nb, bool diag, int mode,
+                             double *Ct = nullptr, long ldct = 0, double *Csm = nullptr, int tri = 0) {
     const TileJob J{Cb, ldc, mr, nc, Ab, lda, ar, Bb, ldb, bt, bc, nb, diag, mode};
-    double *As = sm, *Bs = sm + 64 * TP;
+    double *As = region(0), *Bs = region(1);
     stage_job(J, As, Bs);
     double cv[4][2][2];
     load_c(J, cv);  // while the operand copies are in flight
     cpa_wait_all();
     __syncthreads();
     double acc[4][2][2];
-    dmma_tile(As, Bs, (nb + 3) & ~3, acc);
+    dmma_tile(As, Bs, (nb + 3) & ~3, acc, tri);
     store_tile(J, cv, acc, Ct, ldct, Csm);
     __syncthreads();
 }
@@ -454,12 +518,12 @@ __device__ void tile_mma_dev(double *Cb, long ldc, int mr, int nc, const double 
 // entries loaded into registers while the current job's products run. The jobs'
 // C tiles must be disjoint from each other and from every operand.
 template <typename JobOf>
-__device__ void tile_stream(JobOf job_of, long t0, long t1, long step, double *sm) {
+__device__ void tile_stream(JobOf job_of, long t0, long t1, long step) {
     if (t0 >= t1) return;
     TileJob cur, nxt;
     job_of(t0, cur);
     int b = 0;
-    stage_job(cur, sm + (size_t) (2 * b) * 64 * TP, sm + (size_t) (2 * b + 1) * 64 * TP);
+    stage_job(cur, region(2 * b), region(2 * b + 1));
     asm volatile("cp.async.commit_group;\n" ::);
     double cv[4][2][2], cvn[4][2][2];
     load_c(cur, cv);
@@ -467,7 +531,7 @@ __device__ void tile_stream(JobOf job_of, long t0, long t1, long step, double *s
         const bool more = t + step < t1;
         if (more) {
             job_of(t + step, nxt);
-            stage_job(nxt, sm + (size_t) (2 * (b ^ 1)) * 64 * TP, sm + (size_t) (2 * (b ^ 1) + 1) * 64 * TP);
+            stage_job(nxt, region(2 * (b ^ 1)), region(2 * (b ^ 1) + 1));
             asm volatile("cp.async.commit_group;\n" ::);
             load_c(nxt, cvn);
             asm volatile("cp.async.wait_group 1;\n" ::);
@@ -476,7 +540,7 @@ __device__ void tile_stream(JobOf job_of, long t0, long t1, long step, double *s
         }
         __syncthreads();
         double acc[4][2][2];
-        dmma_tile(sm + (size_t) (2 * b) * 64 * TP, sm + (size_t) (2 * b + 1) * 64 * TP, (cur.nb + 3) & ~3, acc);
+        dmma_tile(region(2 * b), region(2 * b + 1), (cur.nb + 3) & ~3, acc);
         store_tile(cur, cv, acc, nullptr, 0, nullptr);
         __syncthreads();  // the buffer just read may be refilled
         if (!more) break;
@@ -510,20 +574,19 @@ __device__ __forceinline__ void tri_index(long t, int &ti, int &tj) {
 // trailing matrix is updated, block row j is finalised as K(j, c) = Dinv_j X(j, c) and
 // K(j, j) = Dinv_j. The strictly upper blocks of K and the strictly lower blocks of KT
 // are never written (they must hold zeros).
-__device__ __forceinline__ void k_update_tile(const double *L, long ld, double *K, int n, int r, int c, int k,
-                                              double *sm) {
+__device__ __forceinline__ void k_update_tile(const double *L, long ld, double *K, int n, int r, int c, int k) {
     const int mr = min(64, n - 64 * r);
     tile_mma_dev(K + (size_t) 64 * r + (size_t) 64 * c * ld, ld, mr, 64, L + (size_t) 64 * r + (size_t) 64 * k * ld,
-                 ld, mr, K + (size_t) 64 * k + (size_t) 64 * c * ld, ld, 0, 64, 64, false, (k == c) ? 2 : 0, sm);
+                 ld, mr, K + (size_t) 64 * k + (size_t) 64 * c * ld, ld, 0, 64, 64, false, (k == c) ? 2 : 0);
 }
 
 __device__ __forceinline__ void k_final_tile(const double *Dinv, long ldd, double *K, double *KT, long ld, int n,
-                                             int bj, int c, double *sm) {
+                                             int bj, int c) {
     const int mr = min(64, n - 64 * bj);
     if (c < bj) {
         double *X = K + (size_t) 64 * bj + (size_t) 64 * c * ld;
-        tile_mma_dev(X, ld, mr, 64, Dinv + (size_t) 64 * bj, ldd, mr, X, ld, 0, 64, mr, false, 1, sm,
-                     KT + (size_t) 64 * c + (size_t) 64 * bj * ld, ld);
+        tile_mma_dev(X, ld, mr, 64, Dinv + (size_t) 64 * bj, ldd, mr, X, ld, 0, 64, mr, false, 1,
+                     KT + (size_t) 64 * c + (size_t) 64 * bj * ld, ld, nullptr, 2);
     } else {
         for (int idx = threadIdx.x; idx < 64 * 64; idx += blockDim.x) {
             const int r = idx & 63, cc = idx >> 6;
@@ -544,9 +607,9 @@ __device__ __forceinline__ void k_final_tile(const double *Dinv, long ldd, doubl
 // result does not depend on it.
 template <class GSync, class GArrive, class GWait>
 __device__ void potrf_body(double *L, long ld, int n, double *Dinv, long ldd, int *info, double *K, double *KT,
-                           int bid, int ngrid, GSync gsync, GArrive garrive, GWait gwait, double *sm) {
+                           int bid, int ngrid, GSync gsync, GArrive garrive, GWait gwait) {
     const int nblk = (n + 63) / 64;
-    if (bid == 0) potf2_dev(L, ld, 0, min(NB, n), Dinv, ldd, info, sm);
+    if (bid == 0) potf2_dev(L, ld, 0, min(NB, n), Dinv, ldd, info);
     gsync();
     for (int j0 = 0; j0 < n; j0 += NB) {
         if (*(volatile int *) info) return;
@@ -565,16 +628,16 @@ __device__ void potrf_body(double *L, long ld, int n, double *Dinv, long ldd, in
         // complete) and keeps its own solved chunk 0, the rows that update that block
         const int nbn = min(NB, rows);
         if (bid == 0)
-            stage_tile(region(sm, R_T), L + (size_t) (j0 + nb) + (size_t) (j0 + nb) * ld, ld, nbn, nbn, 64);
+            stage_tile(region(R_T), L + (size_t) (j0 + nb) + (size_t) (j0 + nb) * ld, ld, nbn, nbn, 64);
         for (long t = bid; t < nchunk + nx; t += ngrid) {
             if (t < nchunk) {
                 const int ch = (int) t;
                 const int mr = min(64, rows - ch * 64);
-                tile_mma_dev(P + ch * 64, ld, mr, nb, P + ch * 64, ld, mr, Dinv + j0, ldd, 1, nb, nb, false, 1, sm,
-                             nullptr, 0, (t == 0) ? region(sm, R_P) : nullptr);
+                tile_mma_dev(P + ch * 64, ld, mr, nb, P + ch * 64, ld, mr, Dinv + j0, ldd, 1, nb, nb, false, 1,
+                             nullptr, 0, (t == 0) ? region(R_P) : nullptr, 1);
             } else {
                 const long u = t - nchunk;
-                k_update_tile(L, ld, K, n, bj + (int) (u / bj), (int) (u % bj), bj - 1, sm);
+                k_update_tile(L, ld, K, n, bj + (int) (u / bj), (int) (u % bj), bj - 1);
             }
         }
         if (bid <= 1) CHOL_STAMP(pb + 1);
@@ -592,7 +655,7 @@ __device__ void potrf_body(double *L, long ld, int n, double *Dinv, long ldd, in
         if (bid == 0) {
             // tile (0, 0) is the next diagonal block: update it in shared memory and factor it
             CHOL_STAMP(pb + 3);
-            potf2_dev(L, ld, j0 + nb, nbn, Dinv, ldd, info, sm, nullptr, 0, true);
+            potf2_dev(L, ld, j0 + nb, nbn, Dinv, ldd, info, true);
             CHOL_STAMP(pb + 4);
         }
         if (early) gwait(tok);
@@ -608,9 +671,9 @@ __device__ void potrf_body(double *L, long ld, int n, double *Dinv, long ldd, in
                 J = TileJob{A22 + (size_t) ti * 64 + (size_t) tj * 64 * ld, ld, mr, nc, P + ti * 64, ld, mr,
                             P + tj * 64, ld, 1, nc, nb, ti == tj, 0};
             };
-            tile_stream(trailing, 1 + wid, ntile, nworker, sm);
+            tile_stream(trailing, 1 + wid, ntile, nworker);
             for (long t = 1 + wid; t < ntile + nk; t += nworker)
-                if (t >= ntile) k_final_tile(Dinv, ldd, K, KT, ld, n, bj, (int) (t - ntile), sm);
+                if (t >= ntile) k_final_tile(Dinv, ldd, K, KT, ld, n, bj, (int) (t - ntile));
         }
         if (bid == 1) CHOL_STAMP(pb + 3);
         gsync();
@@ -620,19 +683,52 @@ __device__ void potrf_body(double *L, long ld, int n, double *Dinv, long ldd, in
     // the last block row of K: its update by block row nblk - 2, then its final form
     const int bj = nblk - 1;
     if (bj >= 1) {
-        for (int c = bid; c < bj; c += ngrid) k_update_tile(L, ld, K, n, bj, c, bj - 1, sm);
+        for (int c = bid; c < bj; c += ngrid) k_update_tile(L, ld, K, n, bj, c, bj - 1);
         gsync();
     }
-    for (int c = bid; c <= bj; c += ngrid) k_final_tile(Dinv, ldd, K, KT, ld, n, bj, c, sm);
+    for (int c = bid; c <= bj; c += ngrid) k_final_tile(Dinv, ldd, K, KT, ld, n, bj, c);
 }
+
+// Grid-wide barrier of a cooperative launch on a counter that starts at zero: every block adds
+// one per barrier and waits for the counter to reach the number of blocks times the barriers so
+// far. One thread of the last warp arrives and waits, so that the arrival of the block that goes
+// on to the diagonal block (a fence and an atomic, 1 us) runs beside the sweeps of the other
+// warps. The wait is bounded; on giving up it sets *info, which every block checks.
+struct GridBarrier {
+    unsigned *count;
+    int *info;
+    unsigned target = 0;
+    static constexpr int kThread = COOP_THREADS - 32;
+    __device__ unsigned arrive() {
+        __syncthreads();
+        target += gridDim.x;
+        if (threadIdx.x == kThread) {
+            __threadfence();
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+        }
+        return target;
+    }
+    __device__ void wait(unsigned t) {
+        if (threadIdx.x == kThread) {
+            unsigned v = 0;
+            long it = 0;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+            } while ((int) (v - t) < 0 && ++it < (1L << 22));
+            if ((int) (v - t) < 0) *(volatile int *) info = -1;
+            __threadfence();
+        }
+        __syncthreads();
+    }
+    __device__ void sync() { wait(arrive()); }
+};
 
 __global__ void __launch_bounds__(COOP_THREADS, 1) potrf_coop_kernel(double *L, long ld, int n, double *Dinv,
                                                                   long ldd, int *info, double *K, double *KT) {
-    cg::grid_group grid = cg::this_grid();
-    extern __shared__ double sm[];
+    GridBarrier bar{reinterpret_cast<unsigned *>(info + 1), info};
     potrf_body(
-        L, ld, n, Dinv, ldd, info, K, KT, (int) blockIdx.x, (int) gridDim.x, [&]() { grid.sync(); },
-        [&]() { return grid.barrier_arrive(); }, [&](unsigned int t) { grid.barrier_wait(std::move(t)); }, sm);
+        L, ld, n, Dinv, ldd, info, K, KT, (int) blockIdx.x, (int) gridDim.x, [&]() { bar.sync(); },
+        [&]() { return bar.arrive(); }, [&](unsigned int t) { bar.wait(t); });
 }
 
 // Several factorisations in one launch, one CTA each: the copy of the lower triangle, the
@@ -678,7 +774,7 @@ __device__ double logdiag_1024(int n, const double *L, long ld) {
     return x;
 }
 
-__device__ void small_factor_job(const SmallFactorJob &J, double *sm) {
+__device__ void small_factor_job(const SmallFactorJob &J) {
     const int n = J.n;
     for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
         const int r = idx % n, c = idx / n;
@@ -693,7 +789,7 @@ __device__ void small_factor_job(const SmallFactorJob &J, double *sm) {
             __syncthreads();
             return 0u;
         },
-        [](unsigned int) {}, sm);
+        [](unsigned int) {});
     __syncthreads();
     double acc = 0.0;
     if (J.logdet) {
@@ -711,21 +807,18 @@ __device__ void small_factor_job(const SmallFactorJob &J, double *sm) {
 }
 
 __global__ void __launch_bounds__(COOP_THREADS, 1) potrf_small_batch_kernel(const SmallFactorBatch B) {
-    extern __shared__ double sm[];
-    small_factor_job(B.job[blockIdx.x], sm);
+    small_factor_job(B.job[blockIdx.x]);
 }
 
 // the same, the jobs in global memory (more than fit the parameters)
 __global__ void __launch_bounds__(COOP_THREADS, 1) potrf_batch_array_kernel(const SmallFactorJob *__restrict__ jobs) {
-    extern __shared__ double sm[];
     const SmallFactorJob J = jobs[blockIdx.x];
-    small_factor_job(J, sm);
+    small_factor_job(J);
 }
 
 __global__ void __launch_bounds__(COOP_THREADS, 1) trtri_coop_kernel(const double *L, double *K, long ld, int n,
                                                                   const double *Dinv, long ldd) {
     cg::grid_group grid = cg::this_grid();
-    extern __shared__ double sm[];
     for (int i0 = 0; i0 < n; i0 += NB) {
         const int nb = min(NB, n - i0);
         const int cend = i0 + nb;
@@ -734,7 +827,7 @@ __global__ void __launch_bounds__(COOP_THREADS, 1) trtri_coop_kernel(const doubl
             // X_i chunk <- Dinv_i * X_i chunk  (in place)
             const int nc = min(64, cend - ch * 64);
             double *Xc = K + i0 + (size_t) ch * 64 * ld;
-            tile_mma_dev(Xc, ld, nb, nc, Dinv + i0, ldd, nb, Xc, ld, 0, nc, nb, false, 1, sm);
+            tile_mma_dev(Xc, ld, nb, nc, Dinv + i0, ldd, nb, Xc, ld, 0, nc, nb, false, 1, nullptr, 0, nullptr, 2);
         }
         grid.sync();
         const int rows = n - cend;
@@ -749,7 +842,7 @@ __global__ void __launch_bounds__(COOP_THREADS, 1) trtri_coop_kernel(const doubl
                         L + (size_t) (cend + ti * 64) + (size_t) i0 * ld, ld, mr, K + i0 + (size_t) tj * 64 * ld, ld,
                         0, nc, nb, false, 0};
         };
-        tile_stream(update, blockIdx.x, ntile, gridDim.x, sm);
+        tile_stream(update, blockIdx.x, ntile, gridDim.x);
         grid.sync();
     }
 }
@@ -783,7 +876,7 @@ __global__ void __launch_bounds__(COOP_THREADS, 1)
                           const double *b, double *t, double *x, unsigned *flag_f, unsigned *flag_b,
                           unsigned epoch) {
     cg::grid_group grid = cg::this_grid();
-    extern __shared__ double sm[];
+    double *sm = dyn_smem;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int G = gridDim.x, me = blockIdx.x;
     const int nblk = (n + 63) / 64;
@@ -987,7 +1080,8 @@ __global__ void identity_k(int n, double *A, long lda) {
     }
 }
 
-__global__ void zero_info_k(int *p) { *p = 0; }
+// the status word and the barrier counter after it
+__global__ void zero_info_k(int *p) { p[0] = p[1] = 0; }
 
 int sm_count() { return device_sm_count(); }
 
@@ -1064,7 +1158,7 @@ __global__ void rec_info_kernel(const RecLeaves R, const int *leaf_info, int *in
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     int v = 0;
     for (int q = 0; q < R.count && v == 0; ++q)
-        if (leaf_info[q] != 0) v = leaf_info[q] + R.off[q];
+        if (leaf_info[2 * q] != 0) v = leaf_info[2 * q] < 0 ? -1 : leaf_info[2 * q] + R.off[q];
     *info = v;
 }
 
@@ -1096,7 +1190,7 @@ bool rec_leaf(cudaStream_t s, DenseFactor &F, int off, int n, double *Kp, double
     V.Dinv = F.Dinv + off;
     V.K = Kp;
     V.KT = KTp;
-    V.d_info = F.d_rec_info + R.count;
+    V.d_info = F.d_rec_info + 2 * R.count;
     V.fuse_k = true;
     V.kfamily = F.kfamily;
     R.off[R.count++] = off;
@@ -1159,7 +1253,7 @@ bool rec_factor_nok(cudaStream_t s, DenseFactor &F, int off, int n, RecLeaves &R
 
 bool rec_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS) {
     const int n = F.n;
-    if (!F.d_rec_info && hb::cmalloc(&F.d_rec_info, sizeof(int) * kRecMaxLeaves) != cudaSuccess) {
+    if (!F.d_rec_info && hb::cmalloc(&F.d_rec_info, 2 * sizeof(int) * kRecMaxLeaves) != cudaSuccess) {
         F.d_rec_info = nullptr;
         return false;
     }
@@ -1167,7 +1261,7 @@ bool rec_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long
         F.d_rec_w = nullptr;
         return false;
     }
-    HB_CUDA(cudaMemsetAsync(F.d_rec_info, 0, sizeof(int) * kRecMaxLeaves, s));
+    HB_CUDA(cudaMemsetAsync(F.d_rec_info, 0, 2 * sizeof(int) * kRecMaxLeaves, s));
     copy_lower_k<<<hb::counted(grid_for_n((long) n * n)), 256, 0, s>>>(n, S, ldS, F.L, F.ld);
     RecLeaves R;
     R.count = 0;
@@ -1180,7 +1274,7 @@ bool rec_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long
 bool rec_factorize_nok_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS) {
     const int n = F.n;
     const size_t strip = (size_t) F.ld * kRecLeafMaxN;
-    if (!F.d_rec_info && hb::cmalloc(&F.d_rec_info, sizeof(int) * kRecMaxLeaves) != cudaSuccess) {
+    if (!F.d_rec_info && hb::cmalloc(&F.d_rec_info, 2 * sizeof(int) * kRecMaxLeaves) != cudaSuccess) {
         F.d_rec_info = nullptr;
         return false;
     }
@@ -1200,7 +1294,7 @@ bool rec_factorize_nok_enqueue(cudaStream_t s, DenseFactor &F, const double *S, 
         HB_CUDA(cudaMemsetAsync(F.d_rec_ks, 0, sizeof(double) * strip, s));
         HB_CUDA(cudaMemsetAsync(F.d_rec_kts, 0, sizeof(double) * strip, s));
     }
-    HB_CUDA(cudaMemsetAsync(F.d_rec_info, 0, sizeof(int) * kRecMaxLeaves, s));
+    HB_CUDA(cudaMemsetAsync(F.d_rec_info, 0, 2 * sizeof(int) * kRecMaxLeaves, s));
     copy_lower_k<<<hb::counted(grid_for_n((long) n * n)), 256, 0, s>>>(n, S, ldS, F.L, F.ld);
     RecLeaves R;
     R.count = 0;

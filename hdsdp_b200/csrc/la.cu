@@ -973,8 +973,9 @@ void factorize_small_batch(cudaStream_t s, DenseFactor *const *F, const double *
 }
 
 bool factor_status_ready(DenseFactor &F) {
+    if (*(volatile int *) F.h_info < 0) device_error_flag() = 1;   // a wait inside the kernel gave up
     F.ok = (*(volatile int *) F.h_info == 0);
-    F.k_valid = F.ok && F.k_pending;
+    F.k_valid = F.ok && F.k_pending;  // K and KT were formed by the factorisation kernel
     F.k_pending = false;
     F.logdet_valid = F.ok && F.stat_logdet;
     if (F.logdet_valid) F.logdet = 2.0 * reinterpret_cast<const volatile double *>(F.h_info)[1];
@@ -983,12 +984,7 @@ bool factor_status_ready(DenseFactor &F) {
 
 bool factor_status(cudaStream_t s, DenseFactor &F) {
     HB_CUDA(cudaStreamSynchronize(s));
-    F.ok = (*F.h_info == 0);
-    F.k_valid = F.ok && F.k_pending;  // K and KT were formed by the factorisation kernel
-    F.k_pending = false;
-    F.logdet_valid = F.ok && F.stat_logdet;
-    if (F.logdet_valid) F.logdet = 2.0 * reinterpret_cast<const double *>(F.h_info)[1];
-    return F.ok;
+    return factor_status_ready(F);
 }
 
 bool factorize(cudaStream_t s, DenseFactor &F, const double *S, long ldS) {

@@ -98,6 +98,9 @@ extern "C" int hdsdpb_cholesky_noalloc(int n, const double *S, double *L, double
     if (cudaMemcpy2D(dS, sizeof(double) * ld, S, sizeof(double) * n, sizeof(double) * n, n,
                      cudaMemcpyHostToDevice) != cudaSuccess)
         return -1;
+    // the factorisation writes only the lower triangles of Dinv's blocks, and an earlier call of
+    // another order has left its own there
+    if (cudaMemsetAsync(F.Dinv, 0, sizeof(double) * ld * 64, s) != cudaSuccess) return -1;
     const bool ok = factorize(s, F, dS, ld);
     if (ok) {
         log_diag_sum(s, F, dl);
