@@ -1,12 +1,18 @@
 // Persistent cooperative Cholesky factorisation and triangular inverse.
 //
-// One cooperative launch covers the whole factorisation: for every 64-column
-// panel, block 0 factors the diagonal block (and inverts it), the grid
-// synchronises, all blocks solve the panel rows, synchronise, then update the
-// trailing lower triangle tile by tile on the DMMA path, and synchronise
-// again. A failed pivot (non-positive or NaN, the dpotrf test used by the
-// reference's positive-definiteness checks, linalg/hdsdp_linsolver.c:521-553)
-// is published in *info and every block leaves at the next grid barrier.
+// One cooperative launch covers the whole factorisation: for every 64-column panel, block 0
+// factors the diagonal block (and inverts it), all blocks solve the panel rows, then update the
+// trailing lower triangle tile by tile on the DMMA path. Block 0's chain (its first rows of the
+// panel, the next diagonal block) sets the time; the blocks signal one another through counters
+// and wait only for what they read. A failed pivot (non-positive or NaN, the dpotrf test used by
+// the reference's positive-definiteness checks, linalg/hdsdp_linsolver.c:521-553) is published
+// in *info and every block leaves at its next wait for a diagonal block. The status and
+// sum log L_ii go to the host from the same launch.
+//
+// Measured (factor only / with K = L^-1, ms, copy and status included): order 64 0.038 / 0.048
+// -> 0.017 / 0.021, 200 0.111 / 0.123 -> 0.049 / 0.061, 500 0.205 / 0.222 -> 0.105 / 0.115,
+// 1000 0.394 / 0.408 -> 0.209 / 0.226, 2000 0.782 / 0.957 -> 0.529 / 0.754 (before: shuffled
+// 16-column sweeps, two grid barriers a panel, five launches a factorisation).
 //
 // The triangular inverse K = L^-1 uses the same structure on block rows:
 // X_i <- Dinv_i X_i, then X_below -= L_below,i X_i.
@@ -63,22 +69,25 @@ __device__ __forceinline__ void cpa16(double *sdst, const double *gsrc, int byte
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(gsrc), "r"(bytes));
 }
 
-// Stage columns 0..ncols-1 of the 64-row tile G (column-major, pitch ldg) into S (pitch
-// TP): entries with row < nr and column < nc are copied, the rest of those columns is
-// zero. Two rows move per copy when G and ldg keep every pair 16-byte aligned. The
-// caller waits with cpa_wait_all().
-__device__ __forceinline__ void stage_tile(double *S, const double *G, long ldg, int nr, int nc, int ncols) {
+// Stage columns 0..ncols-1 of the R-row tile G (column-major, pitch ldg) into S (pitch PS):
+// entries with row < nr and column < nc are copied, the rest of those columns is zero. Two rows
+// move per copy when G and ldg keep every pair 16-byte aligned. With `lower` the entries above
+// the diagonal (zeros in global memory) are not fetched. The caller waits with cpa_wait_all().
+template <int R = 64, int PS = TP>
+__device__ __forceinline__ void stage_tile(double *S, const double *G, long ldg, int nr, int nc, int ncols,
+                                           bool lower = false) {
     if (((((size_t) G) & 15) == 0) && ((ldg & 1) == 0)) {
-        for (int idx = threadIdx.x; idx < 32 * ncols; idx += blockDim.x) {
-            const int r = (idx & 31) * 2, c = idx >> 5;
-            const int cnt = (c < nc) ? min(2, max(0, nr - r)) : 0;
-            cpa16(&S[r + c * TP], cnt ? G + (size_t) r + (size_t) c * ldg : G, 8 * cnt);
+#pragma unroll 4
+        for (int idx = threadIdx.x; idx < (R / 2) * ncols; idx += blockDim.x) {
+            const int r = (idx % (R / 2)) * 2, c = idx / (R / 2);
+            const int cnt = (c < nc && !(lower && r + 1 < c)) ? min(2, max(0, nr - r)) : 0;
+            cpa16(&S[r + c * PS], cnt ? G + (size_t) r + (size_t) c * ldg : G, 8 * cnt);
         }
     } else {
-        for (int idx = threadIdx.x; idx < 64 * ncols; idx += blockDim.x) {
-            const int r = idx & 63, c = idx >> 6;
+        for (int idx = threadIdx.x; idx < R * ncols; idx += blockDim.x) {
+            const int r = idx % R, c = idx / R;
             const bool ok = r < nr && c < nc;
-            cpa8(&S[r + c * TP], ok ? G + (size_t) r + (size_t) c * ldg : G, ok);
+            cpa8(&S[r + c * PS], ok ? G + (size_t) r + (size_t) c * ldg : G, ok);
         }
     }
 }
@@ -103,7 +112,7 @@ __device__ __forceinline__ void dmma_c(double &d0, double &d1, double a, double 
 // life with that sweep) and bring it up to date while warp 0 is in the next sweep. A block with
 // its update by the previous panel takes 7.3 us (13,000 cycles, of which 740 a
 // sweep are warp 0's arithmetic); 16.3 us with 16-column sweeps by shuffles and a separate
-// inverse. Order 1000: 0.394 -> 0.235 ms, with K = L^-1 0.408 -> 0.290 ms.
+// inverse.
 // ---------------------------------------------------------------------------------
 
 // c += -(A B^T) over 64 columns for operand fragments na = -A and the 8-row block B in shared
@@ -179,10 +188,22 @@ __device__ __forceinline__ bool sweep8(double (&a)[8][8], double (&x)[8]) {
     return fine;
 }
 
-// The same for any pivots, a column at a time with rsqrt(); returns the first column whose
-// pivot is not positive, or 8.
-__device__ __noinline__ int sweep8_any(const double *d, double (&x)[8]) {
-    double a[8][8];
+// The lane's row at the start of a sweep: lanes 8-15 carry the pivot block's rows (and end with
+// L_ss), lanes 0-7 the identity's (E_ss = L_ss^-T); the upper half warp repeats them.
+__device__ __forceinline__ void load_row8(const double *d, double (&x)[8]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const double t = d[(lane & 7) + c * TP];
+        x[c] = (lane & 8) ? t : ((lane & 7) == c ? 1.0 : 0.0);
+    }
+}
+
+// The sweep over the pivot block d for any pivots, a column at a time with rsqrt(), the lane's
+// row to out (pitch po); returns the first column whose pivot is not positive, or 8.
+__device__ __noinline__ int sweep8_any(const double *d, double *out, int po) {
+    double a[8][8], x[8];
+    load_row8(d, x);
     load8(d, a);
     int bad = 8;
 #pragma unroll
@@ -200,6 +221,8 @@ __device__ __noinline__ int sweep8_any(const double *d, double (&x)[8]) {
             x[q] -= x[c] * a[q][c];
         }
     }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) out[c * po] = x[c];
     return bad;
 }
 
@@ -223,7 +246,11 @@ __device__ __forceinline__ double *region(int r) { return dyn_smem + r * 64 * TP
 // (barrier 1). Every row block multiplies its tile of column s by E_ss; those of T are published
 // as operands (barrier 2, without warp 0), and each row block is updated with them. The owner
 // of row s + 1 updates the next pivot block before all else and hands it to warp 0 (barrier 3).
-__device__ bool potf2_dev(double *L, long ld, int j0, int nb, double *Dinv, long ldd, int *info, bool staged = false) {
+//
+// mid() is called by one thread of warp 2 near the end, where that warp has time to spare.
+template <class Mid>
+__device__ __forceinline__ bool potf2_dev(double *L, long ld, int j0, int nb, double *Dinv, long ldd, int *info,
+                                          bool staged, Mid mid) {
     double *T = region(R_T), *P = region(R_P);
     // E_ss and L_ss of alternate sweeps (8 columns, pitch PU), the published tiles of column s
     // (pitch PB). An 8 x 8 tile held as accumulators serves as a DMMA operand as it is: register h
@@ -236,7 +263,7 @@ __device__ bool potf2_dev(double *L, long ld, int j0, int nb, double *Dinv, long
     double *Ljj = L + (size_t) j0 + (size_t) j0 * ld;
     double *Dj = Dinv + j0;
     const bool vec = ((((size_t) Dj) & 15) == 0) && ((ldd & 1) == 0);   // two rows of Dinv a store
-    if (!staged) stage_tile(T, Ljj, ld, nb, nb, 64);
+    if (!staged) stage_tile(T, Ljj, ld, nb, nb, 64, true);
     cpa_wait_all();
     if (tid == 0) fail = 0;
     for (int r = nb + tid; r < 64; r += blockDim.x) T[r + r * TP] = 1.0;  // pad with the identity
@@ -262,23 +289,15 @@ __device__ bool potf2_dev(double *L, long ld, int j0, int nb, double *Dinv, long
             const int o = 8 * s;
             const double *d = T + o + o * TP;
             if (s > 0) asm volatile("bar.sync 3, 64;" ::: "memory");
-            // lanes 8-15 carry the pivot block's rows (L_ss), lanes 0-7 the identity's (E_ss);
-            // the upper half warp repeats them
             double a[8][8], x[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const double t = d[(lane & 7) + c * TP];
-                x[c] = (lane & 8) ? t : ((lane & 7) == c ? 1.0 : 0.0);
-            }
+            load_row8(d, x);
             load8(d, a);
-            int bad = 8;
-            if (!sweep8(a, x)) {
-                for (int c = 0; c < 8; ++c) x[c] = (lane & 8) ? d[(lane & 7) + c * TP] : ((lane & 7) == c ? 1.0 : 0.0);
-                bad = sweep8_any(d, x);
-            }
             double *out = ((lane & 8) ? Ls : U) + (s & 1) * 8 * PU + (lane & 7);
+            const bool fine = sweep8(a, x);
 #pragma unroll
             for (int c = 0; c < 8; ++c) out[c * PU] = x[c];
+            int bad = 8;
+            if (!fine) bad = sweep8_any(d, out, PU);
             if (bad < 8) fail = o + bad + 1;
             asm volatile("bar.arrive 1, 256;" ::: "memory");
             CHOL_STAMP(sb + 1 + s);
@@ -342,6 +361,7 @@ __device__ bool potf2_dev(double *L, long ld, int j0, int nb, double *Dinv, long
                 }
             }
             asm volatile("bar.sync 2, 224;" ::: "memory");
+            if (j == 2 && s == max(0, nq - 2) && lane == 0) mid();
             if (live) {
                 if (j == s + 1) {
                     // from here on row block s of E: E_ss, and -E_ss T(q, s)^T to its right
@@ -350,14 +370,23 @@ __device__ bool potf2_dev(double *L, long ld, int j0, int nb, double *Dinv, long
                     c[0] = Us[fr + 2 * fc * PU];
                     c[1] = Us[fr + (2 * fc + 1) * PU];
                 }
-                const int last = (j > s + 1) ? j - s : (j <= s + 1 ? nq - 1 - s : 0);
+                // every operand first (those past the last column block are read, not used)
+                const int last = (j > s + 1) ? j - s : nq - 1 - s;
+                const double *b = B + 8 * s + fr + 2 * fc * PB;
+                double bv[8][2];
 #pragma unroll
                 for (int r = 1; r < 8; ++r) {
-                    if (r > last) break;
-                    const double *b = B + 8 * (s + r) + fr + 2 * fc * PB;
-                    dmma_c(acc[r][0], acc[r][1], -c[0], b[0]);
-                    dmma_c(acc[r][0], acc[r][1], -c[1], b[PB]);
+                    bv[r][0] = b[8 * r];
+                    bv[r][1] = b[8 * r + PB];
                 }
+                c[0] = -c[0];
+                c[1] = -c[1];
+#pragma unroll
+                for (int r = 1; r < 8; ++r)
+                    if (r <= last) dmma_c(acc[r][0], acc[r][1], c[0], bv[r][0]);
+#pragma unroll
+                for (int r = 1; r < 8; ++r)
+                    if (r <= last) dmma_c(acc[r][0], acc[r][1], c[1], bv[r][1]);
                 if (staged && j > s + 1) mma8_64(acc[2], na, P + 8 * (s + 2));
 #pragma unroll
                 for (int r = 0; r < 7; ++r) {
@@ -405,112 +434,138 @@ struct TileJob {
     int mode;
 };
 
-// Issue the copies of a job's operands into As / Bs (pitch TP, zero padded).
-__device__ __forceinline__ void stage_job(const TileJob &J, double *As, double *Bs) {
-    const int kp = (J.nb + 3) & ~3;
-    stage_tile(As, J.A, J.lda, J.ar, J.nb, kp);
-    if (J.bt) {
-        stage_tile(Bs, J.B, J.ldb, J.bc, J.nb, kp);
-    } else {
-        for (int idx = threadIdx.x; idx < 64 * kp; idx += blockDim.x) {
-            const int r = idx & 63, k = idx >> 6;
-            const bool okb = r < J.bc && k < J.nb;
-            cpa8(&Bs[r + k * TP], okb ? J.B + (size_t) k + (size_t) r * J.ldb : J.B, okb);
+// An MR x NC tile (32 or 64 each) of a job by the block's 8 warps, 16 columns and MR NC / 128
+// rows a warp, in 8 x 8 DMMA tiles. Operands sit in shared memory as A (row r, column k at
+// r + k (MR + 4)) and B, by rows of op(B)^T (c + k (NC + 4)) or, untransposed, by columns of
+// op(B) (k + c TP): pitches that are 4 modulo 16 keep the fragment reads of either free of bank
+// conflicts. Every entry is the same chain of products over k = 0, 4, 8, ... whatever the tile,
+// so the result does not depend on the tile size.
+template <int MR, int NC>
+struct Tile {
+    static constexpr int WN = NC / 16, WM = 8 / WN, RW = MR / WM, TI = RW / 8, PA = MR + 4, PB = NC + 4;
+    static constexpr int A_DOUBLES = 64 * PA;
+    // Warps w and w + 4 share an SM sub-partition: of a 64 x 64 tile they take opposite rows and
+    // columns (0 and 3, 1 and 2 of the column parts), so that a triangular operand leaves every
+    // sub-partition the same work.
+    static __device__ __forceinline__ int row0() {
+        const int w = threadIdx.x >> 5;
+        return (WN == 4 ? ((w & 1) ^ (w >> 2)) : (w & 3)) * RW;
+    }
+    static __device__ __forceinline__ int col0() {
+        const int w = threadIdx.x >> 5;
+        return (WN == 4 ? ((w < 4) ? (w >> 1) : 3 - ((w - 4) >> 1)) : (w >> 2)) * 16;
+    }
+    // issue the copies of the operands (zero padded); tri 1: op(B)^T is lower triangular, tri 2: A is
+    static __device__ __forceinline__ void stage(const TileJob &J, double *As, double *Bs, int tri = 0) {
+        const int kp = (J.nb + 3) & ~3;
+        stage_tile<MR, PA>(As, J.A, J.lda, J.ar, J.nb, kp, tri == 2);
+        if (J.bt) stage_tile<NC, PB>(Bs, J.B, J.ldb, J.bc, J.nb, kp, tri == 1);
+        else stage_tile<64, TP>(Bs, J.B, J.ldb, J.nb, J.bc, NC);
+    }
+    // this thread's C entries of a mode-0 job (zero otherwise), in fragment order
+    static __device__ __forceinline__ void load_c(const TileJob &J, double (&cv)[TI][2][2]) {
+        const int lane = threadIdx.x & 31, wm = row0(), wn = col0();
+#pragma unroll
+        for (int i = 0; i < TI; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int r = wm + i * 8 + (lane >> 2), c = wn + j * 8 + (lane & 3) * 2 + e;
+                    cv[i][j][e] = (J.mode == 0 && r < J.mr && c < J.nc && !(J.diag && r < c))
+                                      ? J.C[(size_t) r + (size_t) c * J.ldc]
+                                      : 0.0;
+                }
+    }
+    // acc = A op(B) over k < kp, the zero part of a triangular operand skipped
+    template <bool BT>
+    static __device__ __forceinline__ void mma(const double *As, const double *Bs, int kp, double (&acc)[TI][2][2],
+                                               int tri) {
+        const int lane = threadIdx.x & 31, wm = row0(), wn = col0();
+#pragma unroll
+        for (int i = 0; i < TI; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+        if (tri == 1) kp = min(kp, wn + 16);
+        if (tri == 2) kp = min(kp, wm + RW);
+#pragma unroll 4
+        for (int k = 0; k < kp; k += 4) {
+            const int kk = k + (lane & 3);
+            double a[TI], b[2];
+#pragma unroll
+            for (int i = 0; i < TI; ++i) a[i] = As[(wm + i * 8 + (lane >> 2)) + kk * PA];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int c = wn + j * 8 + (lane >> 2);
+                b[j] = BT ? Bs[c + kk * PB] : Bs[kk + c * TP];
+            }
+#pragma unroll
+            for (int i = 0; i < TI; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) dmma_c(acc[i][j][0], acc[i][j][1], a[i], b[j]);
         }
     }
-}
-
-// The 32 x 16 part of the 64 x 64 tile that this warp computes. Warps w and w + 4 share an SM
-// sub-partition: they take opposite rows and columns (0 and 3, 1 and 2 of the four column
-// parts), so that a triangular operand leaves every sub-partition the same work.
-__device__ __forceinline__ int warp_row() { return (((threadIdx.x >> 5) & 1) ^ (threadIdx.x >> 7)) * 32; }
-__device__ __forceinline__ int warp_col() {
-    const int w = threadIdx.x >> 5;
-    return ((w < 4) ? (w >> 1) : 3 - ((w - 4) >> 1)) * 16;
-}
-
-// This thread's C entries of a mode-0 job (zero otherwise), in fragment order.
-__device__ __forceinline__ void load_c(const TileJob &J, double (&cv)[4][2][2]) {
-    const int lane = threadIdx.x & 31, wm = warp_row(), wn = warp_col();
+    // write the result; with Ct also transposed to Ct (pitch ldct), with Csm also into shared
+    // memory (pitch TP, zeros outside the written entries)
+    static __device__ __forceinline__ void store(const TileJob &J, const double (&cv)[TI][2][2],
+                                                 const double (&acc)[TI][2][2], double *Ct, long ldct, double *Csm) {
+        const int lane = threadIdx.x & 31, wm = row0(), wn = col0();
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < TI; ++i) {
+            const int r = wm + i * 8 + (lane >> 2);
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+            for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int r = wm + i * 8 + (lane >> 2), c = wn + j * 8 + (lane & 3) * 2 + e;
-                cv[i][j][e] = (J.mode == 0 && r < J.mr && c < J.nc && !(J.diag && r < c))
-                                  ? J.C[(size_t) r + (size_t) c * J.ldc]
-                                  : 0.0;
-            }
-}
-
-// acc = As * Bs^T over k < kp (8 warps: a 32 x 16 block of 8 x 8 DMMA tiles each). tri 1: Bs is
-// lower triangular (Bs(c, k) = 0 for k > c), tri 2: As is; the zero part is skipped.
-__device__ __forceinline__ void dmma_tile(const double *As, const double *Bs, int kp, double (&acc)[4][2][2],
-                                          int tri = 0) {
-    const int lane = threadIdx.x & 31, wm = warp_row(), wn = warp_col();
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    if (tri == 1) kp = min(kp, wn + 16);
-    if (tri == 2) kp = min(kp, wm + 32);
-    for (int k = 0; k < kp; k += 4) {
-        const int kk = k + (lane & 3);
-        double a[4], b[2];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = As[(wm + i * 8 + (lane >> 2)) + kk * TP];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) b[j] = Bs[(wn + j * 8 + (lane >> 2)) + kk * TP];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) dmma_c(acc[i][j][0], acc[i][j][1], a[i], b[j]);
-    }
-}
-
-// Write the job's result; with Ct also transposed to Ct (pitch ldct), with Csm also
-// into shared memory (pitch TP, zeros outside the written entries).
-__device__ __forceinline__ void store_tile(const TileJob &J, const double (&cv)[4][2][2],
-                                           const double (&acc)[4][2][2], double *Ct, long ldct, double *Csm) {
-    const int lane = threadIdx.x & 31, wm = warp_row(), wn = warp_col();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = wm + i * 8 + (lane >> 2);
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int c = wn + j * 8 + (lane & 3) * 2 + e;
-                const bool valid = r < J.mr && c < J.nc && !(J.diag && r < c);
-                const double val =
-                    (J.mode == 0) ? cv[i][j][e] - acc[i][j][e] : (J.mode == 2) ? -acc[i][j][e] : acc[i][j][e];
-                if (valid) {
-                    J.C[(size_t) r + (size_t) c * J.ldc] = val;
-                    if (Ct) Ct[(size_t) c + (size_t) r * ldct] = val;
+                for (int e = 0; e < 2; ++e) {
+                    const int c = wn + j * 8 + (lane & 3) * 2 + e;
+                    const bool valid = r < J.mr && c < J.nc && !(J.diag && r < c);
+                    const double val =
+                        (J.mode == 0) ? cv[i][j][e] - acc[i][j][e] : (J.mode == 2) ? -acc[i][j][e] : acc[i][j][e];
+                    if (valid) {
+                        J.C[(size_t) r + (size_t) c * J.ldc] = val;
+                        if (Ct) Ct[(size_t) c + (size_t) r * ldct] = val;
+                    }
+                    if (Csm) Csm[r + c * TP] = valid ? val : 0.0;
                 }
-                if (Csm) Csm[r + c * TP] = valid ? val : 0.0;
-            }
+        }
     }
-}
+    // One tile product. Operands are staged first, so C may alias A or B (in-place solves).
+    // issued() is called when their copies are on the way.
+    template <class Issued>
+    static __device__ __forceinline__ void run(const TileJob &J, int tri, double *Ct, long ldct, double *Csm,
+                                               Issued issued) {
+        double *As = dyn_smem, *Bs = dyn_smem + A_DOUBLES;
+        stage(J, As, Bs, tri);
+        issued();
+        double cv[TI][2][2];
+        load_c(J, cv);  // while the operand copies are in flight
+        cpa_wait_all();
+        __syncthreads();
+        double acc[TI][2][2];
+        if (J.bt) mma<true>(As, Bs, (J.nb + 3) & ~3, acc, tri);
+        else mma<false>(As, Bs, (J.nb + 3) & ~3, acc, tri);
+        store(J, cv, acc, Ct, ldct, Csm);
+        __syncthreads();
+    }
+    static __device__ __forceinline__ void run(const TileJob &J, int tri = 0, double *Ct = nullptr, long ldct = 0) {
+        run(J, tri, Ct, ldct, nullptr, []() {});
+    }
+};
+using Tile64 = Tile<64, 64>;
 
-// One tile product with its operands staged in regions 0 and 1. Operands are staged
-// first, so C may alias A or B (in-place panel solves).
-__device__ void tile_mma_dev(double *Cb, long ldc, int mr, int nc, const double *Ab, long lda, int ar,
-                             const double *Bb, long ldb, int bt, int bc, int nb, bool diag, int mode,
-                             double *Ct = nullptr, long ldct = 0, double *Csm = nullptr, int tri = 0) {
-    const TileJob J{Cb, ldc, mr, nc, Ab, lda, ar, Bb, ldb, bt, bc, nb, diag, mode};
-    double *As = region(0), *Bs = region(1);
-    stage_job(J, As, Bs);
-    double cv[4][2][2];
-    load_c(J, cv);  // while the operand copies are in flight
-    cpa_wait_all();
-    __syncthreads();
-    double acc[4][2][2];
-    dmma_tile(As, Bs, (nb + 3) & ~3, acc, tri);
-    store_tile(J, cv, acc, Ct, ldct, Csm);
-    __syncthreads();
+// A job's part of MR x NC at row r0 and column c0 of its tile; false when nothing of it is left.
+__device__ __forceinline__ bool sub_job(TileJob &J, int MR, int NC, int r0, int c0) {
+    if (J.diag && r0 + MR <= c0) return false;   // above the diagonal
+    J.mr = min(MR, J.mr - r0);
+    J.nc = min(NC, J.nc - c0);
+    if (J.mr <= 0 || J.nc <= 0) return false;
+    J.ar = J.mr;
+    J.bc = J.nc;
+    J.C += (size_t) r0 + (size_t) c0 * J.ldc;
+    J.A += r0;
+    J.B += J.bt ? (size_t) c0 : (size_t) c0 * J.ldb;
+    J.diag = J.diag && r0 < c0 + NC;
+    return true;
 }
 
 // Mode-0 jobs t0, t0 + step, ... (< t1) of one block, double buffered: the operands
@@ -523,25 +578,26 @@ __device__ void tile_stream(JobOf job_of, long t0, long t1, long step) {
     TileJob cur, nxt;
     job_of(t0, cur);
     int b = 0;
-    stage_job(cur, region(2 * b), region(2 * b + 1));
+    Tile64::stage(cur, region(2 * b), region(2 * b + 1));
     asm volatile("cp.async.commit_group;\n" ::);
     double cv[4][2][2], cvn[4][2][2];
-    load_c(cur, cv);
+    Tile64::load_c(cur, cv);
     for (long t = t0;; t += step) {
         const bool more = t + step < t1;
         if (more) {
             job_of(t + step, nxt);
-            stage_job(nxt, region(2 * (b ^ 1)), region(2 * (b ^ 1) + 1));
+            Tile64::stage(nxt, region(2 * (b ^ 1)), region(2 * (b ^ 1) + 1));
             asm volatile("cp.async.commit_group;\n" ::);
-            load_c(nxt, cvn);
+            Tile64::load_c(nxt, cvn);
             asm volatile("cp.async.wait_group 1;\n" ::);
         } else {
             asm volatile("cp.async.wait_group 0;\n" ::);
         }
         __syncthreads();
         double acc[4][2][2];
-        dmma_tile(region(2 * b), region(2 * b + 1), (cur.nb + 3) & ~3, acc);
-        store_tile(cur, cv, acc, nullptr, 0, nullptr);
+        if (cur.bt) Tile64::mma<true>(region(2 * b), region(2 * b + 1), (cur.nb + 3) & ~3, acc, 0);
+        else Tile64::mma<false>(region(2 * b), region(2 * b + 1), (cur.nb + 3) & ~3, acc, 0);
+        Tile64::store(cur, cv, acc, nullptr, 0, nullptr);
         __syncthreads();  // the buffer just read may be refilled
         if (!more) break;
         cur = nxt;
@@ -557,39 +613,46 @@ __device__ void tile_stream(JobOf job_of, long t0, long t1, long step) {
 }
 
 __device__ __forceinline__ void tri_index(long t, int &ti, int &tj) {
-    ti = (int) ((sqrt(8.0 * (double) t + 1.0) - 1.0) * 0.5);
+    ti = (int) ((sqrtf(8.0f * (float) t + 1.0f) - 1.0f) * 0.5f);   // settled by the loops below
     while ((long) ti * (ti + 1) / 2 > t) --ti;
     while ((long) (ti + 1) * (ti + 2) / 2 <= t) ++ti;
     tj = (int) (t - (long) ti * (ti + 1) / 2);
 }
 
-// Right-looking blocked Cholesky with one-panel look-ahead: in the update phase of
-// panel j, block 0 first updates the diagonal tile of panel j+1 and factors it while
-// the other blocks update the rest of the trailing matrix.
+// Right-looking blocked Cholesky with one-panel look-ahead: while the other blocks solve panel
+// j and update the trailing matrix with it, block 0 solves the panel's first chunk, updates the
+// diagonal block j + 1 with it and factors it.
 //
 // With K set, the inverse factor K = L^-1 (and KT = K^T) is formed alongside, right
 // looking by 64-row blocks, on the blocks that would otherwise wait for block 0:
-// while panel j is solved, the rows below block j-1 of K receive
+// before panel j, the rows below block j-1 of K receive
 // X(r, c) -= L(r, j-1) K(j-1, c) (the first update of a tile assigns -L K); while the
 // trailing matrix is updated, block row j is finalised as K(j, c) = Dinv_j X(j, c) and
 // K(j, j) = Dinv_j. The strictly upper blocks of K and the strictly lower blocks of KT
 // are never written (they must hold zeros).
-__device__ __forceinline__ void k_update_tile(const double *L, long ld, double *K, int n, int r, int c, int k) {
+//
+// A phase whose tiles would leave half the blocks idle takes them in quarters (32 x 32) or
+// halves: a 64 x 64 tile takes a block about 5 us (2.1 us of DMMA, 128 KB through the SM's L2
+// port), a quarter 2 us, so the line lies where the quarters need a second round.
+__device__ __forceinline__ TileJob k_update_job(const double *L, long ld, double *K, int n, int r, int c, int k) {
     const int mr = min(64, n - 64 * r);
-    tile_mma_dev(K + (size_t) 64 * r + (size_t) 64 * c * ld, ld, mr, 64, L + (size_t) 64 * r + (size_t) 64 * k * ld,
-                 ld, mr, K + (size_t) 64 * k + (size_t) 64 * c * ld, ld, 0, 64, 64, false, (k == c) ? 2 : 0);
+    return TileJob{K + (size_t) 64 * r + (size_t) 64 * c * ld, ld, mr, 64, L + (size_t) 64 * r + (size_t) 64 * k * ld,
+                   ld, mr, K + (size_t) 64 * k + (size_t) 64 * c * ld, ld, 0, 64, 64, false, (k == c) ? 2 : 0};
 }
 
+// part h of `parts` (1, or 2: column halves) of block (bj, c) of K's final form
 __device__ __forceinline__ void k_final_tile(const double *Dinv, long ldd, double *K, double *KT, long ld, int n,
-                                             int bj, int c) {
-    const int mr = min(64, n - 64 * bj);
+                                             int bj, int c, int h, int parts) {
+    const int mr = min(64, n - 64 * bj), c0 = 32 * h;
     if (c < bj) {
         double *X = K + (size_t) 64 * bj + (size_t) 64 * c * ld;
-        tile_mma_dev(X, ld, mr, 64, Dinv + (size_t) 64 * bj, ldd, mr, X, ld, 0, 64, mr, false, 1,
-                     KT + (size_t) 64 * c + (size_t) 64 * bj * ld, ld, nullptr, 2);
+        TileJob J{X, ld, mr, 64, Dinv + (size_t) 64 * bj, ldd, mr, X, ld, 0, 64, mr, false, 1};
+        double *Ct = KT + (size_t) (64 * c + c0) + (size_t) 64 * bj * ld;
+        if (parts == 1) Tile64::run(J, 2, Ct, ld);
+        else if (sub_job(J, 64, 32, 0, c0)) Tile<64, 32>::run(J, 2, Ct, ld);
     } else {
-        for (int idx = threadIdx.x; idx < 64 * 64; idx += blockDim.x) {
-            const int r = idx & 63, cc = idx >> 6;
+        for (int idx = threadIdx.x; idx < 64 * 64 / parts; idx += blockDim.x) {
+            const int r = idx & 63, cc = c0 + (idx >> 6);
             if (r < mr && cc < mr) {
                 const double v = Dinv[(size_t) (64 * bj + r) + (size_t) cc * ldd];
                 K[(size_t) (64 * bj + r) + (size_t) (64 * bj + cc) * ld] = v;
@@ -600,135 +663,247 @@ __device__ __forceinline__ void k_final_tile(const double *Dinv, long ldd, doubl
     }
 }
 
-// The factorisation on a grid of ngrid blocks, this one being block bid; gsync() is the
-// grid-wide barrier, garrive() / gwait(token) its two halves. The cooperative kernel runs it
-// on its grid; a batched launch runs it with one block per matrix (bid 0, ngrid 1, gsync a
-// block barrier). Every tile is computed by the same operations whatever the grid, so the
-// result does not depend on it.
-template <class GSync, class GArrive, class GWait>
-__device__ void potrf_body(double *L, long ld, int n, double *Dinv, long ldd, int *info, double *K, double *KT,
-                           int bid, int ngrid, GSync gsync, GArrive garrive, GWait gwait) {
+// The factorisation on a grid of ngrid blocks, this one being block bid, with the signals of
+// `sync` between them. The cooperative kernel runs it on its grid (ONE false, at least two
+// blocks: block 0 does the diagonal blocks and the rows that feed them and nothing else, the
+// others the rest); a batched launch runs it with one block per matrix (ONE, bid 0, ngrid 1).
+// Every tile is computed by the same operations whatever the grid, so the result does not
+// depend on it.
+//
+// Block 0 is the chain that sets the time, so it waits for the others only where it must: it
+// needs the last panel's updates (which are done long before it has finished the diagonal block
+// it is in), and the others need its diagonal blocks and its rows of the panel.
+template <bool ONE, class Sync>
+__device__ __forceinline__ void potrf_body(double *L, long ld, int n, double *Dinv, long ldd, int *info, double *K,
+                                           double *KT, int bid, int ngrid, Sync &sync) {
     const int nblk = (n + 63) / 64;
-    if (bid == 0) potf2_dev(L, ld, 0, min(NB, n), Dinv, ldd, info);
-    gsync();
-    for (int j0 = 0; j0 < n; j0 += NB) {
-        if (*(volatile int *) info) return;
-        const int nb = min(NB, n - j0);
-        const int rows = n - j0 - nb;
-        if (rows <= 0) break;
-        const int bj = j0 / 64;
-        double *P = L + (size_t) (j0 + nb) + (size_t) j0 * ld;
-        const int nchunk = (rows + 63) / 64;
-        const int pb = (j0 / 64) * 16 + (bid == 1 ? 8 : 0);
-        (void) pb;
-        if (bid <= 1) CHOL_STAMP(pb + 0);
-        // panel solve; with K, the update of K's rows r >= bj by block row bj - 1
+    const int nworker = ONE ? 1 : ngrid - 1, wid = ONE ? 0 : bid - 1;
+    for (int jn = 0; jn < n; jn += NB) {
+        // the next diagonal block starts at jn, the panel being finished at j0 = jn - 64
+        const bool first = jn == 0;
+        const int bj = jn / NB - 1;
+        // K's rows r >= bj are updated by block row bj - 1 before the diagonal block bj is waited
+        // for: they need only the other blocks' last updates
         const long nx = (K && bj >= 1) ? (long) (nblk - bj) * bj : 0;
-        // block 0 stages the next diagonal block now (its updates by earlier panels are
-        // complete) and keeps its own solved chunk 0, the rows that update that block
-        const int nbn = min(NB, rows);
-        if (bid == 0)
-            stage_tile(region(R_T), L + (size_t) (j0 + nb) + (size_t) (j0 + nb) * ld, ld, nbn, nbn, 64);
-        for (long t = bid; t < nchunk + nx; t += ngrid) {
-            if (t < nchunk) {
-                const int ch = (int) t;
-                const int mr = min(64, rows - ch * 64);
-                tile_mma_dev(P + ch * 64, ld, mr, nb, P + ch * 64, ld, mr, Dinv + j0, ldd, 1, nb, nb, false, 1,
-                             nullptr, 0, (t == 0) ? region(R_P) : nullptr, 1);
+        if ((ONE || bid > 0) && nx > 0) {
+            auto kjob = [&](long u) { return k_update_job(L, ld, K, n, bj + (int) (u / bj), (int) (u % bj), bj - 1); };
+            if (!ONE) sync.update_wait_all(bj);
+            if (2 * nx <= nworker) {
+                // half the blocks would stay idle: quarter tiles
+                for (long t = wid; t < 4 * nx; t += nworker) {
+                    TileJob J = kjob(t >> 2);
+                    if (sub_job(J, 32, 32, 32 * (int) (t & 1), 32 * (int) ((t >> 1) & 1))) Tile<32, 32>::run(J);
+                }
             } else {
-                const long u = t - nchunk;
-                k_update_tile(L, ld, K, n, bj + (int) (u / bj), (int) (u % bj), bj - 1);
+                tile_stream([&](long u, TileJob &J) { J = kjob(u); }, wid, nx, nworker);
             }
         }
-        if (bid <= 1) CHOL_STAMP(pb + 1);
-        // block 0 goes on to the next diagonal block, which needs only what it holds itself
-        // (its solved chunk 0 and the staged block): it arrives at the barrier without waiting,
-        // and waits for it only after that factorisation
-        const bool early = (bid == 0 && ngrid > 1);
-        unsigned int tok = 0;
-        if (early) tok = garrive();
-        else gsync();
-        if (bid <= 1) CHOL_STAMP(pb + 2);
-        const long ntile = (long) nchunk * (nchunk + 1) / 2;
-        const long nk = K ? bj + 1 : 0;
-        double *A22 = L + (size_t) (j0 + nb) + (size_t) (j0 + nb) * ld;
-        if (bid == 0) {
-            // tile (0, 0) is the next diagonal block: update it in shared memory and factor it
-            CHOL_STAMP(pb + 3);
-            potf2_dev(L, ld, j0 + nb, nbn, Dinv, ldd, info, true);
-            CHOL_STAMP(pb + 4);
+        if (!ONE && !first && bid > 0) sync.diag_wait(jn / NB);
+        if (!first && *(volatile int *) info) {
+            if (bid == 0) sync.diag_release(jn / NB);   // the others wait for it before they look
+            return;
         }
-        if (early) gwait(tok);
-        // remaining tiles (and K's block row bj), spread over the other blocks
-        // (block 0 joins when the grid has one block)
-        const int nworker = (ngrid > 1) ? (int) ngrid - 1 : 1;
-        const int wid = (ngrid > 1) ? (int) bid - 1 : 0;
-        if (wid >= 0) {
+        const int j0 = jn - NB, rows = n - jn, nchunk = (rows + 63) / 64, nbn = min(NB, rows);
+        double *P = L + (size_t) jn + (size_t) j0 * ld, *A22 = L + (size_t) jn + (size_t) jn * ld;
+        const int pb = bj * 16 + (bid == 1 ? 8 : 0);
+        (void) pb;
+        auto chunk = [&](int ch) {
+            const int mr = min(64, rows - ch * 64);
+            return TileJob{P + ch * 64, ld, mr, NB, P + ch * 64, ld, mr, Dinv + j0, ldd, 1, NB, NB, false, 1};
+        };
+        if (!first && bid <= 1) CHOL_STAMP(pb + 0);
+        if (ONE || bid == 0) {
+            if (!first) {
+                // the next diagonal block (its updates by earlier panels are complete) and chunk 0
+                // of the panel, the rows that update it
+                stage_tile(region(R_T), A22, ld, nbn, nbn, 64, true);
+                Tile64::run(chunk(0), 1, nullptr, 0, region(R_P), [&]() { sync.diag_release(jn / NB); });
+                if (bid <= 1) CHOL_STAMP(pb + 1);
+                if (!ONE) sync.panel_arrive();
+                if (bid <= 1) CHOL_STAMP(pb + 2);
+            }
+            potf2_dev(L, ld, jn, nbn, Dinv, ldd, info, !first, [&]() {
+                // the panel's updates by the other blocks, before the next panel
+                if (!ONE && !first) sync.update_wait(jn / NB);
+            });
+            if (!first && bid <= 1) CHOL_STAMP(pb + 4);
+        }
+        if (!first && (ONE || bid > 0)) {
+            // the rest of the panel, by half chunks where the blocks outnumber them
+            const int c1 = nchunk - 1;
+            if (2 * c1 <= nworker) {
+                for (int t = wid; t < 2 * c1; t += nworker) {
+                    TileJob J = chunk(1 + (t >> 1));
+                    const int r0 = 32 * (t & 1);
+                    J.mr = J.ar = min(32, J.mr - r0);
+                    J.C += r0;
+                    J.A += r0;
+                    if (J.mr > 0) Tile<32, 64>::run(J, 1);
+                }
+            } else {
+                for (int t = wid; t < c1; t += nworker) Tile64::run(chunk(1 + t), 1);
+            }
+            if (bid == 1) CHOL_STAMP(pb + 1);
+            if (!ONE) sync.panel_arrive();
+            sync.panel_wait(jn / NB);
+            if (bid == 1) CHOL_STAMP(pb + 2);
+            // the trailing matrix (tile 0 is the next diagonal block) and K's block row bj
+            const long ntile = (long) nchunk * (nchunk + 1) / 2, nk = K ? bj + 1 : 0;
             auto trailing = [&](long t, TileJob &J) {
                 int ti, tj;
                 tri_index(t, ti, tj);
                 const int mr = min(64, rows - ti * 64), nc = min(64, rows - tj * 64);
                 J = TileJob{A22 + (size_t) ti * 64 + (size_t) tj * 64 * ld, ld, mr, nc, P + ti * 64, ld, mr,
-                            P + tj * 64, ld, 1, nc, nb, ti == tj, 0};
+                            P + tj * 64, ld, 1, nc, NB, ti == tj, 0};
             };
-            tile_stream(trailing, 1 + wid, ntile, nworker);
-            for (long t = 1 + wid; t < ntile + nk; t += nworker)
-                if (t >= ntile) k_final_tile(Dinv, ldd, K, KT, ld, n, bj, (int) (t - ntile));
+            if (2 * (ntile - 1 + nk) <= nworker) {
+                const long nt4 = 4 * (ntile - 1);
+                for (long t = wid; t < nt4 + 2 * nk; t += nworker) {
+                    if (t < nt4) {
+                        TileJob J;
+                        trailing(1 + (t >> 2), J);
+                        if (sub_job(J, 32, 32, 32 * (int) (t & 1), 32 * (int) ((t >> 1) & 1))) Tile<32, 32>::run(J);
+                    } else {
+                        k_final_tile(Dinv, ldd, K, KT, ld, n, bj, (int) ((t - nt4) >> 1), (int) ((t - nt4) & 1), 2);
+                    }
+                }
+            } else {
+                tile_stream(trailing, 1 + wid, ntile, nworker);
+                for (long t = 1 + wid; t < ntile + nk; t += nworker)
+                    if (t >= ntile) k_final_tile(Dinv, ldd, K, KT, ld, n, bj, (int) (t - ntile), 0, 1);
+            }
+            if (bid == 1) CHOL_STAMP(pb + 3);
+            sync.update_arrive();
         }
-        if (bid == 1) CHOL_STAMP(pb + 3);
-        gsync();
-        if (bid <= 1) CHOL_STAMP(pb + 5);
+        if (!first && bid <= 1) CHOL_STAMP(pb + 5);
     }
+    if (bid > 0) sync.diag_wait(nblk);
+    else sync.diag_release(nblk);
     if (!K || *(volatile int *) info) return;
     // the last block row of K: its update by block row nblk - 2, then its final form
     const int bj = nblk - 1;
-    if (bj >= 1) {
-        for (int c = bid; c < bj; c += ngrid) k_update_tile(L, ld, K, n, bj, c, bj - 1);
-        gsync();
+    if (2 * bj <= ngrid) {
+        for (int t = bid; t < 4 * bj; t += ngrid) {
+            TileJob J = k_update_job(L, ld, K, n, bj, t >> 2, bj - 1);
+            if (sub_job(J, 32, 32, 32 * (t & 1), 32 * ((t >> 1) & 1))) Tile<32, 32>::run(J);
+        }
+        if (bj >= 1) sync.all();
+        for (int t = bid; t < 2 * (bj + 1); t += ngrid) k_final_tile(Dinv, ldd, K, KT, ld, n, bj, t >> 1, t & 1, 2);
+        return;
     }
-    for (int c = bid; c <= bj; c += ngrid) k_final_tile(Dinv, ldd, K, KT, ld, n, bj, c);
+    for (int c = bid; c < bj; c += ngrid) Tile64::run(k_update_job(L, ld, K, n, bj, c, bj - 1));
+    if (bj >= 1) sync.all();
+    for (int c = bid; c <= bj; c += ngrid) k_final_tile(Dinv, ldd, K, KT, ld, n, bj, c, 0, 1);
 }
 
-// Grid-wide barrier of a cooperative launch on a counter that starts at zero: every block adds
-// one per barrier and waits for the counter to reach the number of blocks times the barriers so
-// far. One thread of the last warp arrives and waits, so that the arrival of the block that goes
-// on to the diagonal block (a fence and an atomic, 1 us) runs beside the sweeps of the other
-// warps. The wait is bounded; on giving up it sets *info, which every block checks.
-struct GridBarrier {
-    unsigned *count;
+// The signals between the blocks of a cooperative launch: counters in global memory that start
+// at zero and only grow. One thread of a block (of warp 3, which has time to spare in the
+// diagonal blocks) signals and waits for all of it. Waits are bounded; a wait that gives up
+// sets *info, which every block checks after its waits.
+struct GridSync {
+    unsigned *c;    // 0: all(), 1: panel, 2: updates, 3: diagonal blocks done
     int *info;
-    unsigned target = 0;
-    static constexpr int kThread = COOP_THREADS - 32;
-    __device__ unsigned arrive() {
+    unsigned nall = 0;
+    static constexpr int kThread = 96;
+    __device__ __forceinline__ void add(int k) {
         __syncthreads();
-        target += gridDim.x;
         if (threadIdx.x == kThread) {
-            __threadfence();
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(c + k) : "memory");
         }
-        return target;
     }
-    __device__ void wait(unsigned t) {
-        if (threadIdx.x == kThread) {
-            unsigned v = 0;
-            long it = 0;
-            do {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-            } while ((int) (v - t) < 0 && ++it < (1L << 22));
-            if ((int) (v - t) < 0) *(volatile int *) info = -1;
-            __threadfence();
-        }
+    __device__ __forceinline__ void poll(int k, unsigned target) {   // one thread
+        unsigned v = 0;
+        long it = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(c + k) : "memory");
+        } while ((int) (v - target) < 0 && ++it < (1L << 22));
+        if ((int) (v - target) < 0) *(volatile int *) info = -1;
+    }
+    __device__ __forceinline__ void wait(int k, unsigned target) {
+        if (threadIdx.x == kThread) poll(k, target);
         __syncthreads();
     }
-    __device__ void sync() { wait(arrive()); }
+    // every block has finished its part of panel p (block 0 its chunk 0)
+    __device__ __forceinline__ void panel_arrive() { add(1); }
+    __device__ __forceinline__ void panel_wait(int p) { wait(1, (unsigned) p * gridDim.x); }
+    // the blocks beside block 0 have finished their updates by panel p (awaited by one thread of block 0)
+    __device__ __forceinline__ void update_arrive() { add(2); }
+    __device__ __forceinline__ void update_wait(int p) { poll(2, (unsigned) p * (gridDim.x - 1)); }
+    __device__ __forceinline__ void update_wait_all(int p) { wait(2, (unsigned) p * (gridDim.x - 1)); }
+    // block 0 has finished d diagonal blocks (and seen the updates before the last of them)
+    __device__ __forceinline__ void diag_release(int d) {   // after a block barrier
+        if (threadIdx.x == kThread) {
+            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(c + 3), "r"(d) : "memory");
+        }
+    }
+    __device__ __forceinline__ void diag_wait(int d) { wait(3, (unsigned) d); }
+    __device__ __forceinline__ void all() {
+        add(0);
+        wait(0, ++nall * gridDim.x);
+    }
 };
 
-__global__ void __launch_bounds__(COOP_THREADS, 1) potrf_coop_kernel(double *L, long ld, int n, double *Dinv,
-                                                                  long ldd, int *info, double *K, double *KT) {
-    GridBarrier bar{reinterpret_cast<unsigned *>(info + 1), info};
-    potrf_body(
-        L, ld, n, Dinv, ldd, info, K, KT, (int) blockIdx.x, (int) gridDim.x, [&]() { bar.sync(); },
-        [&]() { return bar.arrive(); }, [&](unsigned int t) { bar.wait(t); });
+// the same for a grid of one block
+struct BlockSync {
+    __device__ __forceinline__ void panel_arrive() {}
+    __device__ __forceinline__ void panel_wait(int) { __syncthreads(); }
+    __device__ __forceinline__ void update_arrive() { __syncthreads(); }
+    __device__ __forceinline__ void update_wait(int) {}
+    __device__ __forceinline__ void update_wait_all(int) {}
+    __device__ __forceinline__ void diag_release(int) {}
+    __device__ __forceinline__ void diag_wait(int) {}
+    __device__ __forceinline__ void all() { __syncthreads(); }
+};
+
+// sum_i log L_ii summed as the log-diagonal kernel sums it with its 1024 threads (terms v,
+// v + 1024, ... per thread, a shuffle tree per warp, then one over the 32 warp sums), by
+// COOP_THREADS threads each standing in for four: the same additions in the same order. The
+// sum is thread 0's.
+__device__ double logdiag_1024(int n, const double *L, long ld) {
+    __shared__ double red[32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    constexpr int kV = 1024 / COOP_THREADS;
+#pragma unroll
+    for (int q = 0; q < kV; ++q) {
+        double x = 0.0;
+        for (int v = t + COOP_THREADS * q; v < n; v += 1024) x += log(__ldcg(L + (size_t) v + (size_t) v * ld));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (lane == 0) red[w + (COOP_THREADS / 32) * q] = x;
+    }
+    __syncthreads();
+    double x = 0.0;
+    if (w == 0) {
+        x = red[lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    }
+    __syncthreads();
+    return x;
+}
+
+// The factor's status at the end of its kernel, by one block: the word *info and, with
+// `logdet`, sum log L_ii in the double after it, both also straight into the host's pinned
+// mirror when there is one.
+__device__ void write_status(int n, const double *L, long ld, int *info, double *hinfo, int logdet) {
+    double sum = 0.0;
+    if (logdet) sum = logdiag_1024(n, L, ld);
+    if (threadIdx.x != 0) return;
+    const int v = *(volatile int *) info;
+    if (logdet) reinterpret_cast<double *>(info)[1] = sum;
+    if (hinfo) {
+        reinterpret_cast<volatile int *>(hinfo)[0] = v;
+        if (logdet) hinfo[1] = sum;
+    }
+}
+
+__global__ void __launch_bounds__(COOP_THREADS, 1)
+    potrf_coop_kernel(double *L, long ld, int n, double *Dinv, long ldd, int *info, double *K, double *KT,
+                      double *hinfo, int logdet) {
+    GridSync sync{reinterpret_cast<unsigned *>(info) + kInfoCounters, info};
+    potrf_body<false>(L, ld, n, Dinv, ldd, info, K, KT, (int) blockIdx.x, (int) gridDim.x, sync);
+    // block 0 has the last word on *info: the others' waits end before its own work does
+    if (blockIdx.x == 0 && (logdet || hinfo)) write_status(n, L, ld, info, hinfo, logdet);
 }
 
 // Several factorisations in one launch, one CTA each: the copy of the lower triangle, the
@@ -748,32 +923,6 @@ struct SmallFactorBatch {
     SmallFactorJob job[kSmallBatch];
 };
 
-// sum_i log L_ii (n <= 1024) summed as the log-diagonal kernel sums it with its 1024
-// threads (one term per thread, a shuffle tree per warp, then one over the 32 warp sums),
-// by COOP_THREADS threads each standing in for four: the same additions in the same order.
-__device__ double logdiag_1024(int n, const double *L, long ld) {
-    __shared__ double red[32];
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    constexpr int kV = 1024 / COOP_THREADS;
-#pragma unroll
-    for (int q = 0; q < kV; ++q) {
-        const int v = t + COOP_THREADS * q;
-        double x = (v < n) ? log(L[(size_t) v + (size_t) v * ld]) : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if (lane == 0) red[w + (COOP_THREADS / 32) * q] = x;
-    }
-    __syncthreads();
-    double x = 0.0;
-    if (w == 0) {
-        x = red[lane];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    }
-    __syncthreads();
-    return x;
-}
-
 __device__ void small_factor_job(const SmallFactorJob &J) {
     const int n = J.n;
     for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
@@ -783,27 +932,11 @@ __device__ void small_factor_job(const SmallFactorJob &J) {
     if (threadIdx.x == 0) *J.info = 0;
     __threadfence_block();
     __syncthreads();
-    potrf_body(
-        J.L, J.ld, n, J.Dinv, J.ld, J.info, J.K, J.KT, 0, 1, []() { __syncthreads(); },
-        []() {
-            __syncthreads();
-            return 0u;
-        },
-        [](unsigned int) {});
+    BlockSync sync;
+    potrf_body<true>(J.L, J.ld, n, J.Dinv, J.ld, J.info, J.K, J.KT, 0, 1, sync);
+    __threadfence_block();
     __syncthreads();
-    double acc = 0.0;
-    if (J.logdet) {
-        __threadfence_block();
-        __syncthreads();
-        acc = logdiag_1024(n, J.L, J.ld);
-        if (threadIdx.x == 0) reinterpret_cast<double *>(J.info)[1] = acc;
-    }
-    if (threadIdx.x == 0) {
-        // the status words straight into the host's pinned mirror
-        const int v = *(volatile int *) J.info;
-        reinterpret_cast<volatile int *>(J.hinfo)[0] = v;
-        if (J.logdet) J.hinfo[1] = acc;
-    }
+    write_status(n, J.L, J.ld, J.info, J.hinfo, J.logdet);
 }
 
 __global__ void __launch_bounds__(COOP_THREADS, 1) potrf_small_batch_kernel(const SmallFactorBatch B) {
@@ -827,7 +960,7 @@ __global__ void __launch_bounds__(COOP_THREADS, 1) trtri_coop_kernel(const doubl
             // X_i chunk <- Dinv_i * X_i chunk  (in place)
             const int nc = min(64, cend - ch * 64);
             double *Xc = K + i0 + (size_t) ch * 64 * ld;
-            tile_mma_dev(Xc, ld, nb, nc, Dinv + i0, ldd, nb, Xc, ld, 0, nc, nb, false, 1, nullptr, 0, nullptr, 2);
+            Tile64::run(TileJob{Xc, ld, nb, nc, Dinv + i0, ldd, nb, Xc, ld, 0, nc, nb, false, 1}, 2);
         }
         grid.sync();
         const int rows = n - cend;
@@ -1064,12 +1197,15 @@ __global__ void __launch_bounds__(COOP_THREADS, 1)
     asm volatile("cp.async.wait_all;\n" ::);
 }
 
-__global__ void copy_lower_k(int n, const double *S, long lds, double *L, long ldl) {
-    const long total = (long) n * n;
-    for (long idx = blockIdx.x * (long) blockDim.x + threadIdx.x; idx < total; idx += (long) gridDim.x * blockDim.x) {
-        const int r = (int) (idx % n), c = (int) (idx / n);
+// L = the lower triangle of S; with info, the status words and the counters after them cleared
+__global__ void copy_lower_k(int n, const double *S, long lds, double *L, long ldl, int *info) {
+    if (info && blockIdx.x == 0 && threadIdx.x < kInfoBytes / 4) info[threadIdx.x] = 0;
+    const int r = (blockIdx.x % ((n + 255) / 256)) * 256 + threadIdx.x;
+    if (r >= n) return;
+    const int step = gridDim.x / ((n + 255) / 256);
+#pragma unroll 4
+    for (int c = blockIdx.x / ((n + 255) / 256); c < n; c += step)
         L[(size_t) r + (size_t) c * ldl] = (r >= c) ? S[(size_t) r + (size_t) c * lds] : 0.0;
-    }
 }
 
 __global__ void identity_k(int n, double *A, long lda) {
@@ -1079,9 +1215,6 @@ __global__ void identity_k(int n, double *A, long lda) {
         A[(size_t) r + (size_t) c * lda] = (r == c) ? 1.0 : 0.0;
     }
 }
-
-// the status word and the barrier counter after it
-__global__ void zero_info_k(int *p) { p[0] = p[1] = 0; }
 
 int sm_count() { return device_sm_count(); }
 
@@ -1109,16 +1242,31 @@ int grid_for_n(long total) {
 }
 }  // namespace
 
-bool coop_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS) {
+// blocks of copy_lower_k: a whole number of row ranges of 256, about four columns a thread
+static int copy_lower_grid(int n) {
+    const int rb = (n + 255) / 256;
+    return rb * std::max(1, std::min((n + 3) / 4, 148 * 16 / rb));
+}
+
+// `status`: the kernel also writes the status and sum log L_ii (d_info, and the pinned mirror
+// where it is mapped; *mirrored tells the caller that no copy is needed)
+bool coop_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS, bool status, bool *mirrored) {
     const int n = F.n;
-    zero_info_k<<<hb::counted(1), 1, 0, s>>>(F.d_info);
-    copy_lower_k<<<hb::counted(grid_for_n((long) n * n)), 256, 0, s>>>(n, S, ldS, F.L, F.ld);
+    copy_lower_k<<<hb::counted(copy_lower_grid(n)), 256, 0, s>>>(n, S, ldS, F.L, F.ld, F.d_info);
+    double *hinfo = nullptr;
+    if (status && cudaHostGetDevicePointer((void **) &hinfo, F.h_info, 0) != cudaSuccess) {
+        cudaGetLastError();
+        hinfo = nullptr;
+    }
+    if (mirrored) *mirrored = hinfo != nullptr;
+    int logdet = (status && F.stat_logdet) ? 1 : 0;
     const void *fn = (const void *) potrf_coop_kernel;
     const long t0 = (long) ((n - 1) / 64 + 1);
     // with the fused inverse, the update of K's rows needs up to t0^2 / 4 tiles per phase
     // at most one block per SM, so that the block factoring the diagonal never shares an SM
-    const long want = F.fuse_k ? t0 * (t0 + 1) / 2 + t0 * t0 / 4 : t0 * (t0 + 1) / 2;
-    const int grid = (int) std::max(1L, std::min<long>(std::min(coop_grid(fn), sm_count()), want));
+    // (four quarter tiles a tile where the blocks outnumber the tiles)
+    const long want = 1 + 4 * (F.fuse_k ? t0 * (t0 + 1) / 2 + t0 * t0 / 4 : t0 * (t0 + 1) / 2);
+    const int grid = (int) std::max(2L, std::min<long>(std::min(coop_grid(fn), sm_count()), want));
     double *Lp = F.L;
     long ld = F.ld;
     int nn = n;
@@ -1127,7 +1275,7 @@ bool coop_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, lon
     int *ip = F.d_info;
     double *Kp = F.fuse_k ? F.K : nullptr;
     double *KTp = F.fuse_k ? F.KT : nullptr;
-    void *args[] = {&Lp, &ld, &nn, &Dp, &ldd, &ip, &Kp, &KTp};
+    void *args[] = {&Lp, &ld, &nn, &Dp, &ldd, &ip, &Kp, &KTp, &hinfo, &logdet};
     const bool timed = kstat_on(F.kfamily);
     if (timed) kstat_begin(F.kfamily, s, (double) n * n * n / 3.0);
     cudaError_t e = cudaLaunchCooperativeKernel(fn, hb::counted(grid), COOP_THREADS, args, SM_DOUBLES * sizeof(double), s);
@@ -1148,7 +1296,7 @@ bool coop_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, lon
 // in a word of its own; the first failure (with its global pivot index) becomes the
 // factor's status.
 namespace {
-constexpr int kRecMaxLeaves = 128;
+constexpr int kRecMaxLeaves = 128;   // status words of kInfoBytes each
 struct RecLeaves {
     int off[kRecMaxLeaves];
     int count;
@@ -1158,7 +1306,7 @@ __global__ void rec_info_kernel(const RecLeaves R, const int *leaf_info, int *in
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     int v = 0;
     for (int q = 0; q < R.count && v == 0; ++q)
-        if (leaf_info[2 * q] != 0) v = leaf_info[2 * q] < 0 ? -1 : leaf_info[2 * q] + R.off[q];
+        if (const int w = leaf_info[kInfoBytes / 4 * q]) v = w < 0 ? -1 : w + R.off[q];
     *info = v;
 }
 
@@ -1190,11 +1338,11 @@ bool rec_leaf(cudaStream_t s, DenseFactor &F, int off, int n, double *Kp, double
     V.Dinv = F.Dinv + off;
     V.K = Kp;
     V.KT = KTp;
-    V.d_info = F.d_rec_info + 2 * R.count;
+    V.d_info = F.d_rec_info + kInfoBytes / 4 * R.count;
     V.fuse_k = true;
     V.kfamily = F.kfamily;
     R.off[R.count++] = off;
-    return coop_factorize_enqueue(s, V, V.L, F.ld);
+    return coop_factorize_enqueue(s, V, V.L, F.ld, false, nullptr);
 }
 
 bool rec_factor(cudaStream_t s, DenseFactor &F, int off, int n, RecLeaves &R) {
@@ -1253,7 +1401,7 @@ bool rec_factor_nok(cudaStream_t s, DenseFactor &F, int off, int n, RecLeaves &R
 
 bool rec_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS) {
     const int n = F.n;
-    if (!F.d_rec_info && hb::cmalloc(&F.d_rec_info, 2 * sizeof(int) * kRecMaxLeaves) != cudaSuccess) {
+    if (!F.d_rec_info && hb::cmalloc(&F.d_rec_info, kInfoBytes * kRecMaxLeaves) != cudaSuccess) {
         F.d_rec_info = nullptr;
         return false;
     }
@@ -1261,8 +1409,8 @@ bool rec_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long
         F.d_rec_w = nullptr;
         return false;
     }
-    HB_CUDA(cudaMemsetAsync(F.d_rec_info, 0, 2 * sizeof(int) * kRecMaxLeaves, s));
-    copy_lower_k<<<hb::counted(grid_for_n((long) n * n)), 256, 0, s>>>(n, S, ldS, F.L, F.ld);
+    HB_CUDA(cudaMemsetAsync(F.d_rec_info, 0, kInfoBytes * kRecMaxLeaves, s));
+    copy_lower_k<<<hb::counted(copy_lower_grid(n)), 256, 0, s>>>(n, S, ldS, F.L, F.ld, nullptr);
     RecLeaves R;
     R.count = 0;
     const bool ok = rec_factor(s, F, 0, n, R);
@@ -1274,7 +1422,7 @@ bool rec_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long
 bool rec_factorize_nok_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS) {
     const int n = F.n;
     const size_t strip = (size_t) F.ld * kRecLeafMaxN;
-    if (!F.d_rec_info && hb::cmalloc(&F.d_rec_info, 2 * sizeof(int) * kRecMaxLeaves) != cudaSuccess) {
+    if (!F.d_rec_info && hb::cmalloc(&F.d_rec_info, kInfoBytes * kRecMaxLeaves) != cudaSuccess) {
         F.d_rec_info = nullptr;
         return false;
     }
@@ -1294,8 +1442,8 @@ bool rec_factorize_nok_enqueue(cudaStream_t s, DenseFactor &F, const double *S, 
         HB_CUDA(cudaMemsetAsync(F.d_rec_ks, 0, sizeof(double) * strip, s));
         HB_CUDA(cudaMemsetAsync(F.d_rec_kts, 0, sizeof(double) * strip, s));
     }
-    HB_CUDA(cudaMemsetAsync(F.d_rec_info, 0, 2 * sizeof(int) * kRecMaxLeaves, s));
-    copy_lower_k<<<hb::counted(grid_for_n((long) n * n)), 256, 0, s>>>(n, S, ldS, F.L, F.ld);
+    HB_CUDA(cudaMemsetAsync(F.d_rec_info, 0, kInfoBytes * kRecMaxLeaves, s));
+    copy_lower_k<<<hb::counted(copy_lower_grid(n)), 256, 0, s>>>(n, S, ldS, F.L, F.ld, nullptr);
     RecLeaves R;
     R.count = 0;
     const bool ok = rec_factor_nok(s, F, 0, n, R);

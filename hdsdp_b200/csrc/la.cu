@@ -842,7 +842,7 @@ void DenseFactor::alloc(int n_, int fuse_inverse) {
     HB_CUDA(hb::cmalloc(&L, sizeof(double) * ld * n));
     HB_CUDA(hb::cmalloc(&Dinv, sizeof(double) * ld * NB));
     // the info word and, 8 bytes on, sum log L_ii of the last factorisation
-    HB_CUDA(hb::cmalloc(&d_info, 2 * sizeof(double)));
+    HB_CUDA(hb::cmalloc(&d_info, kInfoBytes));
     HB_CUDA(hb::cmalloc_host(&h_info, 2 * sizeof(double)));
     *h_info = 0;
     stat_logdet = true;
@@ -899,7 +899,7 @@ static void ensure_attrs() {
     });
 }
 
-bool coop_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS);
+bool coop_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS, bool status, bool *mirrored);
 bool rec_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS);
 bool rec_factorize_nok_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS);
 bool coop_inverse_enqueue(cudaStream_t s, DenseFactor &F);
@@ -930,9 +930,12 @@ void factorize_async(cudaStream_t s, DenseFactor &F, const double *S, long ldS) 
         status_copy();
         return;
     }
-    if (coop_factorize_enqueue(s, F, S, ldS)) {
+    bool mirrored = false;
+    if (coop_factorize_enqueue(s, F, S, ldS, true, &mirrored)) {
         F.k_pending = F.fuse_k && F.K && F.KT;
-        status_copy();
+        if (!mirrored)
+            HB_CUDA(cudaMemcpyAsync(F.h_info, F.d_info, F.stat_logdet ? 2 * sizeof(double) : sizeof(int),
+                                    cudaMemcpyDeviceToHost, s));
         return;
     }
     zero_int_kernel<<<hb::counted(1), 1, 0, s>>>(F.d_info);

@@ -93,6 +93,10 @@ constexpr int kRecLeafMaxN = 2560;
 // recursive): order 6016 5.62 / 6.67, 8000 11.8 / 11.7, 12000 36.8 / 31.2, 16000 83.9 / 64.4.
 constexpr int kRecNoKMinN = 8192;
 
+// A factor's status words on the device: the info word, 8 bytes on sum log L_ii, then the
+// cooperative kernel's counters (from int kInfoCounters on), cleared by every factorisation.
+constexpr int kInfoBytes = 32, kInfoCounters = 4;
+
 struct DenseFactor {
     int n = 0;
     long ld = 0;
@@ -100,11 +104,11 @@ struct DenseFactor {
     double *Dinv = nullptr;   // n x 64 (block b at rows [64b, 64b+64))
     double *K = nullptr;
     double *KT = nullptr;
-    int *d_info = nullptr;    // device: 0 = success, k > 0 = pivot k failed
+    int *d_info = nullptr;    // device: 0 = success, k > 0 = pivot k failed, -1 = a wait gave up (kInfoBytes)
     int *h_info = nullptr;    // pinned host mirror
-    // With stat_logdet set (the default; alloc() makes d_info and h_info 16 bytes each), a
-    // factorisation also writes sum log L_ii next to the info word and both come back in one
-    // copy; factor_status() then holds log det = 2 sum log L_ii in `logdet`.
+    // With stat_logdet set (the default; alloc() makes h_info 16 bytes), a factorisation also
+    // writes sum log L_ii next to the info word, on the device and in h_info; factor_status()
+    // then holds log det = 2 sum log L_ii in `logdet`.
     bool stat_logdet = true;
     bool logdet_valid = false;
     double logdet = 0.0;

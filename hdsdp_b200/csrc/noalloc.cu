@@ -38,7 +38,7 @@ namespace {
 constexpr int kMaxN = HDSDPB_NOALLOC_MAX_N;
 constexpr long kLd = kMaxN;  // pad_ld(256) = 256
 constexpr size_t kMatDoubles = (size_t) kLd * kMaxN;
-constexpr size_t kScratchDoubles = 2 * kMatDoubles + (size_t) kLd * 64 + 2;
+constexpr size_t kScratchDoubles = 2 * kMatDoubles + (size_t) kLd * 64 + 1 + kInfoBytes / sizeof(double);
 
 static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
