@@ -1870,111 +1870,191 @@ __global__ void __launch_bounds__(kLzThreads, 1)
     }
 }
 
-// ---- Lanczos for blocks of order <= kSmallLanczosN: one CTA holds K = L^-1, D and the
-// Lanczos basis in shared memory and runs every step in one launch (the stepwise path
-// spends four launches per step, which dominates for small blocks).
+// ---- Lanczos for blocks of order <= kSmallLanczosN: one CTA runs every step in one launch
+// (the stepwise path spends four launches per step, which dominates for small blocks).
+//
+// It forms the operator M = K (-D) K^T once, by DMMA, and keeps it in registers: warp w holds
+// rows 8w .. 8w + 7 as accumulators. A step is then one product, for which only the vector is
+// read from shared memory, and the recurrence, which warp 0 takes on vectors in its registers:
+// two block barriers. With K and D in shared memory and three products a step it was bound by
+// shared-memory reads and shuffles. 30 steps at order 50 / 80: 230 / 322 us with 8 warps, one a
+// column, 47 / 52 us now (M itself is n^3 FMAs, 2 to 8 us on one SM).
 constexpr int kSmallLanczosN = kSmallLanczosMaxN;
+constexpr int kSmallBlocks = kSmallLanczosN / 8;              // 8-row blocks
+constexpr int kSmallLanczosThreads = 32 * kSmallBlocks;
+constexpr int kSmallPitch = kSmallLanczosN + 4;               // 4 modulo 16: conflict-free fragments
+constexpr int kSmallRitzThreads = 1024;
 
 __host__ __device__ inline int small_ld(int n) { return n | 1; }  // odd stride: fewer bank conflicts
 
-inline size_t small_lanczos_smem(int n, int maxdim) {
-    return sizeof(double) * ((size_t) 2 * n * small_ld(n) + (size_t) (maxdim + 1) * n + 4 * (size_t) n);
+inline size_t small_lanczos_smem(int n) {
+    return sizeof(double) * ((size_t) 2 * (((n + 7) / 8) * 8) * kSmallPitch + 2 * kSmallLanczosN);
+}
+inline size_t small_ritz_smem(int n) { return sizeof(double) * ((size_t) 2 * n * small_ld(n) + 4 * (size_t) n); }
+
+__device__ __forceinline__ void lz_dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// sum over a warp of three entries a lane
+__device__ __forceinline__ double sum96(const double (&x)[3]) { return warp_sum((x[0] + x[1]) + x[2]); }
+
+// Start vector v0 = normalise(a + b) (a may be null), then maxdim steps of the
+// three-term recurrence as lanczos_orth_kernel takes them; the basis V (all maxdim + 1
+// columns, zero past a breakdown) and alpha / beta go to global memory.
+__device__ void lanczos_small_body(int n, const double *K, long ldk, const double *D, long ldD, const double *a,
+                                   const double *b, double *V, long ldv, double *ab, int maxdim) {
+    static_assert(kSmallLanczosN == 96, "three entries a lane, twelve row blocks");
+    extern __shared__ double sm[];
+    constexpr int P = kSmallPitch;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fc = lane & 3;
+    const int nb = (n + 7) / 8, np = 8 * nb;
+    double *sK = sm, *sD = sK + np * P, *sv = sD + np * P, *sw = sv + kSmallLanczosN;
+    for (int j = warp; j < np; j += kSmallBlocks)
+        for (int i = lane; i < np; i += 32) {
+            const bool in = i < n && j < n;
+            sK[i + j * P] = (in && i >= j) ? K[(size_t) i + (size_t) j * ldk] : 0.0;
+            sD[i + j * P] = in ? D[(size_t) i + (size_t) j * ldD] : 0.0;
+        }
+    if (threadIdx.x < kSmallLanczosN) sv[threadIdx.x] = sw[threadIdx.x] = 0.0;
+    __syncthreads();
+    double M[kSmallBlocks][2];
+#pragma unroll
+    for (int j = 0; j < kSmallBlocks; ++j) M[j][0] = M[j][1] = 0.0;
+    if (warp < nb) {
+        // this warp's rows of K D, then of (K D) K^T; an accumulator pair is an operand as it
+        // stands, register h being column 2 fc + h
+        double T[kSmallBlocks][2];
+#pragma unroll
+        for (int j = 0; j < kSmallBlocks; ++j) T[j][0] = T[j][1] = 0.0;
+        for (int k = 0; k <= warp; ++k) {
+            const double a0 = sK[8 * warp + fr + (8 * k + fc) * P], a1 = sK[8 * warp + fr + (8 * k + fc + 4) * P];
+#pragma unroll
+            for (int j = 0; j < kSmallBlocks; ++j) {
+                if (j >= nb) break;
+                lz_dmma(T[j], a0, sD[8 * j + fr + (8 * k + fc) * P]);
+                lz_dmma(T[j], a1, sD[8 * j + fr + (8 * k + fc + 4) * P]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kSmallBlocks; ++k) {
+            if (k >= nb) break;
+#pragma unroll
+            for (int j = k; j < kSmallBlocks; ++j) {
+                if (j >= nb) break;
+                lz_dmma(M[j], -T[k][0], sK[8 * j + fr + (8 * k + 2 * fc) * P]);
+                lz_dmma(M[j], -T[k][1], sK[8 * j + fr + (8 * k + 2 * fc + 1) * P]);
+            }
+        }
+    }
+    // v_k and v_{k-1} in warp 0
+    double v[3], vp[3] = {}, x[3], q[3];
+    if (warp == 0) {
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            const int i = lane + 32 * m;
+            v[m] = (i < n) ? (a ? a[i] : 0.0) + b[i] : 0.0;
+            q[m] = v[m] * v[m];
+        }
+        const double nrm = sqrt(sum96(q));
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            const int i = lane + 32 * m;
+            v[m] = (nrm > 0.0) ? v[m] / nrm : 0.0;
+            if (i < n) sv[i] = V[i] = v[m];
+        }
+        if (lane < 2) ab[2 * maxdim + lane] = 0.0;
+    }
+    double betaPrev = 0.0;
+    for (int k = 0; k < maxdim; ++k) {
+        __syncthreads();
+        if (warp < nb) {
+            double p0 = 0.0, p1 = 0.0, p2 = 0.0, p3 = 0.0;
+#pragma unroll
+            for (int j = 0; j < kSmallBlocks; j += 2) {   // (M and v are zero past the order)
+                const double2 y0 = *reinterpret_cast<const double2 *>(sv + 8 * j + 2 * fc);
+                const double2 y1 = *reinterpret_cast<const double2 *>(sv + 8 * (j + 1) + 2 * fc);
+                p0 += M[j][0] * y0.x;
+                p1 += M[j][1] * y0.y;
+                p2 += M[j + 1][0] * y1.x;
+                p3 += M[j + 1][1] * y1.y;
+            }
+            double w = (p0 + p1) + (p2 + p3);
+            w += __shfl_xor_sync(0xffffffffu, w, 1);
+            w += __shfl_xor_sync(0xffffffffu, w, 2);
+            if (fc == 0) sw[8 * warp + fr] = w;
+        }
+        __syncthreads();
+        if (warp > 0) continue;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            x[m] = sw[lane + 32 * m];
+            if (k > 0) x[m] -= betaPrev * vp[m];
+            q[m] = x[m] * v[m];
+        }
+        const double alp = sum96(q);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            x[m] -= alp * v[m];
+            q[m] = x[m] * x[m];
+        }
+        const double nrm = sqrt(sum96(q));
+        betaPrev = (nrm > 0.0) ? nrm : 0.0;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            const int i = lane + 32 * m;
+            vp[m] = v[m];
+            v[m] = (nrm > 0.0) ? x[m] / nrm : 0.0;
+            if (i < n) sv[i] = V[(size_t) i + (size_t) (k + 1) * ldv] = v[m];
+        }
+        if (lane == 0) {
+            ab[k] = alp;
+            ab[maxdim + k] = betaPrev;
+        }
+    }
 }
 
 // K (lower, leading dimension ldk) and D into shared memory (leading dimension small_ld(n))
 __device__ void small_load(int n, const double *K, long ldk, const double *D, long ldD, double *sK, double *sD) {
-    const int ls = small_ld(n);
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int i = e % n, j = e / n;
-        sK[i + j * ls] = (i >= j) ? K[(size_t) i + (size_t) j * ldk] : 0.0;
-        sD[i + j * ls] = D[(size_t) i + (size_t) j * ldD];
-    }
+    const int ls = small_ld(n), lane = threadIdx.x & 31;
+    for (int j = threadIdx.x >> 5; j < n; j += blockDim.x >> 5)
+        for (int i = lane; i < n; i += 32) {
+            sK[i + j * ls] = (i >= j) ? K[(size_t) i + (size_t) j * ldk] : 0.0;
+            sD[i + j * ls] = D[(size_t) i + (size_t) j * ldD];
+        }
     __syncthreads();
 }
 
-// y = K (-D) (K^T x), one warp per output entry
+// y = K (-D) (K^T x), eight lanes an output entry, every entry at once; ends with a block
+// barrier. Lane q of eight forms the partial sums l = q, q + 8, q + 16, q + 24 of 32 (rows
+// first + l, + 32, + 64) and adds them as a 32-lane shuffle tree would; a whole warp an entry
+// spends 10 shuffles on each.
 __device__ void small_mv(int n, const double *sK, const double *sD, const double *x, double *t, double *u,
                          double *y) {
-    const int ls = small_ld(n), lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int i = warp; i < n; i += nw) {  // t = K^T x
-        double a = 0.0;
-        for (int k = i + lane; k < n; k += 32) a += sK[k + i * ls] * x[k];
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) t[i] = a;
-    }
-    __syncthreads();
-    for (int i = warp; i < n; i += nw) {  // u = -D t
-        double a = 0.0;
-        for (int k = lane; k < n; k += 32) a += sD[k + i * ls] * t[k];
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) u[i] = -a;
-    }
-    __syncthreads();
-    for (int i = warp; i < n; i += nw) {  // y = K u
-        double a = 0.0;
-        for (int k = lane; k <= i; k += 32) a += sK[i + k * ls] * u[k];
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) y[i] = a;
-    }
-    __syncthreads();
-}
-
-// Start vector v0 = normalise(a + b) (a may be null), then maxdim steps of the
-// three-term recurrence exactly as lanczos_orth_kernel takes them; the basis V (all
-// maxdim + 1 columns, zero past a breakdown) and alpha / beta go to global memory.
-__device__ void lanczos_small_body(int n, const double *K, long ldk, const double *D, long ldD, const double *a,
-                                   const double *b, double *V, long ldv, double *ab, int maxdim) {
-    extern __shared__ double sm[];
-    const int ls = small_ld(n);
-    double *sK = sm, *sD = sK + (size_t) n * ls, *sV = sD + (size_t) n * ls, *w = sV + (size_t) (maxdim + 1) * n;
-    double *t = w + n, *u = t + n, *sab = u + n;  // sab: 2 * maxdim + 2 <= 4n is not guaranteed: kept in ab
-    (void) sab;
-    small_load(n, K, ldk, D, ldD, sK, sD);
-    for (int e = threadIdx.x; e < (maxdim + 1) * n; e += blockDim.x) sV[e] = 0.0;
-    for (int e = threadIdx.x; e < 2 * maxdim + 2; e += blockDim.x) ab[e] = 0.0;
-    __syncthreads();
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double x = (a ? a[i] : 0.0) + b[i];
-        sV[i] = x;
-        acc += x * x;
-    }
-    double nrm = sqrt(bsum(acc));
-    for (int i = threadIdx.x; i < n; i += blockDim.x) sV[i] = (nrm > 0.0) ? sV[i] / nrm : 0.0;
-    __syncthreads();
-    double betaPrev = 0.0;
-    for (int k = 0; k < maxdim; ++k) {
-        const double *vk = sV + (size_t) k * n;
-        small_mv(n, sK, sD, vk, t, u, w);
-        if (k > 0) {
-            const double *vp = sV + (size_t) (k - 1) * n;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) w[i] -= betaPrev * vp[i];
-            __syncthreads();
-        }
-        acc = 0.0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) acc += w[i] * vk[i];
-        const double alp = bsum(acc);
-        acc = 0.0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            const double x = w[i] - alp * vk[i];
-            w[i] = x;
-            acc += x * x;
-        }
-        nrm = sqrt(bsum(acc));
-        if (threadIdx.x == 0) ab[k] = alp;
-        betaPrev = 0.0;
-        if (nrm > 0.0) {
-            double *vn = sV + (size_t) (k + 1) * n;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) vn[i] = w[i] / nrm;
-            if (threadIdx.x == 0) ab[maxdim + k] = nrm;
-            betaPrev = nrm;
-        }
+    static_assert(kSmallRitzThreads / 8 >= kSmallLanczosN && kSmallLanczosN <= 96, "one pass");
+    const int ls = small_ld(n), i = threadIdx.x >> 3, q = threadIdx.x & 7;
+    // out[i] = sign * sum over first(i) <= k < end(i) of A[k ks + i is] v[k]
+    auto product = [&](const double *A, int ks, int is, const double *v, double *out, int mode, double sign) {
+        double p[4] = {};
+        const int k0 = (mode == 1 ? i : 0) + q, k1 = (i < n) ? (mode == 2 ? i + 1 : n) : 0;
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const int k = k0 + 8 * h + 32 * r;
+                if (k < k1) p[h] += A[k * ks + i * is] * v[k];
+            }
+        double acc = (p[0] + p[2]) + (p[1] + p[3]);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (q == 0 && i < n) out[i] = sign * acc;
         __syncthreads();
-    }
-    for (int e = threadIdx.x; e < (maxdim + 1) * n; e += blockDim.x) {
-        const int i = e % n, j = e / n;
-        V[(size_t) i + (size_t) j * ldv] = sV[e];
-    }
+    };
+    product(sK, 1, ls, x, t, 1, 1.0);    // t = K^T x
+    product(sD, 1, ls, t, u, 0, -1.0);   // u = -D t
+    product(sK, ls, 1, u, y, 2, 1.0);    // y = K u
 }
 
 // The Ritz part of a converged check: z1 = V y1, z2 = M z1 (warm <- z2),
@@ -2007,12 +2087,12 @@ __device__ void lanczos_small_ritz_body(int n, const double *K, long ldk, const 
     }
 }
 
-__global__ void lanczos_small_kernel(int n, const double *K, long ldk, const double *D, long ldD, const double *a,
+__global__ void __launch_bounds__(kSmallLanczosThreads) lanczos_small_kernel(int n, const double *K, long ldk, const double *D, long ldD, const double *a,
                                      const double *b, double *V, long ldv, double *ab, int maxdim) {
     lanczos_small_body(n, K, ldk, D, ldD, a, b, V, ldv, ab, maxdim);
 }
 
-__global__ void lanczos_small_ritz_kernel(int n, const double *K, long ldk, const double *D, long ldD,
+__global__ void __launch_bounds__(kSmallRitzThreads) lanczos_small_ritz_kernel(int n, const double *K, long ldk, const double *D, long ldD,
                                           const double *V, long ldv, int kp1, const double *y, double lam,
                                           double *warm, double *out) {
     lanczos_small_ritz_body(n, K, ldk, D, ldD, V, ldv, kp1, y, lam, warm, out);
@@ -2026,6 +2106,7 @@ struct LzStepJob {
     double *V, *ab, *hab;
     long ldk, ldD, ldv;
     int n, maxdim;
+    static constexpr int kThreads = kSmallLanczosThreads;
 };
 struct LzRitzJob {
     const double *K, *D, *V, *y;
@@ -2033,6 +2114,7 @@ struct LzRitzJob {
     long ldk, ldD, ldv;
     double lam;
     int n, kp1;
+    static constexpr int kThreads = kSmallRitzThreads;
 };
 constexpr int kLzBatch = 32;
 constexpr int kLzHostParallel = 8;   // cones from which the host replays run on several threads
@@ -2057,8 +2139,8 @@ __device__ void lz_run(const LzRitzJob &J) {
         if (threadIdx.x < 2) J.hout[threadIdx.x] = J.out[threadIdx.x];
     }
 }
-template <class Job> __global__ void lz_pack_kernel(const LzPack<Job> B) { lz_run(B.job[blockIdx.x]); }
-template <class Job> __global__ void lz_array_kernel(const Job *__restrict__ jobs) { lz_run(jobs[blockIdx.x]); }
+template <class Job> __global__ void __launch_bounds__(Job::kThreads) lz_pack_kernel(const LzPack<Job> B) { lz_run(B.job[blockIdx.x]); }
+template <class Job> __global__ void __launch_bounds__(Job::kThreads) lz_array_kernel(const Job *__restrict__ jobs) { lz_run(jobs[blockIdx.x]); }
 
 // one launch over every job: by value when they fit the parameters, else from a device copy
 // kept per host thread, device and job type (stream-ordered behind the launches before it)
@@ -2068,7 +2150,7 @@ template <class Job> void lz_launch(cudaStream_t s, const std::vector<Job> &jobs
     if (count <= kLzBatch) {
         LzPack<Job> B;
         for (int q = 0; q < count; ++q) B.job[q] = jobs[q];
-        lz_pack_kernel<Job><<<hb::counted(count), 256, smem, s>>>(B);
+        lz_pack_kernel<Job><<<hb::counted(count), Job::kThreads, smem, s>>>(B);
         HB_CUDA(cudaGetLastError());
         return;
     }
@@ -2086,7 +2168,7 @@ template <class Job> void lz_launch(cudaStream_t s, const std::vector<Job> &jobs
         b.cap = jobs.size();
     }
     HB_CUDA(cudaMemcpyAsync(b.p, jobs.data(), sizeof(Job) * jobs.size(), cudaMemcpyHostToDevice, s));
-    lz_array_kernel<Job><<<hb::counted(count), 256, smem, s>>>(b.p);
+    lz_array_kernel<Job><<<hb::counted(count), Job::kThreads, smem, s>>>(b.p);
     HB_CUDA(cudaGetLastError());
 }
 template <class Job> void lz_allow_smem(int bytes) {
@@ -2233,13 +2315,13 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
     if (small) {
         static std::atomic<unsigned long long> attr{0};
         once_per_device(attr, [] {
-            const int bytes = (int) small_lanczos_smem(kSmallLanczosN, 30);
-            HB_CUDA(cudaFuncSetAttribute((const void *) lanczos_small_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+            HB_CUDA(cudaFuncSetAttribute((const void *) lanczos_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int) small_lanczos_smem(kSmallLanczosN)));
             HB_CUDA(cudaFuncSetAttribute((const void *) lanczos_small_ritz_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int) small_ritz_smem(kSmallLanczosN)));
         });
-        lanczos_small_kernel<<<hb::counted(1), 256, small_lanczos_smem(n, maxdim), s>>>(
+        lanczos_small_kernel<<<hb::counted(1), kSmallLanczosThreads, small_lanczos_smem(n), s>>>(
             n, F.K, F.ld, D, ldD, nComputed == 0 ? nullptr : warm, nComputed == 0 ? init_vec : pert_vec, V, ld, d_ab,
             maxdim);
         HB_CUDA(cudaGetLastError());
@@ -2371,7 +2453,7 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
         }
         HB_CUDA(cudaMemcpyAsync(d_y, yy.data(), sizeof(double) * 2 * kp1, cudaMemcpyHostToDevice, s));
         if (small) {
-            lanczos_small_ritz_kernel<<<hb::counted(1), 256, small_lanczos_smem(n, maxdim), s>>>(
+            lanczos_small_ritz_kernel<<<hb::counted(1), kSmallRitzThreads, small_ritz_smem(n), s>>>(
                 n, F.K, F.ld, D, ldD, V, ld, kp1, d_y, eigMin1, warm, d_scal);
             HB_CUDA(cudaGetLastError());
             if (tm) tm->n_lanczos_mv += 2;
@@ -2512,21 +2594,16 @@ void lanczos_small_batch(std::vector<LzTask> &tasks) {
     Timers *tm = tasks[0].tm;
     static std::atomic<unsigned long long> attr{0};
     once_per_device(attr, [] {
-        const int bytes = (int) small_lanczos_smem(kSmallLanczosN, 30);
-        lz_allow_smem<LzStepJob>(bytes);
-        lz_allow_smem<LzRitzJob>(bytes);
+        lz_allow_smem<LzStepJob>((int) small_lanczos_smem(kSmallLanczosN));
+        lz_allow_smem<LzRitzJob>((int) small_ritz_smem(kSmallLanczosN));
     });
     for (LzTask &t : tasks) {
         t.ret = HDSDP_RETCODE_OK;
         compute_inverse_factor(s, *t.F);
     }
     if (tm) tm->lz_inverse += wall() - t0;   // enqueue time: the steps' launch follows without a wait
-    int maxn = 0, maxdim = 0;
-    for (LzTask &t : tasks) {
-        maxn = std::max(maxn, t.lz->n);
-        maxdim = std::max(maxdim, t.lz->maxdim);
-    }
-    const size_t smem = small_lanczos_smem(maxn, maxdim);
+    int maxn = 0;
+    for (LzTask &t : tasks) maxn = std::max(maxn, t.lz->n);
     // device addresses of the pinned mirrors (alpha / beta and the Ritz residuals), which
     // the kernels write directly; a task without one gets copies
     std::vector<double *> hab(tasks.size()), hsc(tasks.size());
@@ -2540,7 +2617,7 @@ void lanczos_small_batch(std::vector<LzTask> &tasks) {
                              L.nComputed == 0 ? L.init_vec : L.pert_vec, L.V, L.d_ab, hab[q], t.F->ld, t.ldD,
                              L.ld, L.n, L.maxdim};
     }
-    lz_launch(s, steps, smem);
+    lz_launch(s, steps, small_lanczos_smem(maxn));
     for (size_t q = 0; q < tasks.size(); ++q) {
         Lanczos &L = *tasks[q].lz;
         if (!hab[q])
@@ -2569,7 +2646,7 @@ void lanczos_small_batch(std::vector<LzTask> &tasks) {
             ritz[q] = LzRitzJob{R.t->F->K, R.t->D, L.V, L.dm_yv ? L.dm_yv : L.d_y, L.warm, L.d_scal,
                                 hsc[R.t - tasks.data()], R.t->F->ld, R.t->ldD, L.ld, R.eigMin1, L.n, R.kc + 1};
         }
-        lz_launch(s, ritz, smem);
+        lz_launch(s, ritz, small_ritz_smem(maxn));
         for (LzRun *R : want) {
             Lanczos &L = *R->t->lz;
             if (!hsc[R->t - tasks.data()])
