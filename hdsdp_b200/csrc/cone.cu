@@ -1870,6 +1870,289 @@ __global__ void __launch_bounds__(kLzThreads, 1)
     }
 }
 
+// ---- Lanczos for blocks above the one-CTA kernel up to order kLzClusterMaxN: one cluster of 16
+// CTAs holds the columns of K, K^T and D in its shared memory (as the cooperative variant does
+// over the whole grid) and exchanges the vectors by stores into one another's shared memory. A
+// step is four exchanges, so what a barrier costs sets its time: 0.25 us in a cluster against
+// 1.2 us over the grid. The order limit is what 16 x 227 KB hold. A step bound (12 steps and the
+// Ritz part; order 100 / 200 / 300 / 456): 170 / 174 / 176 / 179 us with the cooperative kernel in
+// launches of three steps and a Ritz part of eleven launches, now 64 / 72 / 89 / 107 in two.
+constexpr int kLzCl = 16, kLzClThreads = 512, kLzClWarps = kLzClThreads / 32;
+constexpr int kLzClusterMaxN = 456;
+
+__host__ __device__ inline int lz_cl_cpb(int n) { return (n + kLzCl - 1) / kLzCl; }
+inline size_t lz_cl_smem(int n) {
+    return sizeof(double) * ((size_t) lz_cached_doubles(n, lz_cl_cpb(n)) + 5 * (size_t) n + 2 * kLzCl + kLzClWarps + 64);
+}
+
+__device__ __forceinline__ void lz_cl_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// One CTA's part of the operator and the exchange: local column c is column j0 + c.
+struct LzCluster {
+    int n, j0, nc, lane, warp;
+    double *sK, *sKT, *sD, *vec;   // vec: what follows the columns
+    unsigned base, rbase;          // shared-window address of the dynamic memory here and in CTA `lane`
+
+    __device__ __forceinline__ void init(int n_, const double *K, const double *KT, long ldk, const double *D, long ldD) {
+        extern __shared__ double dyn[];
+        n = n_;
+        lane = threadIdx.x & 31;
+        warp = threadIdx.x >> 5;
+        const int cpb = lz_cl_cpb(n);
+        j0 = min(n, (int) blockIdx.x * cpb);
+        nc = min(n, j0 + cpb) - j0;
+        sK = dyn;
+        sKT = sK + ((long) nc * (n - j0) - (long) nc * (nc - 1) / 2);
+        sD = sKT + ((long) nc * (j0 + 1) + (long) nc * (nc - 1) / 2);
+        vec = dyn + lz_cached_doubles(n, cpb);
+        base = (unsigned) __cvta_generic_to_shared(dyn);
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbase) : "r"(base), "r"(lane & (kLzCl - 1)));
+        for (int c = warp; c < nc; c += kLzClWarps) {
+            const int j = j0 + c;
+            double *dk = colK(c), *dkt = colKT(c), *dd = sD + (long) c * n;
+            const double *gk = K + (size_t) j * ldk, *gkt = KT + (size_t) j * ldk, *gd = D + (size_t) j * ldD;
+#pragma unroll 8
+            for (int i = j + lane; i < n; i += 32) dk[i] = __ldg(gk + i);
+#pragma unroll 8
+            for (int i = lane; i <= j; i += 32) dkt[i] = __ldg(gkt + i);
+#pragma unroll 8
+            for (int i = lane; i < n; i += 32) dd[i] = __ldg(gd + i);
+        }
+    }
+    // column c of K / K^T, indexed by the matrix row
+    __device__ __forceinline__ double *colK(int c) const {
+        return sK + ((long) c * (n - j0) - (long) c * (c - 1) / 2) - (j0 + c);
+    }
+    __device__ __forceinline__ double *colKT(int c) const { return sKT + ((long) c * (j0 + 1) + (long) c * (c - 1) / 2); }
+    // sum over rows lo <= i < hi of col[i] x[i], by the warp
+    __device__ __forceinline__ double dot(const double *col, const double *x, int lo, int hi) const {
+        double p[4] = {};
+        int i = lo + lane;
+        for (; i + 96 < hi; i += 128) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) p[q] += col[i + 32 * q] * x[i + 32 * q];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (i + 32 * q < hi) p[q] += col[i + 32 * q] * x[i + 32 * q];
+        return warp_sum((p[0] + p[2]) + (p[1] + p[3]));
+    }
+    // v (the same in every lane) to the address of *slot in every CTA of the cluster
+    __device__ __forceinline__ void share(double v, const double *slot) const {
+        const unsigned off = (unsigned) __cvta_generic_to_shared(slot) - base;
+        if (lane < kLzCl) asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(rbase + off), "d"(v) : "memory");
+    }
+    // the block's sum of one value a warp (v the same in every lane), into part[this CTA] everywhere
+    __device__ __forceinline__ void share_sum(double v, double *red, const double *part) const {
+        if (lane == 0) red[warp] = v;
+        __syncthreads();
+        if (warp == 0) {
+            double x = (lane < kLzClWarps) ? red[lane] : 0.0;
+            x = warp_sum(x);
+            share(x, part + blockIdx.x);
+        }
+    }
+    static __device__ __forceinline__ double total(const double *part) {
+        double t = 0.0;
+#pragma unroll
+        for (int r = 0; r < kLzCl; ++r) t += part[r];
+        return t;
+    }
+};
+
+// Steps k0 .. k1-1, as lanczos_orth_kernel takes them; step 0 starts from normalise(a + b) (a may
+// be null). alpha and beta go to ab and, when set, to the host's mirror hab; V's columns k0 + 1 ..
+// k1 to global memory (zero past a breakdown).
+__global__ void __launch_bounds__(kLzClThreads, 1)
+    lz_cluster_steps_kernel(int n, const double *K, const double *KT, long ldk, const double *D, long ldD,
+                            const double *a, const double *b, double *V, long ldv, double *ab, double *hab, int maxdim,
+                            int k0, int k1) {
+    LzCluster C;
+    C.init(n, K, KT, ldk, D, ldD);
+    const int tid = threadIdx.x, warp = C.warp;
+    double *v = C.vec, *vp = v + n, *st = vp + n, *su = st + n, *sw = su + n, *part = sw + n, *qpart = part + kLzCl,
+           *red = qpart + kLzCl;
+    const bool first = blockIdx.x == 0;
+    double betaPrev = 0.0;
+    if (k0 == 0) {
+        double acc = 0.0;
+        for (int i = tid; i < n; i += kLzClThreads) {
+            const double x = (a ? a[i] : 0.0) + b[i];
+            v[i] = x;
+            acc += x * x;
+        }
+        const double nrm = sqrt(bsum(acc));
+        for (int i = tid; i < n; i += kLzClThreads) {
+            v[i] = (nrm > 0.0) ? v[i] / nrm : 0.0;
+            if (first) V[i] = v[i];
+        }
+    } else {
+        for (int i = tid; i < n; i += kLzClThreads) {
+            v[i] = V[(size_t) k0 * ldv + i];
+            vp[i] = V[(size_t) (k0 - 1) * ldv + i];
+        }
+        betaPrev = ab[maxdim + k0 - 1];
+    }
+    lz_cl_sync();   // every CTA is there, its vector and columns in place
+    for (int k = k0; k < k1; ++k) {
+        for (int c = warp; c < C.nc; c += kLzClWarps)       // t = K^T v
+            C.share(C.dot(C.colK(c), v, C.j0 + c, n), st + C.j0 + c);
+        lz_cl_sync();
+        for (int c = warp; c < C.nc; c += kLzClWarps)       // u = -D t
+            C.share(-C.dot(C.sD + (long) c * n, st, 0, n), su + C.j0 + c);
+        lz_cl_sync();
+        double w[2] = {}, p = 0.0;
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {                       // w = K u - beta v_{k-1}
+            const int c = warp + m * kLzClWarps, j = C.j0 + c;
+            if (c >= C.nc) break;
+            w[m] = C.dot(C.colKT(c), su, 0, j + 1);
+            if (k > 0) w[m] -= betaPrev * vp[j];
+            p += w[m] * v[j];
+        }
+        C.share_sum(p, red, part);
+        lz_cl_sync();
+        const double alp = LzCluster::total(part);
+        p = 0.0;
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const int c = warp + m * kLzClWarps, j = C.j0 + c;
+            if (c >= C.nc) break;
+            w[m] -= alp * v[j];
+            p += w[m] * w[m];
+            C.share(w[m], sw + j);
+        }
+        C.share_sum(p, red, qpart);
+        lz_cl_sync();
+        const double nrm = sqrt(LzCluster::total(qpart));
+        betaPrev = (nrm > 0.0) ? nrm : 0.0;
+        for (int i = tid; i < n; i += kLzClThreads) {
+            const double x = (nrm > 0.0) ? sw[i] / nrm : 0.0;
+            vp[i] = x;
+            if (first) V[(size_t) (k + 1) * ldv + i] = x;
+        }
+        if (first && tid == 0) {
+            ab[k] = alp;
+            ab[maxdim + k] = betaPrev;
+            if (hab) {
+                hab[k] = alp;
+                hab[maxdim + k] = betaPrev;
+            }
+        }
+        double *const x = v;
+        v = vp;
+        vp = x;
+        __syncthreads();
+    }
+}
+
+// The Ritz part of a check: z_q = V y_q and m_q = M z_q for both coefficient vectors (y, then
+// y + kp1), warm = m_0, out[q] = |m_q - lam z_q| (and in the host's mirror hout when set).
+__global__ void __launch_bounds__(kLzClThreads, 1)
+    lz_cluster_ritz_kernel(int n, const double *K, const double *KT, long ldk, const double *D, long ldD,
+                           const double *V, long ldv, int kp1, const double *y, double lam, double *warm, double *out,
+                           double *hout) {
+    LzCluster C;
+    C.init(n, K, KT, ldk, D, ldD);
+    const int tid = threadIdx.x, lane = C.lane, warp = C.warp;
+    double *z = C.vec, *st = z + 2 * n, *part = st + 2 * n, *red = part + 2 * kLzCl, *sy = red + kLzClWarps;
+    if (tid < 2 * kp1) sy[tid] = y[tid];
+    __syncthreads();
+    for (int i = tid; i < 2 * n; i += kLzClThreads) {
+        const int q = i >= n, r = i - q * n;
+        double acc = 0.0;
+#pragma unroll 8
+        for (int j = 0; j < kp1; ++j) acc += V[(size_t) r + (size_t) j * ldv] * sy[q * kp1 + j];
+        z[i] = acc;
+    }
+    lz_cl_sync();
+    double own[2][2];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        const int c = warp + m * kLzClWarps, j = C.j0 + c;
+        if (c >= C.nc) break;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            own[m][q] = z[q * n + j];
+            C.share(C.dot(C.colK(c), z + q * n, j, n), st + q * n + j);
+        }
+    }
+    lz_cl_sync();   // nobody reads z any more: u = -D t takes its place
+    for (int c = warp; c < C.nc; c += kLzClWarps)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            C.share(-C.dot(C.sD + (long) c * n, st + q * n, 0, n), z + q * n + C.j0 + c);
+    lz_cl_sync();
+    double p[2] = {};
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        const int c = warp + m * kLzClWarps, j = C.j0 + c;
+        if (c >= C.nc) break;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const double x = C.dot(C.colKT(c), z + q * n, 0, j + 1);
+            if (q == 0 && lane == 0) warm[j] = x;
+            const double r = x - lam * own[m][q];
+            p[q] += r * r;
+        }
+    }
+    C.share_sum(p[0], red, part);
+    __syncthreads();
+    C.share_sum(p[1], red, part + kLzCl);
+    lz_cl_sync();
+    if (blockIdx.x == 0 && tid < 2) {
+        const double r = sqrt(LzCluster::total(part + tid * kLzCl));
+        out[tid] = r;
+        if (hout) hout[tid] = r;
+    }
+}
+
+// a launch of one cluster
+template <class... P, class... A>
+cudaError_t lz_cluster_launch(void (*fn)(P...), size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(hb::counted(kLzCl));
+    cfg.blockDim = dim3(kLzClThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {kLzCl, 1, 1};
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, (P) args...);
+}
+
+// whether the device takes a cluster of 16 with the largest order's shared memory (per device)
+bool lz_cluster_available() {
+    static std::atomic<int> state[kMaxDevices];   // 0 unknown, 1 yes, 2 no
+    const int dev = current_device();
+    int v = state[dev].load(std::memory_order_acquire);
+    if (v) return v == 1;
+    const int smem = (int) lz_cl_smem(kLzClusterMaxN);
+    bool ok = true;
+    for (const void *fn : {(const void *) lz_cluster_steps_kernel, (const void *) lz_cluster_ritz_kernel}) {
+        ok = ok && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+             cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kLzCl);
+        cfg.blockDim = dim3(kLzClThreads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim = {kLzCl, 1, 1};
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        ok = ok && cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters >= 1;
+    }
+    if (!ok) cudaGetLastError();
+    state[dev].store(ok ? 1 : 2, std::memory_order_release);
+    return ok;
+}
+
 // ---- Lanczos for blocks of order <= kSmallLanczosN: one CTA runs every step in one launch
 // (the stepwise path spends four launches per step, which dominates for small blocks).
 //
@@ -2178,9 +2461,11 @@ template <class Job> void lz_allow_smem(int bytes) {
 
 // All eigenpairs of the symmetric tridiagonal matrix with diagonal d[0..n) and
 // off-diagonal e[0..n-1): QL iteration with implicit Wilkinson shifts, rotations
-// accumulated into Z (column-major n x n, columns are eigenvectors).
+// accumulated into Z (column-major n x n, columns are eigenvectors). Only rows r0 .. n - 1 of Z
+// are formed, each by the same operations whatever r0 (a check reads the last row alone, which
+// costs n^2 instead of n^3).
 void tridiag_eig(int n, std::vector<double> d, std::vector<double> e, std::vector<double> &evals,
-                 std::vector<double> &Z) {
+                 std::vector<double> &Z, int r0 = 0) {
     Z.assign((size_t) n * n, 0.0);
     for (int i = 0; i < n; ++i) Z[(size_t) i * n + i] = 1.0;
     e.resize(n, 0.0);
@@ -2214,7 +2499,7 @@ void tridiag_eig(int n, std::vector<double> d, std::vector<double> e, std::vecto
                 p = sn * r;
                 d[i + 1] = g + p;
                 g = c * r - b;
-                for (int k = 0; k < n; ++k) {
+                for (int k = r0; k < n; ++k) {
                     f = Z[(size_t) (i + 1) * n + k];
                     Z[(size_t) (i + 1) * n + k] = sn * Z[(size_t) i * n + k] + c * f;
                     Z[(size_t) i * n + k] = c * Z[(size_t) i * n + k] - sn * f;
@@ -2312,6 +2597,7 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
     // small blocks: every step in one launch, then the checks below replay the schedule on
     // the recorded alpha / beta (a step's values do not depend on later steps)
     const bool small = !hyOp && n <= kSmallLanczosN;
+    const bool cluster = !hyOp && !small && n <= kLzClusterMaxN && lz_cluster_available();
     if (small) {
         static std::atomic<unsigned long long> attr{0};
         once_per_device(attr, [] {
@@ -2328,7 +2614,7 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
         HB_CUDA(cudaMemcpyAsync(h_ab, d_ab, sizeof(double) * (2 * maxdim + 2), cudaMemcpyDeviceToHost, s));
         HB_CUDA(cudaStreamSynchronize(s));
         if (tm) tm->n_lanczos_mv += maxdim;
-    } else {
+    } else if (!cluster) {
         HB_CUDA(cudaMemsetAsync(V, 0, sizeof(double) * ld * (maxdim + 1), s));
         HB_CUDA(cudaMemsetAsync(d_ab, 0, sizeof(double) * (2 * maxdim + 2), s));
         if (nComputed == 0) lanczos_start_kernel<<<hb::counted(1), 1024, 0, s>>>(n, nullptr, init_vec, V);
@@ -2338,7 +2624,7 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
     // columns of K, K^T and D held in shared memory when one block's share fits. Above
     // kLzFusedMaxN the three matrices stream from DRAM, where the per-step launches keep
     // more loads in flight than the cooperative grid.
-    const bool fused = !small && !hyOp && n <= kLzFusedMaxN;
+    const bool fused = !small && !cluster && !hyOp && n <= kLzFusedMaxN;
     int lzGrid = 0;
     bool lzCached = false;
     size_t lzSmem = 0;
@@ -2385,16 +2671,24 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
     std::vector<double> T, ev, evec;
     auto scheduled = [&](int k) { return ((k + 1) % freq == 0) || k >= maxdim - 1; };
     for (int k = 0; k < maxdim && !done; ++k) {
-        if (fused) {
+        if (fused || cluster) {
             if (k >= stepsDone) {
-                int k1 = k;
+                // to about where the last bound stopped (the checks below look at every scheduled
+                // step of it), then on: in the cluster three steps past the end cost less (10 us)
+                // than one more wait, over the grid (40 us at order 1,000) they cost more
+                int k1 = cluster ? ((k == 0) ? lastSteps : k + 2 * freq) : ((k == 0) ? lastSteps - freq : k + freq);
+                k1 = std::max(k + 1, std::min(maxdim, k1)) - 1;
                 while (!scheduled(k1)) ++k1;
-                k1 += 1;  // through the next check
+                k1 += 1;
                 const double *Kp = F.K, *KTp = F.KT, *Dp = D;
                 long ldk = F.ld, ldd = ldD, ldv = ld;
                 int nn = n, md = maxdim, ka = k, kb = k1;
                 double *Vp = V, *abp = d_ab, *tp = t1, *up = u, *wp = w, *pp = part;
-                if (lzCached) {
+                if (cluster) {
+                    HB_CUDA(lz_cluster_launch(lz_cluster_steps_kernel, lz_cl_smem(n), s, n, F.K, F.KT, F.ld, D, ldD,
+                                              nComputed == 0 ? nullptr : warm, nComputed == 0 ? init_vec : pert_vec, V,
+                                              ld, d_ab, dm_ab, maxdim, k, k1));
+                } else if (lzCached) {
                     void *args[] = {&nn, &Kp, &KTp, &ldk, &Dp, &ldd, &Vp, &ldv, &abp, &md, &ka, &kb, &wp, &tp, &up, &pp};
                     HB_CUDA(cudaLaunchCooperativeKernel((const void *) lanczos_steps_smem_kernel, hb::counted(lzGrid),
                                                         kLzThreads, args, lzSmem, s));
@@ -2405,6 +2699,11 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
                 }
                 if (tm) tm->n_lanczos_mv += k1 - k;
                 stepsDone = k1;
+                if (!cluster || !dm_ab)
+                    HB_CUDA(cudaMemcpyAsync(h_ab, d_ab, sizeof(double) * (2 * maxdim + 2), cudaMemcpyDeviceToHost, s));
+                const double tw = wall();
+                HB_CUDA(cudaStreamSynchronize(s));
+                if (tm) tm->lz_wait += wall() - tw;
             }
         } else if (!small) {
             mv(V + (size_t) k * ld, w);
@@ -2412,7 +2711,7 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
         }
         const bool sched = scheduled(k);
         if (!sched) continue;
-        if (!small) {
+        if (!small && !fused && !cluster) {
             HB_CUDA(cudaMemcpyAsync(h_ab, d_ab, sizeof(double) * (2 * maxdim + 2), cudaMemcpyDeviceToHost, s));
             double tw = wall();
             HB_CUDA(cudaStreamSynchronize(s));
@@ -2431,7 +2730,7 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
         }
         std::vector<double> dd(h_ab, h_ab + kp1), ee(h_ab + maxdim, h_ab + maxdim + kp1);
         ee[kp1 - 1] = 0.0;
-        tridiag_eig(kp1, dd, ee, ev, evec);
+        tridiag_eig(kp1, dd, ee, ev, evec, kp1 - 1);
         if (tm) tm->lz_host += wall() - th;
         int i1 = 0, i2 = 0;  // largest, second largest
         for (int i = 1; i < kp1; ++i)
@@ -2446,13 +2745,21 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
             continue;
         }
         const double eigMin1 = ev[i1], eigMin2 = ev[i2];
+        tridiag_eig(kp1, dd, ee, ev, evec);
         std::vector<double> yy(2 * kp1);
         for (int i = 0; i < kp1; ++i) {
             yy[i] = evec[(size_t) i + (size_t) i1 * kp1];
             yy[kp1 + i] = evec[(size_t) i + (size_t) i2 * kp1];
         }
-        HB_CUDA(cudaMemcpyAsync(d_y, yy.data(), sizeof(double) * 2 * kp1, cudaMemcpyHostToDevice, s));
-        if (small) {
+        lastSteps = kp1;
+        const bool mapped = cluster && dm_yv && dm_scal;   // coefficients and residuals in place
+        if (mapped) std::memcpy(h_yv, yy.data(), sizeof(double) * 2 * kp1);
+        else HB_CUDA(cudaMemcpyAsync(d_y, yy.data(), sizeof(double) * 2 * kp1, cudaMemcpyHostToDevice, s));
+        if (cluster) {
+            HB_CUDA(lz_cluster_launch(lz_cluster_ritz_kernel, lz_cl_smem(n), s, n, F.K, F.KT, F.ld, D, ldD, V, ld, kp1,
+                                      mapped ? dm_yv : d_y, eigMin1, warm, d_scal, mapped ? dm_scal : nullptr));
+            if (tm) tm->n_lanczos_mv += 2;
+        } else if (small) {
             lanczos_small_ritz_kernel<<<hb::counted(1), kSmallRitzThreads, small_ritz_smem(n), s>>>(
                 n, F.K, F.ld, D, ldD, V, ld, kp1, d_y, eigMin1, warm, d_scal);
             HB_CUDA(cudaGetLastError());
@@ -2466,7 +2773,7 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
             mv(z2, z1);
             lanczos_resid_kernel<<<hb::counted(1), 1024, 0, s>>>(n, z1, z2, eigMin1, d_scal + 1);
         }
-        HB_CUDA(cudaMemcpyAsync(h_scal, d_scal, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
+        if (!mapped) HB_CUDA(cudaMemcpyAsync(h_scal, d_scal, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
         HB_CUDA(cudaStreamSynchronize(s));
         const double resiVal1 = h_scal[0], resiVal2 = h_scal[1];
         const double resiDiff = eigMin1 - eigMin2 - resiVal2;
@@ -2533,7 +2840,7 @@ bool lz_advance(LzRun &R) {
         }
         std::vector<double> dd(L.h_ab, L.h_ab + kp1), ee(L.h_ab + maxdim, L.h_ab + maxdim + kp1);
         ee[kp1 - 1] = 0.0;
-        tridiag_eig(kp1, dd, ee, R.ev, R.evec);
+        tridiag_eig(kp1, dd, ee, R.ev, R.evec, kp1 - 1);
         R.host_s += wall() - th;
         int i1 = 0, i2 = 0;
         for (int i = 1; i < kp1; ++i)
@@ -2551,6 +2858,7 @@ bool lz_advance(LzRun &R) {
         R.eigMin1 = R.ev[i1];
         R.eigMin2 = R.ev[i2];
         R.betak = betak;
+        tridiag_eig(kp1, dd, ee, R.ev, R.evec);
         std::vector<double> yy(2 * kp1);
         for (int i = 0; i < kp1; ++i) {
             yy[i] = R.evec[(size_t) i + (size_t) i1 * kp1];

@@ -62,6 +62,7 @@ struct Lanczos {
     double *h_yv = nullptr;
     double *dm_ab = nullptr, *dm_scal = nullptr, *dm_yv = nullptr;
     int nComputed = 0;
+    int lastSteps = 12;       // steps the last bound took: as many go into the next one's first launch
     // when set, the operator is built from this sparse factor of S instead of F
     HybridFactor *hyOp = nullptr;
     void init(int n_, cudaStream_t s_);
