@@ -243,11 +243,20 @@ int kstat_read(int family, long long *launches, double *ms, double *work) {
 }
 
 // ------------------------------------------------------------------------------------
-// GEMM: 64 x 64 x 16 CTA tile, 4 warps (2 x 2), 32 x 32 warp tile of 8 x 8 DMMA tiles.
+// GEMM: BM x BN x 16 CTA tiles, four warps (2 x 2), fragments by DMMA, a cp.async pipeline of P_ST
+// stages. What bounds it is the FP64 tensor pipe, which one warp per scheduler can fill as long as
+// little else is issued between two DMMAs: the copies of tile kt + P_ST - 1 go out in four parts
+// between the four k-steps of tile kt, 16 bytes each from addresses kept in registers, and the
+// fragments of a k-step are read while the previous one multiplies (also across the barrier). Only
+// k-tiles that the end of K or a triangle's edge crosses, and unaligned operands, are copied by
+// elements with a test each. Order 2000 / 4000 / 8000: 23.2 / 26.8 / 28.1 TFLOP/s with 128 x 128
+// tiles of 8 warps that copied and tested every element, now 31.4 / 33.7 / 34.8 of the 36.6 that
+// DMMA alone reaches; order 200: 24.8 us (64 x 64 tiles, one load in flight), now 8.2.
+// Shared-memory layout per operand follows its global contiguity so the loads stay coalesced;
+// row pitches of BM + 4 (k-major) and 20 doubles (m/n-major) make the fragment reads
+// conflict-free.
 // ------------------------------------------------------------------------------------
 namespace {
-constexpr int BM = 64, BN = 64, BK = 16, GT = 128;
-
 using GemmP = GemmDesc;
 
 __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
@@ -256,112 +265,197 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
-__device__ __forceinline__ double load_a(const GemmP &p, int m, int k) {
-    if (m >= p.M || k >= p.K) return 0.0;
-    if ((p.flags & GEMM_A_LOWER) && k > m) return 0.0;
-    if ((p.flags & GEMM_A_UPPER) && k < m) return 0.0;
-    return p.ta ? p.A[(size_t) k + (size_t) m * p.lda] : p.A[(size_t) m + (size_t) k * p.lda];
+constexpr int P_T = 128, P_BK = 16, P_PM = P_BK + 4;
+
+__device__ __forceinline__ void cp_async(unsigned sdst, const double *gsrc, int bytes) {   // 8 bytes, zero past `bytes`
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sdst), "l"(gsrc), "r"(bytes));
 }
-
-__device__ __forceinline__ double load_b(const GemmP &p, int k, int n) {
-    if (n >= p.N || k >= p.K) return 0.0;
-    if ((p.flags & GEMM_B_LOWER) && k < n) return 0.0;
-    if ((p.flags & GEMM_B_UPPER) && k > n) return 0.0;
-    return p.tb ? p.B[(size_t) n + (size_t) k * p.ldb] : p.B[(size_t) k + (size_t) n * p.ldb];
+__device__ __forceinline__ void cp_async2(unsigned sdst, const double *gsrc) {   // 16 bytes
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sdst), "l"(gsrc));
 }
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-// one 64 x 64 tile (bx, by) of C
-__device__ __forceinline__ void gemm_tile(const GemmP &p, int bx, int by) {
-    const int m0 = bx * BM;
-    const int n0 = by * BN;
-    if ((p.flags & GEMM_C_LOWER) && m0 + BM - 1 < n0) return;
-    if (p.abort_flag && *p.abort_flag) return;
+// doubles of one stage of an operand with R rows (m or n) of the tile
+template <int R, bool KMAJOR>
+constexpr int kPStage = KMAJOR ? P_BK * (R + 4) : R * P_PM;
 
-    int kmin = 0, kmax = p.K;
-    if (p.flags & GEMM_A_LOWER) kmax = min(kmax, m0 + BM);
-    if (p.flags & GEMM_A_UPPER) kmin = max(kmin, m0);
-    if (p.flags & GEMM_B_LOWER) kmin = max(kmin, n0);
-    if (p.flags & GEMM_B_UPPER) kmax = min(kmax, n0 + BN);
-    kmin = (kmin / BK) * BK;
-
-    __shared__ double As[2][BK][BM + 4];
-    __shared__ double Bs[2][BK][BN + 4];
-
-    const int t = threadIdx.x;
-    const int lane = t & 31;
-    const int w = t >> 5;
-    const int wm = (w & 1) * 32;
-    const int wn = (w >> 1) * 32;
-
-    double acc[4][4][2];
+// One operand's share of the copies: an R x 16 tile (r along m or n) a k-tile, element (r, k) at
+// src[r + k ld] (KMAJOR: r contiguous) or src[k + r ld].
+template <int R, bool KMAJOR>
+struct PCopy {
+    static constexpr int C1 = KMAJOR ? R : P_BK;           // contiguous extent
+    static constexpr int PITCH = KMAJOR ? R + 4 : P_PM;
+    static constexpr int N = R * P_BK / 2 / P_T;           // 16-byte copies a thread makes per tile
+    static constexpr int STEP = P_T / (C1 / 2);            // lines that one copy of every thread covers
+    const double *p;   // this thread's first source element of the next tile
+    int off[N];        // the copies' offsets from it
+    long tile;         // one tile to the next
+    unsigned dst;      // offset in the stage
+    // Rows past the end repeat the last one (a pair that begins on it takes the element behind it,
+    // which is padding: ld is even, so above an odd number of rows): what the stage holds there
+    // reaches only entries of C that are not stored.
+    __device__ __forceinline__ void init(const double *src, long ld, int r0, int rEnd, int k0) {
+        const int c = 2 * (threadIdx.x & (C1 / 2 - 1)), l = threadIdx.x / (C1 / 2), last = rEnd - 1 - r0;
+        p = KMAJOR ? src + (size_t) (r0 + min(c, last & ~1)) + (size_t) (k0 + l) * ld : src + (size_t) (k0 + c) + (size_t) r0 * ld;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < N; ++i) off[i] = (int) ld * (KMAJOR ? i * STEP : min(l + i * STEP, last));
+        tile = KMAJOR ? P_BK * ld : P_BK;
+        dst = 8 * (l * PITCH + c);
+    }
+    // a quarter of a whole tile, 16 bytes a copy
+    __device__ __forceinline__ void whole(unsigned stage, int part) const {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-    double ra[8], rb[8];
-    auto gload = [&](int k0) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            int r, kk;
-            if (!p.ta) { r = t & 63; kk = (t >> 6) + 2 * i; }
-            else { kk = t & 15; r = (t >> 4) + 8 * i; }
-            ra[i] = load_a(p, m0 + r, k0 + kk);
-            int c, kb;
-            if (!p.tb) { kb = t & 15; c = (t >> 4) + 8 * i; }
-            else { c = t & 63; kb = (t >> 6) + 2 * i; }
-            rb[i] = load_b(p, k0 + kb, n0 + c);
-        }
-    };
-    auto sstore = [&](int buf) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            int r, kk;
-            if (!p.ta) { r = t & 63; kk = (t >> 6) + 2 * i; }
-            else { kk = t & 15; r = (t >> 4) + 8 * i; }
-            As[buf][kk][r] = ra[i];
-            int c, kb;
-            if (!p.tb) { kb = t & 15; c = (t >> 4) + 8 * i; }
-            else { c = t & 63; kb = (t >> 6) + 2 * i; }
-            Bs[buf][kb][c] = rb[i];
-        }
-    };
-
-    if (kmin < kmax) {
-        gload(kmin);
-        sstore(0);
-        __syncthreads();
-        int buf = 0;
-        for (int k0 = kmin; k0 < kmax; k0 += BK) {
-            const bool more = (k0 + BK) < kmax;
-            if (more) gload(k0 + BK);
-#pragma unroll
-            for (int ks = 0; ks < BK; ks += 4) {
-                double a[4], b[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) a[i] = As[buf][ks + (lane & 3)][wm + i * 8 + (lane >> 2)];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) b[j] = Bs[buf][ks + (lane & 3)][wn + j * 8 + (lane >> 2)];
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
-            }
-            if (more) sstore(buf ^ 1);
-            __syncthreads();
-            buf ^= 1;
+        for (int i = 0; i < N; ++i)
+            if (i * 4 / N == part) cp_async2(stage + dst + 8 * (i * STEP * PITCH), p + off[i]);
+    }
+    // a tile at the edge of the matrix or of a triangle, or unaligned: by elements (lo / up: the
+    // operand is zero for k > r / for k < r)
+    static __device__ __forceinline__ void edge(unsigned stage, const double *__restrict__ src, long ld, int r0, int rEnd,
+                                                int k0, int kEnd, bool lo, bool up) {
+        const int c = threadIdx.x & (C1 - 1);
+#pragma unroll 4
+        for (int l = threadIdx.x / C1; l < (KMAJOR ? P_BK : R); l += P_T / C1) {
+            const int r = r0 + (KMAJOR ? c : l), k = k0 + (KMAJOR ? l : c);
+            const bool ok = r < rEnd && k < kEnd && !(lo && k > r) && !(up && k < r);
+            const double *q = KMAJOR ? src + (size_t) r + (size_t) k * ld : src + (size_t) k + (size_t) r * ld;
+            cp_async(stage + 8 * (l * PITCH + c), ok ? q : src, ok ? 8 : 0);
         }
     }
+};
+
+// 16-byte copies: both operands start on a 16-byte boundary and have an even leading dimension
+__host__ __device__ __forceinline__ bool p_pairs(const GemmP &p) {
+    return (((uintptr_t) p.A | (uintptr_t) p.B) % 16 == 0) && ((p.lda | p.ldb) % 2 == 0);
+}
+
+// tile (bx, by) of C
+template <int BM_, int BN_, int P_ST, int TA, int TB>
+__device__ __forceinline__ void gemm_tile(const GemmP &p, int bx, int by) {
+    constexpr int WM = BM_ / 2, WN = BN_ / 2, FM = WM / 8, FN = WN / 8;
+    constexpr int SA = kPStage<BM_, !TA>, SB = kPStage<BN_, TB != 0>;
+    const int m0 = bx * BM_;
+    const int n0 = by * BN_;
+    if ((p.flags & GEMM_C_LOWER) && m0 + BM_ - 1 < n0) return;
+    if (p.abort_flag && *p.abort_flag) return;
+    const bool alo = p.flags & GEMM_A_LOWER, aup = p.flags & GEMM_A_UPPER;
+    // B's roles are swapped: lower means zero for k < n
+    const bool blo = p.flags & GEMM_B_UPPER, bup = p.flags & GEMM_B_LOWER;
+    int kmin = 0, kmax = p.K;
+    if (alo) kmax = min(kmax, m0 + BM_);
+    if (aup) kmin = max(kmin, m0);
+    if (bup) kmin = max(kmin, n0);
+    if (blo) kmax = min(kmax, n0 + BN_);
+    kmin = (kmin / P_BK) * P_BK;
+    const int nk = (kmax > kmin) ? (kmax - kmin + P_BK - 1) / P_BK : 0;
+
+    extern __shared__ __align__(16) double smem[];
+    const unsigned sbase = (unsigned) __cvta_generic_to_shared(smem);
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int wm = (w & 1) * WM, wn = (w >> 1) * WN;
+
+    // k-tiles fLo <= kt < fHi are whole: inside the matrices and off the triangles' edges
+    int fLo = 0, fHi = (p.K - kmin) / P_BK;
+    if (alo) fHi = min(fHi, (m0 + 1 - kmin) / P_BK);
+    if (blo) fHi = min(fHi, (n0 + 1 - kmin) / P_BK);
+    if (aup) fLo = max(fLo, (m0 + BM_ - 1 - kmin + P_BK - 1) / P_BK);
+    if (bup) fLo = max(fLo, (n0 + BN_ - 1 - kmin + P_BK - 1) / P_BK);
+    if (!p_pairs(p)) fHi = 0;
+    PCopy<BM_, !TA> ca;
+    PCopy<BN_, TB != 0> cb;
+    ca.init(p.A, p.lda, m0, p.M, kmin);
+    cb.init(p.B, p.ldb, n0, p.N, kmin);
+    // the part-th quarter of tile kt's copies (an edge tile's all at once); part 3 steps on
+    auto issue = [&](int kt, int stage, int part) {
+        const unsigned st = sbase + 8 * (stage * (SA + SB));
+        if (kt >= fLo && kt < fHi) {
+            ca.whole(st, part);
+            cb.whole(st + 8 * SA, part);
+        } else if (part == 0) {
+            const int k0 = kmin + kt * P_BK;
+            PCopy<BM_, !TA>::edge(st, p.A, p.lda, m0, p.M, k0, p.K, alo, aup);
+            PCopy<BN_, TB != 0>::edge(st + 8 * SA, p.B, p.ldb, n0, p.N, k0, p.K, blo, bup);
+        }
+        if (part == 3) {
+            ca.p += ca.tile;
+            cb.p += cb.tile;
+        }
+    };
+    double a[2][FM], b[2][FN];
+    const int fr = lane >> 2, fk = lane & 3;
+    auto frag = [&](int stage, int ks, int buf) {
+        const double *as = smem + stage * (SA + SB), *bs = as + SA;
+        const int kk = ks * 4 + fk;
+#pragma unroll
+        for (int i = 0; i < FM; ++i) {
+            const int m = wm + i * 8 + fr;
+            a[buf][i] = TA ? as[m * P_PM + kk] : as[kk * (BM_ + 4) + m];
+        }
+#pragma unroll
+        for (int j = 0; j < FN; ++j) {
+            const int n = wn + j * 8 + fr;
+            b[buf][j] = TB ? bs[kk * (BN_ + 4) + n] : bs[n * P_PM + kk];
+        }
+    };
+
+    double acc[FM][FN][2];
+#pragma unroll
+    for (int i = 0; i < FM; ++i)
+#pragma unroll
+        for (int j = 0; j < FN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int row = m0 + wm + i * 8 + (lane >> 2);
+    for (int st = 0; st < P_ST - 1; ++st) {
+        if (st < nk) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) issue(st, st, q);
+        }
+        cp_commit();
+    }
+    if (nk > 0) {
+        cp_wait<P_ST - 2>();
+        __syncthreads();
+        frag(0, 0, 0);
+    }
+    int cur = 0, nxt = P_ST - 1;   // stages of tile kt and of the tile being copied
+    for (int kt = 0; kt < nk; ++kt) {
+        const bool more = kt + P_ST - 1 < nk;
+        int ahead = cur + 1;
+        if (ahead == P_ST) ahead = 0;
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+            if (ks == 3) {   // tile kt + 1 is there and, behind the barrier, nobody reads tile kt - 1's stage
+                cp_commit();
+                cp_wait<P_ST - 2>();
+                __syncthreads();
+                if (kt + 1 < nk) frag(ahead, 0, 0);
+            } else {
+                frag(cur, ks + 1, (ks + 1) & 1);
+                if (more) {
+                    issue(kt + P_ST - 1, nxt, ks);
+                    if (ks == 2) issue(kt + P_ST - 1, nxt, 3);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < FM; ++i)
+#pragma unroll
+                for (int j = 0; j < FN; ++j) dmma(acc[i][j][0], acc[i][j][1], a[ks & 1][i], b[ks & 1][j]);
+        }
+        cur = ahead;
+        if (++nxt == P_ST) nxt = 0;
+    }
+    cp_wait<0>();
+
+#pragma unroll
+    for (int i = 0; i < FM; ++i) {
+        const int row = m0 + wm + i * 8 + fr;
         if (row >= p.M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < FN; ++j) {
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const int col = n0 + wn + j * 8 + (lane & 3) * 2 + e;
+                const int col = n0 + wn + j * 8 + fk * 2 + e;
                 if (col >= p.N) continue;
                 if ((p.flags & GEMM_C_LOWER) && row < col) continue;
                 double *cp = p.C + (size_t) row + (size_t) col * p.ldc;
@@ -373,24 +467,69 @@ __device__ __forceinline__ void gemm_tile(const GemmP &p, int bx, int by) {
     }
 }
 
-__global__ void __launch_bounds__(GT) gemm_kernel(GemmP p) { gemm_tile(p, blockIdx.x, blockIdx.y); }
+template <int BM_, int BN_, int P_ST, int TA, int TB>
+constexpr int kPBytes = P_ST * (kPStage<BM_, !TA> + kPStage<BN_, TB != 0>) * (int) sizeof(double);
 
-// one GEMM of a group per blockIdx.z (tiles beyond its own M x N exit)
-__global__ void __launch_bounds__(GT) gemm_grouped_kernel(const GemmP *__restrict__ ps) {
-    const GemmP p = ps[blockIdx.z];
-    if ((int) blockIdx.x * BM >= p.M || (int) blockIdx.y * BN >= p.N) return;
-    gemm_tile(p, blockIdx.x, blockIdx.y);
-}
-
-// GEMM z of a strided group: operands at A + z sa, B + z sb, C + z sc; with kstep set, the
-// K range [z kstep, (z + 1) kstep) of one product (sa and sb then move along K)
-__global__ void __launch_bounds__(GT) gemm_strided_kernel(GemmP p, long sa, long sb, long sc, int kstep) {
+// GEMM z = blockIdx.z of a strided group (one product: z = 0): operands at A + z sa, B + z sb,
+// C + z sc; with kstep set, the K range [z kstep, (z + 1) kstep) of one product (sa and sb then
+// move along K)
+template <int BM_, int BN_, int P_ST, int MINB, int TA, int TB>
+__global__ void __launch_bounds__(P_T, MINB) gemm_kernel(GemmP p, long sa, long sb, long sc, int kstep) {
     const int z = blockIdx.z;
     p.A += z * sa;
     p.B += z * sb;
     p.C += z * sc;
     if (kstep > 0) p.K = min(kstep, p.K - z * kstep);
-    gemm_tile(p, blockIdx.x, blockIdx.y);
+    gemm_tile<BM_, BN_, P_ST, TA, TB>(p, blockIdx.x, blockIdx.y);
+}
+
+// Tile sizes, by measurement (us for C = A B of order n, the 64 x 64 tile against the 32 x 32 one):
+// n = 200: 14.6 / 8.2, 1000: 83 / 73, 2001: 516 / 511, 4000: 3805 / 3867, 8000: 29250 / 36640. Small
+// products want every SM busy, large ones the operand traffic halved; the line lies at 3072^2
+// entries of C. The small tile's copies run five stages ahead because its DMMAs take only 256
+// cycles a k-tile.
+constexpr long kGemmLargeMN = 3072L * 3072L;
+constexpr int kGemmSt32 = 5, kGemmBlk32 = 4, kGemmSt64 = 3, kGemmBlk64 = 3;
+
+template <int BM_, int BN_, int P_ST, int MINB, int TA, int TB>
+void launch_tiles(const GemmP &p, long sa, long sb, long sc, int count, int kstep, cudaStream_t s) {
+    constexpr int bytes = kPBytes<BM_, BN_, P_ST, TA, TB>;
+    static std::atomic<unsigned long long> init{0};
+    once_per_device(init, [] {
+        HB_CUDA(cudaFuncSetAttribute(gemm_kernel<BM_, BN_, P_ST, MINB, TA, TB>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    });
+    dim3 grid((p.M + BM_ - 1) / BM_, (p.N + BN_ - 1) / BN_, count);
+    gemm_kernel<BM_, BN_, P_ST, MINB, TA, TB><<<hb::counted(grid), P_T, bytes, s>>>(p, sa, sb, sc, kstep);
+    HB_CUDA(cudaGetLastError());
+}
+
+template <int TA, int TB>
+void launch_gemm(const GemmP &p, long sa, long sb, long sc, int count, int kstep, cudaStream_t s) {
+    if ((long) p.M * p.N >= kGemmLargeMN)
+        launch_tiles<64, 64, kGemmSt64, kGemmBlk64, TA, TB>(p, sa, sb, sc, count, kstep, s);
+    else
+        launch_tiles<32, 32, kGemmSt32, kGemmBlk32, TA, TB>(p, sa, sb, sc, count, kstep, s);
+}
+
+void launch_gemm(const GemmP &p, long sa, long sb, long sc, int count, int kstep, cudaStream_t s) {
+    if (!p.ta && !p.tb) launch_gemm<0, 0>(p, sa, sb, sc, count, kstep, s);
+    else if (p.ta && !p.tb) launch_gemm<1, 0>(p, sa, sb, sc, count, kstep, s);
+    else if (!p.ta && p.tb) launch_gemm<0, 1>(p, sa, sb, sc, count, kstep, s);
+    else launch_gemm<1, 1>(p, sa, sb, sc, count, kstep, s);
+}
+
+// one GEMM of a group per blockIdx.z (tiles beyond its own M x N exit)
+__global__ void __launch_bounds__(P_T, kGemmBlk32) gemm_grouped_kernel(const GemmP *__restrict__ ps) {
+    const GemmP p = ps[blockIdx.z];
+    if ((int) blockIdx.x * 32 >= p.M || (int) blockIdx.y * 32 >= p.N) return;
+    if (p.ta) {
+        if (p.tb) gemm_tile<32, 32, kGemmSt32, 1, 1>(p, blockIdx.x, blockIdx.y);
+        else gemm_tile<32, 32, kGemmSt32, 1, 0>(p, blockIdx.x, blockIdx.y);
+    } else {
+        if (p.tb) gemm_tile<32, 32, kGemmSt32, 0, 1>(p, blockIdx.x, blockIdx.y);
+        else gemm_tile<32, 32, kGemmSt32, 0, 0>(p, blockIdx.x, blockIdx.y);
+    }
 }
 }  // namespace
 
@@ -402,167 +541,24 @@ void gemm_strided(cudaStream_t s, const GemmDesc &d, long sa, long sb, long sc, 
         p.B += z0 * sb;
         p.C += z0 * sc;
         if (kstep > 0) p.K -= z0 * kstep;
-        dim3 grid((d.M + BM - 1) / BM, (d.N + BN - 1) / BN, std::min(65535, count - z0));
-        gemm_strided_kernel<<<hb::counted(grid), GT, 0, s>>>(p, sa, sb, sc, kstep);
-        HB_CUDA(cudaGetLastError());
+        launch_gemm(p, sa, sb, sc, std::min(65535, count - z0), kstep, s);
     }
 }
 
 void gemm_grouped(cudaStream_t s, const GemmDesc *d_desc, int count, int maxM, int maxN) {
     if (count <= 0 || maxM <= 0 || maxN <= 0) return;
+    constexpr int bytes = std::max(std::max(kPBytes<32, 32, kGemmSt32, 0, 0>, kPBytes<32, 32, kGemmSt32, 0, 1>),
+                                   std::max(kPBytes<32, 32, kGemmSt32, 1, 0>, kPBytes<32, 32, kGemmSt32, 1, 1>));
+    static std::atomic<unsigned long long> init{0};
+    once_per_device(init, [] {
+        HB_CUDA(cudaFuncSetAttribute(gemm_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    });
     for (int z0 = 0; z0 < count; z0 += 65535) {
-        dim3 grid((maxM + BM - 1) / BM, (maxN + BN - 1) / BN, std::min(65535, count - z0));
-        gemm_grouped_kernel<<<hb::counted(grid), GT, 0, s>>>(d_desc + z0);
+        dim3 grid((maxM + 31) / 32, (maxN + 31) / 32, std::min(65535, count - z0));
+        gemm_grouped_kernel<<<hb::counted(grid), P_T, bytes, s>>>(d_desc + z0);
         HB_CUDA(cudaGetLastError());
     }
 }
-
-// ------------------------------------------------------------------------------------
-// Large-tile GEMM: 128 x 128 x 16 CTA tile, 8 warps (4 along M x 2 along N), warp tile
-// 32 x 64 = 4 x 8 DMMA fragments, 3-stage cp.async pipeline with zero-fill predicates.
-// Shared-memory layout per operand follows its global contiguity so the loads stay
-// coalesced; row pitches of 132 / 20 doubles make the fragment reads conflict-free.
-// ------------------------------------------------------------------------------------
-namespace {
-constexpr int L_BM = 128, L_BN = 128, L_BK = 16, L_T = 256, L_ST = 3;
-constexpr int L_PK = L_BM + 4;   // pitch of a k-major tile row (128 contiguous elements)
-constexpr int L_PM = L_BK + 4;   // pitch of an m/n-major tile row (16 contiguous k)
-constexpr int L_STAGE = 2560;    // doubles per operand per stage (max of 16*132, 128*20)
-
-__device__ __forceinline__ void cp_async8(double *sdst, const double *gsrc, bool pred) {
-    const unsigned saddr = (unsigned) __cvta_generic_to_shared(sdst);
-    const int bytes = pred ? 8 : 0;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(saddr), "l"(gsrc), "r"(bytes));
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
-
-template <int TA, int TB>
-__global__ void __launch_bounds__(L_T) gemm_large_kernel(GemmP p) {
-    const int m0 = blockIdx.x * L_BM;
-    const int n0 = blockIdx.y * L_BN;
-    if ((p.flags & GEMM_C_LOWER) && m0 + L_BM - 1 < n0) return;
-    if (p.abort_flag && *p.abort_flag) return;
-    int kmin = 0, kmax = p.K;
-    if (p.flags & GEMM_A_LOWER) kmax = min(kmax, m0 + L_BM);
-    if (p.flags & GEMM_A_UPPER) kmin = max(kmin, m0);
-    if (p.flags & GEMM_B_LOWER) kmin = max(kmin, n0);
-    if (p.flags & GEMM_B_UPPER) kmax = min(kmax, n0 + L_BN);
-    kmin = (kmin / L_BK) * L_BK;
-    const int nk = (kmax > kmin) ? (kmax - kmin + L_BK - 1) / L_BK : 0;
-
-    extern __shared__ double smem[];
-    double *As = smem;
-    double *Bs = smem + L_ST * L_STAGE;
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const int wm = (w & 3) * 32, wn = (w >> 2) * 64;
-
-    auto issue = [&](int kt, int stage) {
-        const int k0 = kmin + kt * L_BK;
-        double *as = As + stage * L_STAGE;
-        double *bs = Bs + stage * L_STAGE;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            int m, k;
-            if (!TA) { m = t & 127; k = (t >> 7) + 2 * i; }
-            else { k = t & 15; m = (t >> 4) + 16 * i; }
-            const int gm = m0 + m, gk = k0 + k;
-            bool ok = gm < p.M && gk < p.K;
-            if ((p.flags & GEMM_A_LOWER) && gk > gm) ok = false;
-            if ((p.flags & GEMM_A_UPPER) && gk < gm) ok = false;
-            const double *src = ok ? (TA ? p.A + (size_t) gk + (size_t) gm * p.lda : p.A + (size_t) gm + (size_t) gk * p.lda) : p.A;
-            double *dst = TA ? as + m * L_PM + k : as + k * L_PK + m;
-            cp_async8(dst, src, ok);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            int n, k;
-            if (!TB) { k = t & 15; n = (t >> 4) + 16 * i; }
-            else { n = t & 127; k = (t >> 7) + 2 * i; }
-            const int gn = n0 + n, gk = k0 + k;
-            bool ok = gn < p.N && gk < p.K;
-            if ((p.flags & GEMM_B_LOWER) && gk < gn) ok = false;
-            if ((p.flags & GEMM_B_UPPER) && gk > gn) ok = false;
-            const double *src = ok ? (TB ? p.B + (size_t) gn + (size_t) gk * p.ldb : p.B + (size_t) gk + (size_t) gn * p.ldb) : p.B;
-            double *dst = TB ? bs + k * L_PK + n : bs + n * L_PM + k;
-            cp_async8(dst, src, ok);
-        }
-    };
-
-    double acc[4][8][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-#pragma unroll
-    for (int st = 0; st < L_ST - 1; ++st) {
-        if (st < nk) issue(st, st);
-        cp_commit();
-    }
-    for (int kt = 0; kt < nk; ++kt) {
-        cp_wait<L_ST - 2>();
-        __syncthreads();
-        const int nxt = kt + L_ST - 1;
-        if (nxt < nk) issue(nxt, nxt % L_ST);
-        cp_commit();
-        const double *as = As + (kt % L_ST) * L_STAGE;
-        const double *bs = Bs + (kt % L_ST) * L_STAGE;
-#pragma unroll
-        for (int ks = 0; ks < L_BK; ks += 4) {
-            const int kk = ks + (lane & 3);
-            double a[4], b[8];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int m = wm + i * 8 + (lane >> 2);
-                a[i] = TA ? as[m * L_PM + kk] : as[kk * L_PK + m];
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int n = wn + j * 8 + (lane >> 2);
-                b[j] = TB ? bs[kk * L_PK + n] : bs[n * L_PM + kk];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
-        }
-    }
-    cp_wait<0>();
-
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int row = m0 + wm + i * 8 + (lane >> 2);
-        if (row >= p.M) continue;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int col = n0 + wn + j * 8 + (lane & 3) * 2 + e;
-                if (col >= p.N) continue;
-                if ((p.flags & GEMM_C_LOWER) && row < col) continue;
-                double *cp = p.C + (size_t) row + (size_t) col * p.ldc;
-                double v = p.alpha * acc[i][j][e];
-                if (p.beta != 0.0) v += p.beta * (*cp);
-                *cp = v;
-            }
-        }
-    }
-}
-
-constexpr int L_SMEM = 2 * L_ST * L_STAGE * (int) sizeof(double);
-
-template <int TA, int TB>
-void launch_large(const GemmP &p, cudaStream_t s) {
-    static std::atomic<unsigned long long> init{0};
-    once_per_device(init, [] {
-        HB_CUDA(cudaFuncSetAttribute(gemm_large_kernel<TA, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, L_SMEM));
-    });
-    dim3 grid((p.M + L_BM - 1) / L_BM, (p.N + L_BN - 1) / L_BN);
-    gemm_large_kernel<TA, TB><<<hb::counted(grid), L_T, L_SMEM, s>>>(p);
-}
-}  // namespace
 
 void gemm(cudaStream_t s, int M, int N, int K, double alpha, const double *A, long lda, int transA,
           const double *B, long ldb, int transB, double beta, double *C, long ldc, int flags,
@@ -578,18 +574,7 @@ void gemm(cudaStream_t s, int M, int N, int K, double alpha, const double *A, lo
         if (flags & (GEMM_B_LOWER | GEMM_B_UPPER)) f *= 0.5;
         kstat_begin(KF_GEMM, s, f);
     }
-    // Large tiles once the 128 x 128 grid fills the machine; 64 x 64 tiles otherwise.
-    const long tiles = (long) ((M + L_BM - 1) / L_BM) * ((N + L_BN - 1) / L_BN);
-    if (tiles >= 96 && K >= 64) {
-        if (!transA && !transB) launch_large<0, 0>(p, s);
-        else if (transA && !transB) launch_large<1, 0>(p, s);
-        else if (!transA && transB) launch_large<0, 1>(p, s);
-        else launch_large<1, 1>(p, s);
-    } else {
-        dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);
-        gemm_kernel<<<hb::counted(grid), GT, 0, s>>>(p);
-    }
-    HB_CUDA(cudaGetLastError());
+    launch_gemm(p, 0, 0, 0, 1, 0, s);
     if (timed) kstat_end(s);
 }
 

@@ -41,9 +41,9 @@ struct GemmDesc {
     const int *abort_flag;
 };
 // A group of independent GEMMs (device array of descriptors, none larger than maxM x maxN)
-// in one launch on the 64 x 64 DMMA tiles.
+// in one launch on the 32 x 32 DMMA tiles.
 void gemm_grouped(cudaStream_t s, const GemmDesc *d_desc, int count, int maxM, int maxN);
-// `count` GEMMs of one shape in one launch on the same tiles: GEMM z reads A + z sa and
+// `count` GEMMs of one shape in one launch: GEMM z reads A + z sa and
 // B + z sb and writes C + z sc. With kstep set the group is one product split along K: GEMM z
 // takes the K range [z kstep, min(K, (z + 1) kstep)), sa and sb being the strides of kstep
 // steps along K, and the caller adds the `count` partial products up.
