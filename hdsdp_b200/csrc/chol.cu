@@ -949,37 +949,6 @@ __global__ void __launch_bounds__(COOP_THREADS, 1) potrf_batch_array_kernel(cons
     small_factor_job(J);
 }
 
-__global__ void __launch_bounds__(COOP_THREADS, 1) trtri_coop_kernel(const double *L, double *K, long ld, int n,
-                                                                  const double *Dinv, long ldd) {
-    cg::grid_group grid = cg::this_grid();
-    for (int i0 = 0; i0 < n; i0 += NB) {
-        const int nb = min(NB, n - i0);
-        const int cend = i0 + nb;
-        const int nchunk = (cend + 63) / 64;
-        for (int ch = blockIdx.x; ch < nchunk; ch += gridDim.x) {
-            // X_i chunk <- Dinv_i * X_i chunk  (in place)
-            const int nc = min(64, cend - ch * 64);
-            double *Xc = K + i0 + (size_t) ch * 64 * ld;
-            Tile64::run(TileJob{Xc, ld, nb, nc, Dinv + i0, ldd, nb, Xc, ld, 0, nc, nb, false, 1}, 2);
-        }
-        grid.sync();
-        const int rows = n - cend;
-        if (rows <= 0) break;
-        const int rt = (rows + 63) / 64;
-        const long ntile = (long) rt * nchunk;
-        // C = K[cend + 64 ti.., 64 tj..] -= L[cend + 64 ti.., i0..i0+nb) * K[i0..i0+nb, 64 tj..]
-        auto update = [&](long t, TileJob &J) {
-            const int ti = (int) (t % rt), tj = (int) (t / rt);
-            const int mr = min(64, rows - ti * 64), nc = min(64, cend - tj * 64);
-            J = TileJob{K + (size_t) (cend + ti * 64) + (size_t) tj * 64 * ld, ld, mr, nc,
-                        L + (size_t) (cend + ti * 64) + (size_t) i0 * ld, ld, mr, K + i0 + (size_t) tj * 64 * ld, ld,
-                        0, nc, nb, false, 0};
-        };
-        tile_stream(update, blockIdx.x, ntile, gridDim.x);
-        grid.sync();
-    }
-}
-
 // Blocked substitution for L L^T x = b, one cooperative launch. The 64-row blocks of
 // the vector are dealt to the CTAs (block k to CTA k mod grid); a CTA keeps, in shared
 // memory, the accumulated products of its unfinished blocks with the solved ones.
@@ -1208,14 +1177,6 @@ __global__ void copy_lower_k(int n, const double *S, long lds, double *L, long l
         L[(size_t) r + (size_t) c * ldl] = (r >= c) ? S[(size_t) r + (size_t) c * lds] : 0.0;
 }
 
-__global__ void identity_k(int n, double *A, long lda) {
-    const long total = (long) n * n;
-    for (long idx = blockIdx.x * (long) blockDim.x + threadIdx.x; idx < total; idx += (long) gridDim.x * blockDim.x) {
-        const int r = (int) (idx % n), c = (int) (idx / n);
-        A[(size_t) r + (size_t) c * lda] = (r == c) ? 1.0 : 0.0;
-    }
-}
-
 int sm_count() { return device_sm_count(); }
 
 int coop_grid(const void *fn) {
@@ -1236,10 +1197,6 @@ int coop_grid(const void *fn) {
     return cached[dev][slot].load(std::memory_order_acquire);
 }
 
-int grid_for_n(long total) {
-    long b = (total + 255) / 256;
-    return (int) std::min<long>(std::max<long>(b, 1), 148L * 16);
-}
 }  // namespace
 
 // blocks of copy_lower_k: a whole number of row ranges of 256, about four columns a thread
@@ -1559,30 +1516,6 @@ int chol_solve_error() {
         cudaMemcpyToSymbol(g_tri_err, &z, sizeof(int));
     }
     return h;
-}
-
-bool coop_inverse_enqueue(cudaStream_t s, DenseFactor &F) {
-    const int n = F.n;
-    identity_k<<<hb::counted(grid_for_n((long) n * n)), 256, 0, s>>>(n, F.K, F.ld);
-    const void *fn = (const void *) trtri_coop_kernel;
-    const long t0 = (long) ((n - 1) / 64 + 1);
-    const int grid = (int) std::max(1L, std::min<long>(coop_grid(fn), t0 * t0 / 4 + 1));
-    const double *Lp = F.L;
-    double *Kp = F.K;
-    long ld = F.ld;
-    int nn = n;
-    const double *Dp = F.Dinv;
-    long ldd = F.ld;
-    void *args[] = {&Lp, &Kp, &ld, &nn, &Dp, &ldd};
-    const bool timed = kstat_on(KF_TRTRI);
-    if (timed) kstat_begin(KF_TRTRI, s, (double) n * n * n / 3.0);
-    cudaError_t e = cudaLaunchCooperativeKernel(fn, hb::counted(grid), COOP_THREADS, args, SM_DOUBLES * sizeof(double), s);
-    if (timed) kstat_end(s);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return true;
 }
 
 }  // namespace hb

@@ -472,14 +472,20 @@ constexpr int kPBytes = P_ST * (kPStage<BM_, !TA> + kPStage<BN_, TB != 0>) * (in
 
 // GEMM z = blockIdx.z of a strided group (one product: z = 0): operands at A + z sa, B + z sb,
 // C + z sc; with kstep set, the K range [z kstep, (z + 1) kstep) of one product (sa and sb then
-// move along K)
+// move along K); the group's last product has mLast rows and kLast of K when these are set
 template <int BM_, int BN_, int P_ST, int MINB, int TA, int TB>
-__global__ void __launch_bounds__(P_T, MINB) gemm_kernel(GemmP p, long sa, long sb, long sc, int kstep) {
+__global__ void __launch_bounds__(P_T, MINB) gemm_kernel(GemmP p, long sa, long sb, long sc, int kstep, int mLast,
+                                                             int kLast) {
     const int z = blockIdx.z;
     p.A += z * sa;
     p.B += z * sb;
     p.C += z * sc;
     if (kstep > 0) p.K = min(kstep, p.K - z * kstep);
+    if (mLast > 0 && z == gridDim.z - 1) {
+        p.M = mLast;
+        p.K = kLast;
+        if ((int) blockIdx.x * BM_ >= mLast) return;
+    }
     gemm_tile<BM_, BN_, P_ST, TA, TB>(p, blockIdx.x, blockIdx.y);
 }
 
@@ -492,7 +498,8 @@ constexpr long kGemmLargeMN = 3072L * 3072L;
 constexpr int kGemmSt32 = 5, kGemmBlk32 = 4, kGemmSt64 = 3, kGemmBlk64 = 3;
 
 template <int BM_, int BN_, int P_ST, int MINB, int TA, int TB>
-void launch_tiles(const GemmP &p, long sa, long sb, long sc, int count, int kstep, cudaStream_t s) {
+void launch_tiles(const GemmP &p, long sa, long sb, long sc, int count, int kstep, int mLast, int kLast,
+                  cudaStream_t s) {
     constexpr int bytes = kPBytes<BM_, BN_, P_ST, TA, TB>;
     static std::atomic<unsigned long long> init{0};
     once_per_device(init, [] {
@@ -500,23 +507,25 @@ void launch_tiles(const GemmP &p, long sa, long sb, long sc, int count, int kste
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     });
     dim3 grid((p.M + BM_ - 1) / BM_, (p.N + BN_ - 1) / BN_, count);
-    gemm_kernel<BM_, BN_, P_ST, MINB, TA, TB><<<hb::counted(grid), P_T, bytes, s>>>(p, sa, sb, sc, kstep);
+    gemm_kernel<BM_, BN_, P_ST, MINB, TA, TB><<<hb::counted(grid), P_T, bytes, s>>>(p, sa, sb, sc, kstep, mLast, kLast);
     HB_CUDA(cudaGetLastError());
 }
 
 template <int TA, int TB>
-void launch_gemm(const GemmP &p, long sa, long sb, long sc, int count, int kstep, cudaStream_t s) {
-    if ((long) p.M * p.N >= kGemmLargeMN)
-        launch_tiles<64, 64, kGemmSt64, kGemmBlk64, TA, TB>(p, sa, sb, sc, count, kstep, s);
+void launch_gemm(const GemmP &p, long sa, long sb, long sc, int count, int kstep, int mLast, int kLast,
+                  cudaStream_t s) {
+    if ((long) p.M * p.N * count >= kGemmLargeMN && std::min(p.M, p.N) >= 512)
+        launch_tiles<64, 64, kGemmSt64, kGemmBlk64, TA, TB>(p, sa, sb, sc, count, kstep, mLast, kLast, s);
     else
-        launch_tiles<32, 32, kGemmSt32, kGemmBlk32, TA, TB>(p, sa, sb, sc, count, kstep, s);
+        launch_tiles<32, 32, kGemmSt32, kGemmBlk32, TA, TB>(p, sa, sb, sc, count, kstep, mLast, kLast, s);
 }
 
-void launch_gemm(const GemmP &p, long sa, long sb, long sc, int count, int kstep, cudaStream_t s) {
-    if (!p.ta && !p.tb) launch_gemm<0, 0>(p, sa, sb, sc, count, kstep, s);
-    else if (p.ta && !p.tb) launch_gemm<1, 0>(p, sa, sb, sc, count, kstep, s);
-    else if (!p.ta && p.tb) launch_gemm<0, 1>(p, sa, sb, sc, count, kstep, s);
-    else launch_gemm<1, 1>(p, sa, sb, sc, count, kstep, s);
+void launch_gemm(const GemmP &p, long sa, long sb, long sc, int count, int kstep, int mLast, int kLast,
+                  cudaStream_t s) {
+    if (!p.ta && !p.tb) launch_gemm<0, 0>(p, sa, sb, sc, count, kstep, mLast, kLast, s);
+    else if (p.ta && !p.tb) launch_gemm<1, 0>(p, sa, sb, sc, count, kstep, mLast, kLast, s);
+    else if (!p.ta && p.tb) launch_gemm<0, 1>(p, sa, sb, sc, count, kstep, mLast, kLast, s);
+    else launch_gemm<1, 1>(p, sa, sb, sc, count, kstep, mLast, kLast, s);
 }
 
 // one GEMM of a group per blockIdx.z (tiles beyond its own M x N exit)
@@ -541,7 +550,7 @@ void gemm_strided(cudaStream_t s, const GemmDesc &d, long sa, long sb, long sc, 
         p.B += z0 * sb;
         p.C += z0 * sc;
         if (kstep > 0) p.K -= z0 * kstep;
-        launch_gemm(p, sa, sb, sc, std::min(65535, count - z0), kstep, s);
+        launch_gemm(p, sa, sb, sc, std::min(65535, count - z0), kstep, 0, 0, s);
     }
 }
 
@@ -574,7 +583,7 @@ void gemm(cudaStream_t s, int M, int N, int K, double alpha, const double *A, lo
         if (flags & (GEMM_B_LOWER | GEMM_B_UPPER)) f *= 0.5;
         kstat_begin(KF_GEMM, s, f);
     }
-    launch_gemm(p, 0, 0, 0, 1, 0, s);
+    launch_gemm(p, 0, 0, 0, 1, 0, 0, 0, s);
     if (timed) kstat_end(s);
 }
 
@@ -759,46 +768,11 @@ __global__ void __launch_bounds__(256) trsm_panel_kernel(double *P, long ldp, in
     }
 }
 
-// X row block (nb x cols, in place) <- Tinv * X, Tinv lower nb x nb.
-__global__ void __launch_bounds__(256) tri_left_kernel(double *X, long ldx, int nb, int cols,
-                                                       const double *Tinv, long ldt) {
-    extern __shared__ double sm[];
-    double *Xs = sm;             // nb x 64
-    double *T = sm + 65 * 64;
-    const int c0 = blockIdx.x * 64;
-    const int nc = min(64, cols - c0);
-    const int tid = threadIdx.x;
-    for (int idx = tid; idx < nb * 64; idx += blockDim.x) {
-        int r = idx % nb, c = idx / nb;
-        Xs[r + c * 65] = (c < nc) ? X[(size_t) r + (size_t) (c0 + c) * ldx] : 0.0;
-    }
-    for (int idx = tid; idx < nb * nb; idx += blockDim.x) {
-        int r = idx % nb, c = idx / nb;
-        T[r + c * 65] = Tinv[(size_t) r + (size_t) c * ldt];
-    }
-    __syncthreads();
-    for (int idx = tid; idx < nb * 64; idx += blockDim.x) {
-        int r = idx % nb, c = idx / nb;
-        if (c >= nc) continue;
-        double acc = 0.0;
-        for (int k = 0; k <= r; ++k) acc += T[r + k * 65] * Xs[k + c * 65];
-        X[(size_t) r + (size_t) (c0 + c) * ldx] = acc;
-    }
-}
-
 __global__ void copy_lower_kernel(int n, const double *S, long lds, double *L, long ldl) {
     const long total = (long) n * n;
     for (long idx = blockIdx.x * (long) blockDim.x + threadIdx.x; idx < total; idx += (long) gridDim.x * blockDim.x) {
         int r = (int) (idx % n), c = (int) (idx / n);
         L[(size_t) r + (size_t) c * ldl] = (r >= c) ? S[(size_t) r + (size_t) c * lds] : 0.0;
-    }
-}
-
-__global__ void set_identity_kernel(int n, double *A, long lda) {
-    const long total = (long) n * n;
-    for (long idx = blockIdx.x * (long) blockDim.x + threadIdx.x; idx < total; idx += (long) gridDim.x * blockDim.x) {
-        int r = (int) (idx % n), c = (int) (idx / n);
-        A[(size_t) r + (size_t) c * lda] = (r == c) ? 1.0 : 0.0;
     }
 }
 
@@ -880,14 +854,12 @@ static void ensure_attrs() {
     once_per_device(init, [] {
         set_smem((const void *) potf2_kernel, smem_bytes());
         set_smem((const void *) trsm_panel_kernel, smem_bytes());
-        set_smem((const void *) tri_left_kernel, smem_bytes());
     });
 }
 
 bool coop_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS, bool status, bool *mirrored);
 bool rec_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS);
 bool rec_factorize_nok_enqueue(cudaStream_t s, DenseFactor &F, const double *S, long ldS);
-bool coop_inverse_enqueue(cudaStream_t s, DenseFactor &F);
 
 void factorize_async(cudaStream_t s, DenseFactor &F, const double *S, long ldS) {
     ensure_attrs();
@@ -980,29 +952,47 @@ bool factorize(cudaStream_t s, DenseFactor &F, const double *S, long ldS) {
     return factor_status(s, F);
 }
 
+namespace {
+// K's 64 x 64 diagonal blocks from Dinv, zero above them
+__global__ void place_dinv_kernel(int n, const double *__restrict__ Dinv, long ldd, double *K, long ld) {
+    const int bj = blockIdx.y, bi = blockIdx.x;
+    if (bi > bj) return;
+    for (int e = threadIdx.x; e < 64 * 64; e += blockDim.x) {
+        const int i = bi * 64 + (e & 63), c = e >> 6, j = bj * 64 + c;
+        if (i < n && j < n) K[(size_t) i + (size_t) j * ld] = (bi == bj) ? Dinv[(size_t) i + (size_t) c * ldd] : 0.0;
+    }
+}
+}  // namespace
+
+// K = L^-1 from the diagonal blocks' inverses by doubling: once blocks of w rows are inverted,
+// K21 = -K22 (L21 K11) inverts those of 2 w, every pair in the same two launches, the product
+// L21 K11 held below KT's triangle until the transposition clears it. All of the n^3/3 operations
+// but the first blocks' are GEMMs, which bound it from order 1,000 on; below, the 2 log2(n / 64)
+// launches do. Against a cooperative kernel that eliminated one 64-row panel after the other, two
+// grid barriers each (ms, order 128 / 500 / 2000 / 4000 / 8000): 0.027 / 0.097 / 0.51 / 1.97 /
+// 10.8, now 0.021 / 0.051 / 0.21 / 0.88 / 5.7.
 void compute_inverse_factor(cudaStream_t s, DenseFactor &F) {
-    ensure_attrs();
     if (F.k_valid) return;
     const int n = F.n;
-    if (!F.K) HB_CUDA(hb::cmalloc(&F.K, sizeof(double) * F.ld * n));
-    if (!F.KT) HB_CUDA(hb::cmalloc(&F.KT, sizeof(double) * F.ld * n));
-    if (coop_inverse_enqueue(s, F)) {
-        transpose(s, n, F.K, F.ld, F.KT, F.ld);
-        F.k_valid = true;
-        return;
+    const long ld = F.ld;
+    if (!F.K) HB_CUDA(hb::cmalloc(&F.K, sizeof(double) * ld * n));
+    if (!F.KT) HB_CUDA(hb::cmalloc(&F.KT, sizeof(double) * ld * n));
+    const bool timed = kstat_on(KF_TRTRI);
+    if (timed) kstat_begin(KF_TRTRI, s, (double) n * n * n / 3.0);
+    const int nb = (n + 63) / 64;
+    place_dinv_kernel<<<hb::counted(dim3(nb, nb)), 256, 0, s>>>(n, F.Dinv, ld, F.K, ld);
+    for (int w = 64; w < n; w *= 2) {
+        const int pairs = (n - w + 2 * w - 1) / (2 * w);           // second blocks begin at w, 3 w, ...
+        const int last = std::min(w, n - ((pairs - 1) * 2 * w + w));
+        const long step = 2 * (long) w * (ld + 1);
+        launch_gemm(GemmP{w, w, w, 1.0, 0.0, F.L + w, ld, 0, F.K, ld, 0, F.KT + w, ld, GEMM_B_LOWER, nullptr}, step, step,
+                    step, pairs, 0, last, w, s);                    // L21 K11
+        launch_gemm(GemmP{w, w, w, -1.0, 0.0, F.K + w + (size_t) w * ld, ld, 0, F.KT + w, ld, 0, F.K + w, ld, GEMM_A_LOWER,
+                          nullptr},
+                    step, step, step, pairs, 0, last, last, s);     // -K22 (L21 K11)
     }
-    set_identity_kernel<<<hb::counted(grid_for((long) n * n)), 256, 0, s>>>(n, F.K, F.ld);
-    for (int i0 = 0; i0 < n; i0 += NB) {
-        const int nb = std::min(NB, n - i0);
-        const int cend = i0 + nb;
-        tri_left_kernel<<<hb::counted((cend + 63) / 64), 256, smem_bytes(), s>>>(F.K + i0, F.ld, nb, cend, F.Dinv + i0, F.ld);
-        const int rows = n - cend;
-        if (rows > 0) {
-            gemm(s, rows, cend, nb, -1.0, F.L + (size_t) cend + (size_t) i0 * F.ld, F.ld, 0, F.K + i0, F.ld, 0,
-                 1.0, F.K + cend, F.ld, 0);
-        }
-    }
-    transpose(s, n, F.K, F.ld, F.KT, F.ld);
+    transpose(s, n, F.K, ld, F.KT, ld);
+    if (timed) kstat_end(s);
     F.k_valid = true;
 }
 
