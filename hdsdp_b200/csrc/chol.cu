@@ -1383,8 +1383,7 @@ bool rec_factorize_nok_enqueue(cudaStream_t s, DenseFactor &F, const double *S, 
         F.d_rec_info = nullptr;
         return false;
     }
-    if (!F.d_rec_w && hb::cmalloc(&F.d_rec_w, sizeof(double) * F.ld * std::max((n + 1) / 2, kRecLeafMaxN)) !=
-                          cudaSuccess) {
+    if (!F.d_rec_w && hb::cmalloc(&F.d_rec_w, sizeof(double) * strip) != cudaSuccess) {
         F.d_rec_w = nullptr;
         return false;
     }
@@ -1462,9 +1461,81 @@ bool small_factor_batch_enqueue(cudaStream_t s, DenseFactor *const *F, const dou
     return cudaGetLastError() == cudaSuccess;
 }
 
+namespace {
+// y -= A x (rows x cols, column-major): 32 rows a block, its warps taking the columns in turn
+constexpr int kGemvThreads = 1024;
+__global__ void __launch_bounds__(kGemvThreads)
+    gemv_sub_kernel(int rows, int cols, const double *__restrict__ A, long lda, const double *__restrict__ x, double *y) {
+    __shared__ double part[32][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = blockIdx.x * 32 + lane;
+    double p[4] = {};
+    if (r < rows) {
+        const double *a = A + r;
+        int c = w;
+        for (; c + 96 < cols; c += 128) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) p[q] += __ldg(a + (size_t) (c + 32 * q) * lda) * __ldg(x + c + 32 * q);
+        }
+        for (int q = 0; c < cols; c += 32, ++q) p[q] += __ldg(a + (size_t) c * lda) * __ldg(x + c);
+    }
+    part[w][lane] = (p[0] + p[1]) + (p[2] + p[3]);
+    __syncthreads();
+    // warp w sums row w of the block
+    double v = part[lane][w];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const int row = blockIdx.x * 32 + w;
+    if (lane == 0 && row < rows) y[row] -= v;
+}
+
+// the diagonal blocks of the recursive factorisation, in order
+void rec_leaves(int off, int n, std::vector<std::pair<int, int>> &out) {
+    if (n <= kRecLeafMaxN) {
+        out.push_back({off, n});
+        return;
+    }
+    const int n1 = rec_split(n);
+    rec_leaves(off, n1, out);
+    rec_leaves(off + n1, n - n1, out);
+}
+
+// Substitution by the diagonal blocks of the recursive factorisation, with their inverses from
+// the strips: a block is a product with K and one with the rows (columns) of L below it. The two
+// passes over L bound it (order 8000: 80 us of DRAM time); 64-row blocks in one cooperative
+// launch are a chain of 2 n / 64 waits (order 4485 / 6000 / 8000: 684 / 972 / 1300 us, now 130 / 160 /
+// 314).
+bool rec_solve(cudaStream_t s, DenseFactor &F, const double *b, double *x) {
+    const int n = F.n;
+    const long ld = F.ld;
+    std::vector<std::pair<int, int>> leaf;
+    rec_leaves(0, n, leaf);
+    double *t = F.d_tmp;
+    HB_CUDA(cudaMemcpyAsync(t, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+    for (auto [o, m] : leaf) {   // x <- L^-1 b, t the right-hand side left
+        coldot(s, m, m, F.d_rec_kts + o, ld, t + o, x + o, 1.0, 0.0, 2);
+        const int rows = n - o - m;
+        if (rows > 0)
+            gemv_sub_kernel<<<hb::counted((rows + 31) / 32), kGemvThreads, 0, s>>>(
+                rows, m, F.L + (o + m) + (size_t) o * ld, ld, x + o, t + o + m);
+    }
+    for (size_t q = leaf.size(); q-- > 0;) {   // t <- L^-T x
+        const auto [o, m] = leaf[q];
+        const int rows = n - o - m;
+        if (rows > 0) coldot(s, rows, m, F.L + (o + m) + (size_t) o * ld, ld, t + o + m, x + o, -1.0, 1.0, 0);
+        coldot(s, m, m, F.d_rec_ks + o, ld, x + o, t + o, 1.0, 0.0, 1);
+    }
+    HB_CUDA(cudaMemcpyAsync(x, t, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+    return cudaGetLastError() == cudaSuccess;
+}
+}  // namespace
+
 bool chol_solve(cudaStream_t s, DenseFactor &F, const double *b, double *x) {
     const int n = F.n;
     if (n <= 0) return true;
+    if (F.rec_strips) {
+        if (!F.d_tmp) HB_CUDA(hb::cmalloc(&F.d_tmp, sizeof(double) * n));
+        return F.d_tmp && rec_solve(s, F, b, x);
+    }
     const int nblk = (n + 63) / 64;
     if (!F.d_flags) {
         HB_CUDA(hb::cmalloc(&F.d_flags, sizeof(unsigned) * 2 * nblk));

@@ -866,6 +866,7 @@ void factorize_async(cudaStream_t s, DenseFactor &F, const double *S, long ldS) 
     const int n = F.n;
     F.k_valid = false;
     F.k_pending = false;
+    F.rec_strips = false;
     F.factored = true;
     F.logdet_valid = false;
     // info word (and sum log L_ii) back to the host in one copy
@@ -884,6 +885,7 @@ void factorize_async(cudaStream_t s, DenseFactor &F, const double *S, long ldS) 
     }
     if (!F.fuse_k && !F.no_rec && n > kRecNoKMinN && rec_factorize_nok_enqueue(s, F, S, ldS)) {
         F.k_pending = false;
+        F.rec_strips = true;
         status_copy();
         return;
     }

@@ -80,18 +80,20 @@ void ldl_solve(cudaStream_t s, LdlFactor &F, const double *b, double *x);
 // L holds the lower Cholesky factor, Dinv the inverses of its 64 x 64
 // diagonal blocks, K = L^-1 and KT = L^-T (computed on demand).
 constexpr int kFuseInverseMax = 2048;
-// Above kRecMinN a factorisation that also forms K = L^-1 (the Schur matrix below 6000 rows)
-// takes the recursive blocked form: the two diagonal halves (recursively, down to blocks of
+// Above kRecMinN a factorisation that also forms K = L^-1 (the Schur matrix below kTriSolveMinM
+// rows) takes the recursive blocked form: the two diagonal halves (recursively, down to blocks of
 // at most kRecLeafMaxN rows) on the cooperative kernel with their own K, the off-diagonal
-// work as FP64 GEMMs. Measured on B200 (factor and K, ms): order 3595 3.13 one launch
-// against 3.22 recursive, 4096 4.25 / 3.79, 5120 7.48 / 6.36, 5999 11.6 / 9.98.
-constexpr int kRecMinN = 3840;
-constexpr int kRecLeafMaxN = 2560;
+// work as FP64 GEMMs. Measured on B200 (factor and K, ms, one launch against recursive): order
+// 2048 0.756 / 0.764, 2500 1.21 / 1.11, 3000 1.71 / 1.49, 4485 4.56 / 3.39, 6000 9.67 / 6.57. Leaves
+// of at most 1280 and 2100 rows: 6000 6.69 and 6.57, 8000 13.36 and 13.55 (1600: 13.36).
+constexpr int kRecMinN = 2048;
+constexpr int kRecLeafMaxN = 1600;
 // Above kRecNoKMinN a factorisation without K takes the recursive form too: L21 = A21 L11^-T
 // by a recursive triangular solve whose leaves are GEMMs with the diagonal blocks' own K
-// (kept in an n x kRecLeafMaxN strip). Measured on B200 (factor only, ms, one launch against
-// recursive): order 6016 5.62 / 6.67, 8000 11.8 / 11.7, 12000 36.8 / 31.2, 16000 83.9 / 64.4.
-constexpr int kRecNoKMinN = 8192;
+// (kept in an n x kRecLeafMaxN strip, where chol_solve finds them). Measured on B200 (factor
+// only, ms, one launch against recursive): order 3000 1.09 / 1.22, 4000 2.00 / 1.88, 4485 2.62 /
+// 2.38, 6000 5.24 / 4.31, 8000 11.1 / 7.96.
+constexpr int kRecNoKMinN = 3584;
 
 // A factor's status words on the device: the info word, 8 bytes on sum log L_ii, then the
 // cooperative kernel's counters (from int kInfoCounters on), cleared by every factorisation.
@@ -132,6 +134,7 @@ struct DenseFactor {
     int *d_rec_info = nullptr;
     double *d_rec_w = nullptr;
     double *d_rec_ks = nullptr, *d_rec_kts = nullptr;   // the diagonal blocks' K and K^T (no-K form)
+    bool rec_strips = false;  // the strips belong to the last factorisation
     bool no_rec = false;      // keep the one-launch factorisation at every order (timing)
     int kfamily = KF_POTRF;   // kernel-timing family of this factor's factorisations
     void alloc(int n_, int fuse_inverse = -1);
