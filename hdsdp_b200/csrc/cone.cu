@@ -1586,19 +1586,45 @@ __global__ void lanczos_resid_kernel(int n, double *z, const double *x, double l
     if (threadIdx.x == 0) *out = v;
 }
 
-// ---- Lanczos steps of larger blocks in one cooperative launch per check interval.
-//
-// Steps k0 .. k1-1 of the three-term recurrence for M = K (-D) K^T (K = L^-1 lower,
-// KT = K^T), taken exactly as lanczos_orth_kernel takes them (w = M v_k - beta v_{k-1},
-// alpha = w.v_k, w -= alpha v_k, beta = |w|, v_{k+1} = w / beta when beta > 0). Block b
-// owns columns [b*cpb, (b+1)*cpb) of every product and reduces each column with
-// kLzWpc warps; the dot products go through per-block partial sums that every block
-// adds up in the same order, so all blocks hold the same alpha and beta. Four grid-wide
-// barriers per step. Values written inside the launch are read with ld.global.cg.
-constexpr int kLzThreads = 1024, kLzWpc = 4;
-constexpr int kLzCols = kLzThreads / 32 / kLzWpc;   // columns per block and pass
-constexpr int kLzSmemMax = 200 * 1024;              // dynamic shared memory of the cached variant
-constexpr int kLzFusedMaxN = 2048;                  // K, K^T and D (3 x 8 n^2 bytes) still fit the L2
+// ---- D by its entries. The step matrix of a sparse cone has few: a pass over it lists each
+// column's (in row order), and every product with it afterwards reads the lists instead of n^2
+// entries. Only where no column has more than kLzListMax; *flag == epoch says that one has.
+constexpr int kLzListMax = 64;
+struct LzList {
+    int *cnt = nullptr, *idx = nullptr;   // entries of column j: idx / val[j kLzListMax ..)
+    double *val = nullptr;
+    unsigned *flag = nullptr;
+    unsigned epoch = 0;
+};
+
+__global__ void lz_list_kernel(int n, const double *__restrict__ D, long ldD, LzList S) {
+    const int lane = threadIdx.x & 31;
+    const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (j >= n) return;
+    const double *col = D + (size_t) j * ldD;
+    int c = 0;
+    for (int i0 = 0; i0 < n; i0 += 256) {
+        double x[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[q] = (i0 + 32 * q + lane < n) ? __ldg(col + i0 + 32 * q + lane) : 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const unsigned m = __ballot_sync(0xffffffffu, x[q] != 0.0);   // a NaN is an entry too
+            if (!m) continue;
+            const int at = c + __popc(m & ((1u << lane) - 1));
+            if (x[q] != 0.0 && at < kLzListMax) {
+                S.idx[(size_t) j * kLzListMax + at] = i0 + 32 * q + lane;
+                S.val[(size_t) j * kLzListMax + at] = x[q];
+            }
+            c += __popc(m);
+        }
+        if (c > kLzListMax) {
+            if (lane == 0) *(volatile unsigned *) S.flag = S.epoch;
+            return;
+        }
+    }
+    if (lane == 0) S.cnt[j] = c;
+}
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -1606,267 +1632,246 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// out[j] = scale * sum_i A(i, j) x[i] over the rows of column j that `mode` keeps
-// (0 all, 1 i >= j, 2 i <= j), for the block's columns [j0, j1).
-__device__ void lz_block_coldot(int n, const double *__restrict__ A, long lda, const double *x, double *out,
-                                double scale, int mode, int j0, int j1, double *red) {
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cslot = w / kLzWpc, seg = w % kLzWpc;
-    for (int jb = j0; jb < j1; jb += kLzCols) {
-        const int j = jb + cslot;
-        double acc = 0.0;
-        if (j < j1) {
-            const int lo = (mode == 1) ? j : 0, hi = (mode == 2) ? j + 1 : n;
-            const int len = hi - lo;
-            const int chunk = (((len + kLzWpc - 1) / kLzWpc) + 31) & ~31;
-            const int a0 = lo + seg * chunk, a1 = min(hi, a0 + chunk);
-            const double *col = A + (size_t) j * lda;
-            int k = a0 + lane;
-            for (; k + 32 < a1; k += 64) acc += __ldg(col + k) * __ldcg(x + k) + __ldg(col + k + 32) * __ldcg(x + k + 32);
-            for (; k < a1; k += 32) acc += __ldg(col + k) * __ldcg(x + k);
-        }
-        acc = warp_sum(acc);
-        if (lane == 0) red[w] = acc;
-        __syncthreads();
-        if (threadIdx.x < kLzCols && jb + (int) threadIdx.x < j1) {
-            double t = 0.0;
-#pragma unroll
-            for (int q = 0; q < kLzWpc; ++q) t += red[threadIdx.x * kLzWpc + q];
-            out[jb + threadIdx.x] = scale * t;
-        }
-        __syncthreads();
-    }
+// this lane's share of sum_i D(i, j) x[i] over column j's list
+__device__ __forceinline__ double lz_list_dot(const LzList &S, int j, const double *x) {
+    const int lane = threadIdx.x & 31, c = __ldcg(S.cnt + j);
+    double p = 0.0;
+    for (int e = lane; e < c; e += 32) p += __ldcg(S.val + (size_t) j * kLzListMax + e) * x[__ldcg(S.idx + (size_t) j * kLzListMax + e)];
+    return p;
 }
 
-// sum of part[0 .. G) in a fixed order, the same in every block
-__device__ double lz_grid_sum(const double *part, int G, double *red) {
-    if (threadIdx.x < 32) {
-        double v = 0.0;
-        for (int q = threadIdx.x; q < G; q += 32) v += __ldcg(part + q);
-        v = warp_sum(v);
-        if (threadIdx.x == 0) red[0] = v;
+// out = -D x by the lists, or by whole columns where one was too long; a warp per column
+__global__ void lz_list_mv_kernel(int n, const double *__restrict__ D, long ldD, LzList S, const double *__restrict__ x,
+                                  double *out) {
+    const int lane = threadIdx.x & 31, j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (j >= n) return;
+    double acc = 0.0;
+    if (*S.flag != S.epoch) {
+        acc = lz_list_dot(S, j, x);
+    } else {
+        const double *col = D + (size_t) j * ldD;
+        int k = lane;
+        for (; k + 96 < n; k += 128) acc += col[k] * x[k] + col[k + 32] * x[k + 32] + col[k + 64] * x[k + 64] + col[k + 96] * x[k + 96];
+        for (; k < n; k += 32) acc += col[k] * x[k];
     }
-    __syncthreads();
-    const double v = red[0];
-    __syncthreads();
-    return v;
+    acc = warp_sum(acc);
+    if (lane == 0) out[j] = -acc;
 }
 
-// The block's columns held in shared memory for the whole launch: region K (column j,
-// rows j..n-1), region KT (rows 0..j), region D (rows 0..n-1), packed column after column;
-// a block with cpb columns holds cpb (2n + 1) doubles. Local column c starts at
-// c (n - j0) - c (c - 1) / 2 in K, c (j0 + 1) + c (c - 1) / 2 in KT and c n in D.
+// ---- Lanczos steps of larger blocks, all steps up to a check in one cooperative launch.
+//
+// Steps k0 .. k1-1 of the three-term recurrence for M = K (-D) K^T (K = L^-1 lower,
+// KT = K^T), taken exactly as lanczos_orth_kernel takes them (w = M v_k - beta v_{k-1},
+// alpha = w.v_k, w -= alpha v_k, beta = |w|, v_{k+1} = w / beta when beta > 0); step 0 starts
+// from normalise(a + b) (a may be null). Block b owns columns [b cpb, (b + 1) cpb) of every
+// product and reduces each by kLzThreads / 32 / cpb warps. As many of its columns as fit stay in
+// shared memory for the whole launch (K's, K^T's and, unless D goes by its lists, D's; the rest
+// is read from L2 in every step). Every block holds v_k, v_{k-1} and w whole and forms alpha and
+// beta itself, all in the same order, so these need no exchange.
+// What bounds a step is the exchange of t = K^T v, u = -D t and w between the blocks. A grid barrier and the load of the vector behind it take 2.5 us each, so there is none:
+// every number travels with its tag in one 16-byte word, and who needs it polls that word. A word
+// is not written again before every block has used it, because no block gets to its next tag
+// without the others' later words of this one. Every poll is bounded; on giving up a block sets
+// the error word of ab and returns, and the others give up on its words. Us a step, order 500 /
+// 1000 / 2001 (diagonal D): 7.7 / 10 / 13; with a grid barrier for each exchange 17 / 17 / 21, and with
+// launches of three steps and every column of D read 13 / 14 / 34 before.
+constexpr int kLzThreads = 1024, kLzWarps = kLzThreads / 32;
+constexpr int kLzFusedMaxN = 2 * kLzThreads;
+constexpr int kLzMaxSegs = 8;                 // warps per column, at most
+constexpr int kLzPollLimit = 1 << 20;
+
+// K's column j below the diagonal and K^T's above it: n + 1 entries, whatever j
 __host__ __device__ inline long lz_cached_doubles(int n, int cpb) { return (long) cpb * (2L * n + 1); }
 
-// w -= beta_{k-1} v_{k-1} and the block's partial w.v_k into part[blockIdx.x]
-__device__ void lz_orth_partial(int j0, int j1, int k, const double *V, long ldv, const double *ab, int maxdim,
-                                double *w, double *part, double *red) {
-    const double *vk = V + (size_t) k * ldv;
-    const double bprev = (k > 0) ? __ldcg(ab + maxdim + k - 1) : 0.0;
-    double pa = 0.0;
-    for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-        double x = w[j];
-        if (k > 0) x -= bprev * __ldcg(V + (size_t) (k - 1) * ldv + j);
-        w[j] = x;
-        pa += x * __ldcg(vk + j);
-    }
-    pa = warp_sum(pa);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = pa;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double v = 0.0;
-        for (int q = 0; q < kLzThreads / 32; ++q) v += red[q];
-        part[blockIdx.x] = v;
-    }
+// a number and its tag, written and read as one word
+struct __align__(16) LzWord {
+    double x;
+    unsigned long long tag;
+};
+__device__ __forceinline__ void lz_put(LzWord *p, double x, unsigned long long tag) {
+    asm volatile("{.reg .b128 r;\n mov.b128 r, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], r;}" ::"l"(p),
+                 "l"(__double_as_longlong(x)), "l"(tag)
+                 : "memory");
+}
+__device__ __forceinline__ bool lz_get(const LzWord *p, double &x, unsigned long long tag) {
+    long long lo;
+    unsigned long long hi;
+    asm volatile("{.reg .b128 r;\n ld.relaxed.gpu.global.b128 r, [%2];\n mov.b128 {%0, %1}, r;}"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(p)
+                 : "memory");
+    x = __longlong_as_double(lo);
+    return hi == tag;
 }
 
-// w -= alpha v_k and the block's partial |w|^2 into part[G + blockIdx.x]
-__device__ void lz_norm_partial(int j0, int j1, int k, double alp, const double *V, long ldv, double *w, double *part,
-                                int G, double *red) {
-    const double *vk = V + (size_t) k * ldv;
-    double pn = 0.0;
-    for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-        const double x = w[j] - alp * __ldcg(vk + j);
-        w[j] = x;
-        pn += x * x;
-    }
-    pn = warp_sum(pn);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = pn;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double v = 0.0;
-        for (int q = 0; q < kLzThreads / 32; ++q) v += red[q];
-        part[G + blockIdx.x] = v;
-    }
-}
-
-// v_{k+1} = w / beta over the block's columns; alpha and beta recorded by block 0
-__device__ void lz_next(int j0, int j1, int k, double alp, double nrm, double *V, long ldv, double *ab, int maxdim,
-                        const double *w) {
-    if (nrm > 0.0) {
-        double *vn = V + (size_t) (k + 1) * ldv;
-        for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) vn[j] = w[j] / nrm;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ab[k] = alp;
-        if (nrm > 0.0) ab[maxdim + k] = nrm;
-    }
-}
-
-// Streaming variant: the block's columns of K, K^T and D are read from L2 in every step.
 __global__ void __launch_bounds__(kLzThreads, 1)
-    lanczos_steps_kernel(int n, const double *K, const double *KT, long ldk, const double *D, long ldD, double *V,
-                         long ldv, double *ab, int maxdim, int k0, int k1, double *t, double *u, double *w,
-                         double *part) {
-    cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-    __shared__ double red[kLzThreads / 32];
-    const int G = gridDim.x;
-    const int cpb = (n + G - 1) / G;
-    const int j0 = min(n, (int) blockIdx.x * cpb), j1 = min(n, j0 + cpb);
-    for (int k = k0; k < k1; ++k) {
-        const double *vk = V + (size_t) k * ldv;
-        lz_block_coldot(n, K, ldk, vk, t, 1.0, 1, j0, j1, red);     // t = K^T v_k
-        grid.sync();
-        lz_block_coldot(n, D, ldD, t, u, -1.0, 0, j0, j1, red);     // u = -D t
-        grid.sync();
-        lz_block_coldot(n, KT, ldk, u, w, 1.0, 2, j0, j1, red);     // w = K u
-        lz_orth_partial(j0, j1, k, V, ldv, ab, maxdim, w, part, red);
-        grid.sync();
-        const double alp = lz_grid_sum(part, G, red);
-        lz_norm_partial(j0, j1, k, alp, V, ldv, w, part, G, red);
-        grid.sync();
-        const double nrm = sqrt(lz_grid_sum(part + G, G, red));
-        lz_next(j0, j1, k, alp, nrm, V, ldv, ab, maxdim, w);
-        grid.sync();
-    }
-}
-
-// Shared-memory variant (n small enough for a block's share of columns to fit): the
-// block's columns of K, K^T and D are loaded into shared memory once per launch
-// (lz_cached_doubles(n, cpb) doubles) and each product's input vector is staged there (n
-// more doubles); kLzWpc warps reduce each column. v_{k+1} = w / beta is read by the next
-// step's first product straight from w (the last grid barrier of a step publishes w, and
-// every block holds beta), so a step takes four grid-wide barriers.
-__global__ void __launch_bounds__(kLzThreads, 1)
-    lanczos_steps_smem_kernel(int n, const double *K, const double *KT, long ldk, const double *D, long ldD,
-                              double *V, long ldv, double *ab, int maxdim, int k0, int k1, double *w, double *tg,
-                              double *ug, double *part) {
-    cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-    __shared__ double red[kLzThreads / 32];
-    __shared__ double scal[2];
+    lz_grid_steps_kernel(int n, const double *K, const double *KT, long ldk, const double *D, long ldD, LzList S,
+                         const double *a, const double *b, double *V, long ldv, double *ab, double *hab, int maxdim,
+                         int k0, int k1, LzWord *words, unsigned long long tag, long cacheDoubles) {
+    __shared__ double red[kLzWarps];
+    __shared__ int lost;
     extern __shared__ double dyn[];
     const int G = gridDim.x;
     const int cpb = (n + G - 1) / G;
-    const int j0 = min(n, (int) blockIdx.x * cpb), j1 = min(n, j0 + cpb);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = kLzThreads / 32;
-    const long nc = j1 - j0;
-    double *sK = dyn;
-    double *sKT = sK + (nc * (n - j0) - nc * (nc - 1) / 2);
-    double *sD = sKT + (nc * (j0 + 1) + nc * (nc - 1) / 2);
-    double *sx = dyn + lz_cached_doubles(n, cpb);
-    for (long c = 0; c < nc; ++c) {
-        const int j = j0 + (int) c;
-        double *dk = sK + c * (n - j0) - c * (c - 1) / 2;
-        double *dkt = sKT + c * (j0 + 1) + c * (c - 1) / 2;
-        double *dd = sD + c * n;
-        const double *gk = K + (size_t) j * ldk, *gkt = KT + (size_t) j * ldk, *gd = D + (size_t) j * ldD;
-        for (int i = j + threadIdx.x; i < n; i += blockDim.x) dk[i - j] = __ldg(gk + i);
-        for (int i = threadIdx.x; i <= j; i += blockDim.x) dkt[i] = __ldg(gkt + i);
-        for (int i = threadIdx.x; i < n; i += blockDim.x) dd[i] = __ldg(gd + i);
+    const int j0 = min(n, (int) blockIdx.x * cpb), nc = min(n, j0 + cpb) - j0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    LzWord *wt = words, *wu = wt + n, *ww = wu + n;
+    const bool list = S.cnt && *S.flag != S.epoch;
+    double *sx = dyn, *cache = dyn + n;
+    const long per = (list ? 1L : 2L) * n + 1;
+    const int cc = (int) min((long) nc, cacheDoubles / per);   // cached columns
+    if (tid == 0) lost = 0;
+    if (blockIdx.x == 0 && tid == 0 && k0 == 0) {
+        ab[2 * maxdim + 1] = 0.0;
+        if (hab) hab[2 * maxdim + 1] = 0.0;
     }
-    // sx = x / div (div 0: zeros; the same division that forms v_{k+1})
-    auto stage = [&](const double *x, double div) {
-        for (int i = threadIdx.x; i < n; i += blockDim.x)
-            sx[i] = (div == 1.0) ? __ldcg(x + i) : (div > 0.0) ? __ldcg(x + i) / div : 0.0;
+    for (int c = warp; c < cc; c += kLzWarps) {
+        const int j = j0 + c;
+        double *dk = cache + c * per, *dkt = dk + (n - j), *dd = dkt + j + 1;
+        const double *gk = K + (size_t) j * ldk, *gkt = KT + (size_t) j * ldk, *gd = D + (size_t) j * ldD;
+#pragma unroll 8
+        for (int i = j + lane; i < n; i += 32) dk[i - j] = __ldg(gk + i);
+#pragma unroll 8
+        for (int i = lane; i <= j; i += 32) dkt[i] = __ldg(gkt + i);
+        if (!list) {
+#pragma unroll 8
+            for (int i = lane; i < n; i += 32) dd[i] = __ldg(gd + i);
+        }
+    }
+    // sum over rows lo <= i < hi of col[i] sx[i], this lane's share of segment seg of wpc
+    const int wpc = min(kLzMaxSegs, kLzWarps / cpb), slot = warp / wpc, seg = warp % wpc;
+    auto dot = [&](const double *col, int lo, int hi) {
+        const int chunk = (((hi - lo + wpc - 1) / wpc) + 31) & ~31;
+        const int e = min(hi, lo + (seg + 1) * chunk);
+        double p[4] = {}, y[8];
+        int i = lo + seg * chunk + lane;
+        for (; i + 224 < e; i += 256) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) y[q] = col[i + 32 * q];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) p[q & 3] += y[q] * sx[i + 32 * q];
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) y[q] = (i + 32 * q < e) ? col[i + 32 * q] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (i + 32 * q < e) p[q & 3] += y[q] * sx[i + 32 * q];
+        return (p[0] + p[2]) + (p[1] + p[3]);
+    };
+    // the block's columns of one product (mode 0: D, 1: K below the diagonal, 2: K^T above it),
+    // column c's sum to thread c of the first warp; the next call comes behind a barrier
+    auto product = [&](int mode) {
+        const int c = slot, j = j0 + c;
+        double acc = 0.0;
+        if (c < nc) {
+            if (mode == 0 && list) {
+                if (seg == 0) acc = lz_list_dot(S, j, sx);
+            } else {
+                const int lo = (mode == 1) ? j : 0, hi = (mode == 2) ? j + 1 : n;
+                if (c < cc) {
+                    const double *dk = cache + c * per;
+                    acc = dot((mode == 1) ? dk - j : (mode == 2) ? dk + (n - j) : dk + (n + 1), lo, hi);
+                } else {
+                    acc = dot((mode == 1) ? K + (size_t) j * ldk : (mode == 2) ? KT + (size_t) j * ldk : D + (size_t) j * ldD,
+                              lo, hi);
+                }
+            }
+        }
+        acc = warp_sum(acc);
+        if (lane == 0) red[warp] = acc;
+        __syncthreads();
+        double mine = 0.0;
+        if (warp == 0 && lane < nc) {
+#pragma unroll
+            for (int q = 0; q < kLzMaxSegs; ++q)
+                if (q < wpc) mine += red[lane * wpc + q];
+        }
+        return mine;
+    };
+    auto give_up = [&]() {
+        lost = 1;
+        ab[2 * maxdim + 1] = 1.0;
+        if (hab) hab[2 * maxdim + 1] = 1.0;
+    };
+    // this thread's entries of a vector (n <= 2 kLzThreads) once they carry the tag
+    auto fetch = [&](const LzWord *p, unsigned long long tg) {
+        double2 v = make_double2(0.0, 0.0);
+        bool a0 = tid >= n, a1 = tid + kLzThreads >= n;
+        for (int it = 0; it < kLzPollLimit; ++it) {
+            if (!a0) a0 = lz_get(p + tid, v.x, tg);
+            if (!a1) a1 = lz_get(p + tid + kLzThreads, v.y, tg);
+            if (a0 && a1) return v;
+        }
+        give_up();
+        return v;
+    };
+    auto put = [&](double2 v) {
+        if (tid < n) sx[tid] = v.x;
+        if (tid + kLzThreads < n) sx[tid + kLzThreads] = v.y;
         __syncthreads();
     };
-    // out[j] = scale * sum over the rows `mode` keeps (0 all, 1 i >= j, 2 i <= j) of column j
-    const int cslot = warp / kLzWpc, seg = warp % kLzWpc;
-    auto coldot = [&](int mode, const double *reg, double *out, double scale) {
-        for (int jb = j0; jb < j1; jb += kLzCols) {
-            const int j = jb + cslot;
-            double acc = 0.0;
-            if (j < j1) {
-                const long c = j - j0;
-                const int lo = (mode == 1) ? j : 0, hi = (mode == 2) ? j + 1 : n;
-                const double *col = (mode == 1)   ? reg + c * (n - j0) - c * (c - 1) / 2 - lo
-                                    : (mode == 2) ? reg + c * (j0 + 1) + c * (c - 1) / 2
-                                                  : reg + c * n;
-                const int len = hi - lo;
-                const int chunk = (((len + kLzWpc - 1) / kLzWpc) + 31) & ~31;
-                const int a0 = lo + seg * chunk, a1 = min(hi, a0 + chunk);
-                for (int k = a0 + lane; k < a1; k += 32) acc += col[k] * sx[k];
-            }
-            acc = warp_sum(acc);
-            if (lane == 0) red[warp] = acc;
-            __syncthreads();
-            if (threadIdx.x < kLzCols && jb + (int) threadIdx.x < j1) {
-                double t = 0.0;
-#pragma unroll
-                for (int q = 0; q < kLzWpc; ++q) t += red[threadIdx.x * kLzWpc + q];
-                out[jb + threadIdx.x] = scale * t;
-            }
-            if (jb + kLzCols < j1) __syncthreads();   // red is reused by the next pass
-        }
-    };
-    // block total of v (one value per thread) into *slot
-    auto block_part = [&](double v, double *slot) {
+    // the block's sum of v, in an order that does not depend on the block
+    auto block_sum = [&](double v) {
         v = warp_sum(v);
         if (lane == 0) red[warp] = v;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            double tot = 0.0;
-            for (int q = 0; q < nwarp; ++q) tot += red[q];
-            *slot = tot;
-        }
-    };
-    // sum of p[0 .. G) in a fixed order, the same in every block
-    auto grid_total = [&](const double *p, int which) {
-        if (warp == 0) {
-            double v = 0.0;
-            for (int q = lane; q < G; q += 32) v += __ldcg(p + q);
-            v = warp_sum(v);
-            if (lane == 0) scal[which] = v;
-        }
+        v = warp_sum(red[lane]);
         __syncthreads();
-        return scal[which];
+        return v;
     };
-    double nrmPrev = 0.0;
-    for (int k = k0; k < k1; ++k) {
-        const double *vk = V + (size_t) k * ldv;
-        if (k > k0) stage(w, nrmPrev);
-        else stage(vk, 1.0);
-        coldot(1, sK, tg, 1.0);     // t = K^T v_k
-        grid.sync();
-        stage(tg, 1.0);
-        coldot(0, sD, ug, -1.0);    // u = -D t
-        grid.sync();
-        stage(ug, 1.0);
-        coldot(2, sKT, w, 1.0);     // w = K u
-        __syncthreads();
-        // w -= beta_{k-1} v_{k-1}; partial w.v_k
-        const double bprev = (k > 0) ? __ldcg(ab + maxdim + k - 1) : 0.0;
-        double pa = 0.0;
-        for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-            double x = w[j];
-            if (k > 0) x -= bprev * __ldcg(V + (size_t) (k - 1) * ldv + j);
-            w[j] = x;
-            pa += x * __ldcg(vk + j);
+    const bool own = warp == 0 && lane < nc;   // thread of column j0 + lane
+    const int i0 = tid, i1 = tid + kLzThreads;
+    double2 vk, vp = make_double2(0.0, 0.0);   // this thread's entries of v_k and v_{k-1}
+    double beta = 0.0;
+    if (k0 == 0) {
+        vk.x = i0 < n ? (a ? __ldg(a + i0) : 0.0) + __ldg(b + i0) : 0.0;
+        vk.y = i1 < n ? (a ? __ldg(a + i1) : 0.0) + __ldg(b + i1) : 0.0;
+        const double nrm = sqrt(block_sum(vk.x * vk.x + vk.y * vk.y));
+        vk = (nrm > 0.0) ? make_double2(vk.x / nrm, vk.y / nrm) : make_double2(0.0, 0.0);
+        put(vk);
+        if (own) V[j0 + lane] = sx[j0 + lane];
+    } else {
+        const double *v = V + (size_t) k0 * ldv, *u = V + (size_t) (k0 - 1) * ldv;
+        vk = make_double2(i0 < n ? __ldcg(v + i0) : 0.0, i1 < n ? __ldcg(v + i1) : 0.0);
+        vp = make_double2(i0 < n ? __ldcg(u + i0) : 0.0, i1 < n ? __ldcg(u + i1) : 0.0);
+        beta = __ldcg(ab + maxdim + k0 - 1);
+        put(vk);
+    }
+    for (int k = k0; k < k1; ++k, ++tag) {
+        double x = product(1);                  // t = K^T v_k
+        if (own) lz_put(wt + j0 + lane, x, tag);
+        put(fetch(wt, tag));
+        if (lost) return;
+        x = product(0);                         // u = -D t
+        if (own) lz_put(wu + j0 + lane, -x, tag);
+        put(fetch(wu, tag));
+        if (lost) return;
+        x = product(2);                         // w = K u
+        if (own) lz_put(ww + j0 + lane, x, tag);
+        double2 w = fetch(ww, tag);
+        if (k > 0) {
+            w.x -= beta * vp.x;
+            w.y -= beta * vp.y;
         }
-        block_part(pa, part + blockIdx.x);
-        grid.sync();
-        const double alp = grid_total(part, 0);
-        double pn = 0.0;
-        for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-            const double x = w[j] - alp * __ldcg(vk + j);
-            w[j] = x;
-            pn += x * x;
+        __syncthreads();                        // the first warp has read red
+        const double alp = block_sum(w.x * vk.x + w.y * vk.y);
+        w.x -= alp * vk.x;
+        w.y -= alp * vk.y;
+        const double nrm = sqrt(block_sum(w.x * w.x + w.y * w.y));
+        beta = (nrm > 0.0) ? nrm : 0.0;
+        vp = vk;
+        vk = (nrm > 0.0) ? make_double2(w.x / nrm, w.y / nrm) : make_double2(0.0, 0.0);
+        put(vk);
+        if (lost) return;
+        if (own) V[(size_t) (k + 1) * ldv + j0 + lane] = sx[j0 + lane];
+        if (blockIdx.x == 0 && tid == 0) {
+            ab[k] = alp;
+            ab[maxdim + k] = beta;
+            if (hab) {
+                hab[k] = alp;
+                hab[maxdim + k] = beta;
+            }
         }
-        block_part(pn, part + G + blockIdx.x);
-        grid.sync();
-        const double nrm = sqrt(grid_total(part + G, 1));
-        lz_next(j0, j1, k, alp, nrm, V, ldv, ab, maxdim, w);
-        nrmPrev = nrm;
     }
 }
 
@@ -2523,7 +2528,6 @@ void Lanczos::init(int n_, cudaStream_t s_) {
     for (double **p : {&w, &z1, &z2, &t1, &u, &warm, &init_vec, &pert_vec}) HB_CUDA(hb::cmalloc(p, sizeof(double) * ld));
     HB_CUDA(hb::cmalloc(&d_ab, sizeof(double) * (2 * maxdim + 2)));
     HB_CUDA(hb::cmalloc_host(&h_ab, sizeof(double) * (2 * maxdim + 2)));
-    HB_CUDA(hb::cmalloc(&part, sizeof(double) * 2 * kLanczosMaxBlocks));
     HB_CUDA(hb::cmalloc(&d_y, sizeof(double) * 2 * (maxdim + 1)));
     HB_CUDA(hb::cmalloc(&d_scal, sizeof(double) * 4));
     HB_CUDA(hb::cmalloc_host(&h_scal, sizeof(double) * 4));
@@ -2564,7 +2568,7 @@ void Lanczos::init(int n_, cudaStream_t s_) {
 }
 
 void Lanczos::release() {
-    for (double **p : {&V, &w, &z1, &z2, &t1, &u, &warm, &init_vec, &pert_vec, &d_ab, &d_y, &d_scal, &part}) {
+    for (double **p : {&V, &w, &z1, &z2, &t1, &u, &warm, &init_vec, &pert_vec, &d_ab, &d_y, &d_scal, &d_list, &d_words}) {
         if (*p) hb::cache_free(*p);
         *p = nullptr;
     }
@@ -2583,13 +2587,35 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
         compute_inverse_factor(s, F);
     }
     if (tm) tm->lz_inverse += wall() - t0;   // enqueue time: the steps' launch follows without a wait
+    LzList S;
+    if (!hyOp && n > kLzClusterMaxN) {
+        if (!d_list) {
+            const size_t ent = (size_t) n * kLzListMax;
+            if (hb::cmalloc(&d_list, ent * (sizeof(double) + sizeof(int)) + sizeof(int) * ((size_t) n + 1)) != cudaSuccess) {
+                cudaGetLastError();
+                d_list = nullptr;
+            } else {
+                HB_CUDA(cudaMemsetAsync(d_list + ent, 0, sizeof(int), s));
+                listEpoch = 0;
+            }
+        }
+        if (d_list) {
+            S.val = d_list;
+            S.flag = reinterpret_cast<unsigned *>(d_list + (size_t) n * kLzListMax);
+            S.cnt = reinterpret_cast<int *>(S.flag) + 1;
+            S.idx = S.cnt + n;
+            S.epoch = ++listEpoch;
+            lz_list_kernel<<<hb::counted((n + 7) / 8), 256, 0, s>>>(n, D, ldD, S);
+        }
+    }
     // buffers: V columns, w (Mv), t1 / z1 / z2 temporaries
     auto mv = [&](const double *x, double *y) {
         if (hyOp) {
             hyOp->apply_congruence(s, D, ldD, -1.0, x, t1, u, y);  // y = L^-1 (-D) L^-T x
         } else {
             coldot(s, n, n, F.K, F.ld, x, t1, 1.0, 0.0, 1);   // t1 = L^-T x
-            coldot(s, n, n, D, ldD, t1, u, -1.0, 0.0, 0);     // u  = -D t1
+            if (S.cnt) lz_list_mv_kernel<<<hb::counted((n + 7) / 8), 256, 0, s>>>(n, D, ldD, S, t1, u);
+            else coldot(s, n, n, D, ldD, t1, u, -1.0, 0.0, 0);   // u  = -D t1
             coldot(s, n, n, F.KT, F.ld, u, y, 1.0, 0.0, 2);   // y  = L^-1 u
         }
         if (tm) tm->n_lanczos_mv += 1;
@@ -2598,6 +2624,37 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
     // the recorded alpha / beta (a step's values do not depend on later steps)
     const bool small = !hyOp && n <= kSmallLanczosN;
     const bool cluster = !hyOp && !small && n <= kLzClusterMaxN && lz_cluster_available();
+    // above kLzFusedMaxN K and K^T stream from DRAM, where a launch per product keeps more loads
+    // in flight than the cooperative grid
+    bool fused = !small && !cluster && !hyOp && n <= std::min(kLzFusedMaxN, 32 * device_sm_count());
+    if (fused && !d_words) {
+        if (hb::cmalloc(&d_words, sizeof(LzWord) * 3 * n) != cudaSuccess) {
+            cudaGetLastError();
+            d_words = nullptr;
+            fused = false;
+        } else {
+            HB_CUDA(cudaMemsetAsync(d_words, 0, sizeof(LzWord) * 3 * n, s));
+            wordTag = 0;
+        }
+    }
+    int lzGrid = 0, lzSmem = 0;
+    if (fused) {
+        static std::atomic<unsigned long long> attr{0};
+        static std::atomic<int> smemMax[kMaxDevices];
+        once_per_device(attr, [] {
+            int optin = 0;
+            cudaFuncAttributes fa;
+            HB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, current_device()));
+            HB_CUDA(cudaFuncGetAttributes(&fa, lz_grid_steps_kernel));
+            smemMax[current_device()].store(optin - (int) fa.sharedSizeBytes);
+            HB_CUDA(cudaFuncSetAttribute((const void *) lz_grid_steps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         optin - (int) fa.sharedSizeBytes));
+        });
+        const int cpb = (n + device_sm_count() - 1) / device_sm_count();   // at most one block per SM
+        lzGrid = (n + cpb - 1) / cpb;
+        const long want = n + lz_cached_doubles(n, cpb);
+        lzSmem = (int) std::min<long>(smemMax[current_device()].load(), want * (long) sizeof(double));
+    }
     if (small) {
         static std::atomic<unsigned long long> attr{0};
         once_per_device(attr, [] {
@@ -2614,53 +2671,11 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
         HB_CUDA(cudaMemcpyAsync(h_ab, d_ab, sizeof(double) * (2 * maxdim + 2), cudaMemcpyDeviceToHost, s));
         HB_CUDA(cudaStreamSynchronize(s));
         if (tm) tm->n_lanczos_mv += maxdim;
-    } else if (!cluster) {
+    } else if (!cluster && !fused) {
         HB_CUDA(cudaMemsetAsync(V, 0, sizeof(double) * ld * (maxdim + 1), s));
         HB_CUDA(cudaMemsetAsync(d_ab, 0, sizeof(double) * (2 * maxdim + 2), s));
         if (nComputed == 0) lanczos_start_kernel<<<hb::counted(1), 1024, 0, s>>>(n, nullptr, init_vec, V);
         else lanczos_start_kernel<<<hb::counted(1), 1024, 0, s>>>(n, warm, pert_vec, V);
-    }
-    // dense factor: the steps up to each check run in one cooperative launch; with the
-    // columns of K, K^T and D held in shared memory when one block's share fits. Above
-    // kLzFusedMaxN the three matrices stream from DRAM, where the per-step launches keep
-    // more loads in flight than the cooperative grid.
-    const bool fused = !small && !cluster && !hyOp && n <= kLzFusedMaxN;
-    int lzGrid = 0;
-    bool lzCached = false;
-    size_t lzSmem = 0;
-    if (fused) {
-        static std::atomic<int> capacity[kMaxDevices][2];
-        static std::atomic<unsigned long long> attr{0};
-        once_per_device(attr, [] {
-            HB_CUDA(cudaFuncSetAttribute((const void *) lanczos_steps_smem_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kLzSmemMax));
-        });
-        const int sms = device_sm_count();
-        const int cpbCached = (n + sms - 1) / sms;
-        const size_t need = sizeof(double) * (size_t) (lz_cached_doubles(n, cpbCached) + n);
-        lzCached = need <= (size_t) kLzSmemMax;
-        const int slot = lzCached ? 1 : 0;
-        int cap = capacity[current_device()][slot].load(std::memory_order_relaxed);
-        if (!cap) {
-            int per = 0;
-            if (lzCached)
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, lanczos_steps_smem_kernel, kLzThreads, kLzSmemMax);
-            else
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, lanczos_steps_kernel, kLzThreads, 0);
-            cap = std::max(1, per) * sms;
-            capacity[current_device()][slot].store(cap, std::memory_order_relaxed);
-        }
-        if (lzCached) {
-            // one block per SM, so that every block's columns fit its shared memory
-            lzGrid = std::min(std::min(cap, sms), kLanczosMaxBlocks);
-            const int cpb = (n + lzGrid - 1) / lzGrid;
-            lzSmem = sizeof(double) * (size_t) (lz_cached_doubles(n, cpb) + n);
-            if (lzSmem > (size_t) kLzSmemMax) lzCached = false;
-        }
-        if (!lzCached) {
-            lzSmem = 0;
-            lzGrid = std::max(1, std::min(std::min(cap, kLanczosMaxBlocks), (n + kLzCols - 1) / kLzCols));
-        }
     }
     int stepsDone = 0;
 
@@ -2683,27 +2698,35 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
                 const double *Kp = F.K, *KTp = F.KT, *Dp = D;
                 long ldk = F.ld, ldd = ldD, ldv = ld;
                 int nn = n, md = maxdim, ka = k, kb = k1;
-                double *Vp = V, *abp = d_ab, *tp = t1, *up = u, *wp = w, *pp = part;
+                double *Vp = V, *abp = d_ab;
                 if (cluster) {
                     HB_CUDA(lz_cluster_launch(lz_cluster_steps_kernel, lz_cl_smem(n), s, n, F.K, F.KT, F.ld, D, ldD,
                                               nComputed == 0 ? nullptr : warm, nComputed == 0 ? init_vec : pert_vec, V,
                                               ld, d_ab, dm_ab, maxdim, k, k1));
-                } else if (lzCached) {
-                    void *args[] = {&nn, &Kp, &KTp, &ldk, &Dp, &ldd, &Vp, &ldv, &abp, &md, &ka, &kb, &wp, &tp, &up, &pp};
-                    HB_CUDA(cudaLaunchCooperativeKernel((const void *) lanczos_steps_smem_kernel, hb::counted(lzGrid),
-                                                        kLzThreads, args, lzSmem, s));
                 } else {
-                    void *args[] = {&nn, &Kp, &KTp, &ldk, &Dp, &ldd, &Vp, &ldv, &abp, &md, &ka, &kb, &tp, &up, &wp, &pp};
-                    HB_CUDA(cudaLaunchCooperativeKernel((const void *) lanczos_steps_kernel, hb::counted(lzGrid),
-                                                        kLzThreads, args, 0, s));
+                    const double *sa = nComputed == 0 ? nullptr : warm, *sb = nComputed == 0 ? init_vec : pert_vec;
+                    double *hab = dm_ab;
+                    long cache = lzSmem / (long) sizeof(double) - n;
+                    LzWord *words = reinterpret_cast<LzWord *>(d_words);
+                    unsigned long long tag = wordTag + 1;
+                    wordTag += k1 - k;
+                    void *args[] = {&nn, &Kp, &KTp, &ldk, &Dp, &ldd, &S, &sa, &sb, &Vp, &ldv, &abp, &hab, &md, &ka, &kb,
+                                    &words, &tag, &cache};
+                    HB_CUDA(cudaLaunchCooperativeKernel((const void *) lz_grid_steps_kernel, hb::counted(lzGrid),
+                                                        kLzThreads, args, lzSmem, s));
                 }
                 if (tm) tm->n_lanczos_mv += k1 - k;
                 stepsDone = k1;
-                if (!cluster || !dm_ab)
+                if (!dm_ab)
                     HB_CUDA(cudaMemcpyAsync(h_ab, d_ab, sizeof(double) * (2 * maxdim + 2), cudaMemcpyDeviceToHost, s));
                 const double tw = wall();
                 HB_CUDA(cudaStreamSynchronize(s));
                 if (tm) tm->lz_wait += wall() - tw;
+                if (fused && h_ab[2 * maxdim + 1] != 0.0) {   // a block of the launch gave up waiting
+                    device_error_flag() = 1;
+                    ret = HDSDP_RETCODE_FAILED;
+                    break;
+                }
             }
         } else if (!small) {
             mv(V + (size_t) k * ld, w);

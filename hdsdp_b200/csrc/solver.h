@@ -45,7 +45,6 @@ struct Timers {
 };
 
 // Lanczos maximum-step estimator (linalg/hdsdp_lanczos.c:161-292) on the GPU.
-constexpr int kLanczosMaxBlocks = 1024;   // grid bound of the fused Lanczos steps
 struct Lanczos {
     int n = 0, maxdim = 30;
     long ld = 0;
@@ -56,13 +55,16 @@ struct Lanczos {
     double *d_y = nullptr;    // 2 * (maxdim + 1)
     double *d_scal = nullptr, *h_scal = nullptr;
     double *init_vec = nullptr, *pert_vec = nullptr;  // device, deterministic per n
-    double *part = nullptr;   // per-block partial sums of the fused steps (2 x kLanczosMaxBlocks)
     // pinned Ritz coefficients, and the device addresses of the pinned h_ab, h_scal and h_yv
     // (null where the memory is not mapped), for the batched small-block runs
     double *h_yv = nullptr;
     double *dm_ab = nullptr, *dm_scal = nullptr, *dm_yv = nullptr;
     int nComputed = 0;
     int lastSteps = 12;       // steps the last bound took: as many go into the next one's first launch
+    double *d_list = nullptr; // the step matrix's entries by column (orders above the cluster kernel's)
+    unsigned listEpoch = 0;
+    double *d_words = nullptr;               // tagged words of the cooperative steps, and the last tag used
+    unsigned long long wordTag = 0;
     // when set, the operator is built from this sparse factor of S instead of F
     HybridFactor *hyOp = nullptr;
     void init(int n_, cudaStream_t s_);
