@@ -1000,7 +1000,11 @@ void KKT::init(int m_, cudaStream_t stream, Timers *t, bool denseM) {
     asinvcs.assign(m, 0.0);
     diag_add.assign(m, 0.0);
     for (double **p : {&d_rhs, &d_x, &d_r, &d_t, &d_diag}) HB_CUDA(hb::cmalloc(p, sizeof(double) * m));
-    HB_CUDA(hb::cmalloc_host(&h_buf, sizeof(double) * m));
+    HB_CUDA(hb::cmalloc_host(&h_buf, sizeof(double) * ((size_t) m + 1)));   // and a status word
+    if (!h_buf || cudaHostGetDevicePointer((void **) &dm_buf, h_buf, 0) != cudaSuccess) {
+        cudaGetLastError();
+        dm_buf = nullptr;
+    }
 }
 
 void KKT::release() {
@@ -1023,7 +1027,9 @@ void KKT::release() {
         *p = nullptr;
     }
     if (h_buf) hb::cache_free_host(h_buf);
-    h_buf = nullptr;
+    h_buf = dm_buf = nullptr;
+    if (d_words) hb::cache_free(d_words);
+    d_words = nullptr;
 }
 
 void KKT::clean(int type) {
@@ -1445,7 +1451,11 @@ hdsdp_retcode KKT::factorize() {
     return ok && !device_error_flag() ? HDSDP_RETCODE_OK : HDSDP_RETCODE_FAILED;
 }
 
-// x = M^-1 b with one step of iterative refinement on the FP64 residual.
+// x = M^-1 b with one step of iterative refinement on the FP64 residual: t = K b, x = K^T t,
+// r = b - M x (of the unshifted system), x += K^T (K r), in one launch that reads b from and
+// writes x to the pinned buffer (further down, with the kernels).
+static bool kkt_fused_solve(KKT &k);
+
 hdsdp_retcode KKT::solve(const double *rhs, double *lhs) {
     double t0 = wall();
     if (arrow) {
@@ -1457,6 +1467,16 @@ hdsdp_retcode KKT::solve(const double *rhs, double *lhs) {
         return device_error_flag() ? HDSDP_RETCODE_FAILED : HDSDP_RETCODE_OK;
     }
     std::memcpy(h_buf, rhs, sizeof(double) * m);
+    if (!ldlActive && F.fuse_k && kkt_fused_solve(*this)) {
+        HB_CUDA(cudaStreamSynchronize(s));
+        if (h_buf[m] != 0.0) device_error_flag() = 1;   // a block of the launch gave up waiting
+        std::memcpy(lhs, h_buf, sizeof(double) * m);
+        if (tm) {
+            tm->schur_solve += wall() - t0;
+            tm->n_schur_solve += 1;
+        }
+        return device_error_flag() ? HDSDP_RETCODE_FAILED : HDSDP_RETCODE_OK;
+    }
     HB_CUDA(cudaMemcpyAsync(d_rhs, h_buf, sizeof(double) * m, cudaMemcpyHostToDevice, s));
     if (ldlActive) {
         ldl_solve(s, ldl, d_rhs, d_x);
@@ -2130,6 +2150,138 @@ cudaError_t lz_cluster_launch(void (*fn)(P...), size_t smem, cudaStream_t s, A..
     return cudaLaunchKernelEx(&cfg, fn, (P) args...);
 }
 
+// ---- The Schur solve with refinement in one launch (see KKT::solve). Ten operations before (two
+// copies, five products, a copy, an axpy and the copy back), each a launch and a gap.
+//
+// Up to the cluster's order: K, K^T and M in the cluster's shared memory, as for Lanczos.
+// The right-hand side comes with the launch's parameters (a read of host memory takes 3 us), the
+// solution goes to host memory in one piece per CTA (requests of a few bytes cost 0.15 us each).
+struct KktRhs {
+    double v[kLzClusterMaxN];
+};
+__global__ void __launch_bounds__(kLzClThreads, 1)
+    kkt_cluster_solve_kernel(int n, const double *K, const double *KT, long ldk, const double *M, long ldM, double shift,
+                             const __grid_constant__ KktRhs rhs, double *x, double *out) {
+    LzCluster C;
+    C.init(n, K, KT, ldk, M, ldM);
+    double *sb = C.vec, *st = sb + n, *sx = st + n, *sr = sx + n;
+    for (int i = threadIdx.x; i < n; i += kLzClThreads) sb[i] = rhs.v[i];
+    lz_cl_sync();   // every CTA is there, its columns in place
+    auto each = [&](auto f) {
+        for (int c = C.warp; c < C.nc; c += kLzClWarps) f(c, C.j0 + c);
+    };
+    auto lower = [&](int c, int j, const double *v) { return C.dot(C.colKT(c), v, 0, j + 1); };   // K v
+    auto upper = [&](int c, int j, const double *v) { return C.dot(C.colK(c), v, j, n); };        // K^T v
+    each([&](int c, int j) { C.share(lower(c, j, sb), st + j); });
+    lz_cl_sync();
+    each([&](int c, int j) { C.share(upper(c, j, st), sx + j); });
+    lz_cl_sync();
+    each([&](int c, int j) {
+        double v = sb[j] - C.dot(C.sD + (long) c * n, sx, 0, n);
+        if (shift != 0.0) v += shift * sx[j];
+        C.share(v, sr + j);
+    });
+    lz_cl_sync();
+    each([&](int c, int j) { C.share(lower(c, j, sr), st + j); });
+    lz_cl_sync();
+    each([&](int c, int j) {
+        const double v = sx[j] + upper(c, j, st);
+        if (C.lane == 0) sb[j] = v;
+    });
+    __syncthreads();
+    if (C.warp == 0 && C.lane < C.nc) {
+        x[C.j0 + C.lane] = sb[C.j0 + C.lane];
+        out[C.j0 + C.lane] = sb[C.j0 + C.lane];
+    }
+}
+
+// Above it: the grid, every block with the columns of its entries, read from L2, and the vectors
+// exchanged in tagged words as in lz_grid_steps_kernel (each used once a launch).
+constexpr int kKktMaxN = 4 * kLzThreads;
+__global__ void __launch_bounds__(kLzThreads, 1)
+    kkt_grid_solve_kernel(int n, const double *K, const double *KT, long ldk, const double *M, long ldM, double shift,
+                          const double *rhs, double *x, double *err, LzWord *words, unsigned long long tag) {
+    __shared__ double red[kLzWarps];
+    __shared__ int lost;
+    extern __shared__ double sx[];
+    const int G = gridDim.x, cpb = (n + G - 1) / G;
+    const int j0 = min(n, (int) blockIdx.x * cpb), nc = min(n, j0 + cpb) - j0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wpc = min(kLzMaxSegs, kLzWarps / cpb), slot = warp / wpc, seg = warp % wpc;
+    const bool own = warp == 0 && lane < nc;   // thread of entry j0 + lane
+    if (tid == 0) lost = 0;
+    // column j0 + c's product with sx over rows lo(j) <= i < hi(j), to thread c of the first warp
+    auto product = [&](const double *A, long ld, int mode) {
+        double p[4] = {}, y[8];
+        if (slot < nc) {
+            const int j = j0 + slot, lo = (mode == 1) ? j : 0, hi = (mode == 2) ? j + 1 : n;
+            const double *col = A + (size_t) j * ld;
+            const int chunk = (((hi - lo + wpc - 1) / wpc) + 31) & ~31;
+            const int e = min(hi, lo + (seg + 1) * chunk);
+            for (int i = lo + seg * chunk + lane; i < e; i += 256) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) y[q] = (i + 32 * q < e) ? __ldg(col + i + 32 * q) : 0.0;
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (i + 32 * q < e) p[q & 3] += y[q] * sx[i + 32 * q];
+            }
+        }
+        const double acc = warp_sum((p[0] + p[2]) + (p[1] + p[3]));
+        if (lane == 0) red[warp] = acc;
+        __syncthreads();
+        double mine = 0.0;
+        if (own) {
+#pragma unroll
+            for (int q = 0; q < kLzMaxSegs; ++q)
+                if (q < wpc) mine += red[lane * wpc + q];
+        }
+        return mine;
+    };
+    // publishes this block's entries and brings the whole vector into sx; false when given up
+    auto exchange = [&](int which, double v) {
+        LzWord *p = words + (size_t) which * n;
+        if (own) lz_put(p + j0 + lane, v, tag);
+        double y[4];
+        unsigned open = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (tid + q * kLzThreads < n) open |= 1u << q;
+        for (int it = 0; open && it < kLzPollLimit; ++it) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if ((open >> q & 1) && lz_get(p + tid + q * kLzThreads, y[q], tag)) open &= ~(1u << q);
+        }
+        if (open) {
+            lost = 1;
+            *err = 1.0;
+            return;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (tid + q * kLzThreads < n) sx[tid + q * kLzThreads] = y[q];
+    };
+    const double b = own ? rhs[j0 + lane] : 0.0;
+    for (int i = tid; i < n; i += kLzThreads) sx[i] = __ldg(rhs + i);
+    __syncthreads();
+    exchange(0, product(KT, ldk, 2));           // t = K b
+    __syncthreads();
+    if (lost) return;
+    const double x0 = product(K, ldk, 1);       // x = K^T t
+    exchange(1, x0);
+    __syncthreads();
+    if (lost) return;
+    double r = b - product(M, ldM, 0);
+    if (shift != 0.0) r += shift * x0;
+    exchange(2, r);
+    __syncthreads();
+    if (lost) return;
+    exchange(3, product(KT, ldk, 2));
+    __syncthreads();
+    if (lost) return;
+    const double v = x0 + product(K, ldk, 1);
+    if (own) x[j0 + lane] = v;
+}
+
 // whether the device takes a cluster of 16 with the largest order's shared memory (per device)
 bool lz_cluster_available() {
     static std::atomic<int> state[kMaxDevices];   // 0 unknown, 1 yes, 2 no
@@ -2138,7 +2290,8 @@ bool lz_cluster_available() {
     if (v) return v == 1;
     const int smem = (int) lz_cl_smem(kLzClusterMaxN);
     bool ok = true;
-    for (const void *fn : {(const void *) lz_cluster_steps_kernel, (const void *) lz_cluster_ritz_kernel}) {
+    for (const void *fn : {(const void *) lz_cluster_steps_kernel, (const void *) lz_cluster_ritz_kernel,
+                           (const void *) kkt_cluster_solve_kernel}) {
         ok = ok && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
              cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
         cudaLaunchConfig_t cfg = {};
@@ -2519,6 +2672,45 @@ void tridiag_eig(int n, std::vector<double> d, std::vector<double> e, std::vecto
     evals = d;
 }
 }  // namespace
+
+static bool kkt_fused_solve(KKT &k) {
+    const int m = k.m;
+    if (!k.dm_buf || !k.F.K || !k.F.KT || !k.F.k_valid || m < 1) return false;
+    k.h_buf[m] = 0.0;
+    if (m <= kLzClusterMaxN && lz_cluster_available()) {
+        KktRhs rhs;
+        std::memcpy(rhs.v, k.h_buf, sizeof(double) * m);
+        return lz_cluster_launch(kkt_cluster_solve_kernel, lz_cl_smem(m), k.s, m, k.F.K, k.F.KT, k.F.ld, k.M, k.ldm,
+                                 k.shift, rhs, k.d_x, k.dm_buf) == cudaSuccess;
+    }
+    const int sms = device_sm_count();
+    if (m > std::min(kKktMaxN, 32 * sms)) return false;
+    if (!k.d_words) {
+        if (hb::cmalloc(&k.d_words, sizeof(LzWord) * 4 * m) != cudaSuccess) {
+            cudaGetLastError();
+            k.d_words = nullptr;
+            return false;
+        }
+        HB_CUDA(cudaMemsetAsync(k.d_words, 0, sizeof(LzWord) * 4 * m, k.s));
+        k.wordTag = 0;
+    }
+    const int cpb = (m + sms - 1) / sms;
+    int n = m;
+    const double *K = k.F.K, *KT = k.F.KT, *M = k.M, *rhs = k.d_rhs;
+    long ldk = k.F.ld, ldM = k.ldm;
+    double shift = k.shift, *x = k.d_x, *err = k.dm_buf + m;
+    LzWord *words = reinterpret_cast<LzWord *>(k.d_words);
+    unsigned long long tag = ++k.wordTag;
+    HB_CUDA(cudaMemcpyAsync(k.d_rhs, k.h_buf, sizeof(double) * m, cudaMemcpyHostToDevice, k.s));
+    void *args[] = {&n, &K, &KT, &ldk, &M, &ldM, &shift, &rhs, &x, &err, &words, &tag};
+    if (cudaLaunchCooperativeKernel((const void *) kkt_grid_solve_kernel, hb::counted((m + cpb - 1) / cpb), kLzThreads,
+                                    args, sizeof(double) * m, k.s) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    HB_CUDA(cudaMemcpyAsync(k.h_buf, k.d_x, sizeof(double) * m, cudaMemcpyDeviceToHost, k.s));
+    return true;
+}
 
 void Lanczos::init(int n_, cudaStream_t s_) {
     n = n_;

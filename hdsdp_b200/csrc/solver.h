@@ -297,7 +297,9 @@ struct KKT {
     std::vector<double> asinv, asinvrd, asinvcs;
     double dCSinv = 0, dCSinvCSinv = 0, dCSinvRdSinv = 0, dTraceSinv = 0;
     double *d_rhs = nullptr, *d_x = nullptr, *d_r = nullptr, *d_t = nullptr, *d_diag = nullptr;
-    double *h_buf = nullptr;
+    double *h_buf = nullptr, *dm_buf = nullptr;   // pinned, and its device address (null where not mapped)
+    double *d_words = nullptr;                    // tagged words of the fused solve, and the last tag used
+    unsigned long long wordTag = 0;
     std::vector<double> diag_add;     // bound-cone diagonal accumulated before factorisation
     double shift = 0.0;               // diagonal shift applied if the Cholesky of M failed
     // LDL^T (Bunch-Kaufman) factor of M: taken when the Cholesky fails even with the shift
