@@ -470,9 +470,14 @@ void SdpCone::update_buffer(double dC, double dAs, const double *y, double dEye,
     double *target = nullptr;
     const double *ly = nullptr;
     if (buffer_plan(dC, dAs, y, dEye, which, &target, &ly)) {
-        std::memcpy(h_vec, ly, sizeof(double) * m);
-        HB_CUDA(cudaMemcpyAsync(d_y, h_vec, sizeof(double) * m, cudaMemcpyHostToDevice, s));
-        dev.assemble(dC, dAs, d_y, dEye, target, ld);
+        const double *hy = nullptr;
+        if (m <= kAsmParamMax) {
+            hy = ly;   // with the first launch's parameters, which puts it into d_y
+        } else {
+            std::memcpy(h_vec, ly, sizeof(double) * m);
+            HB_CUDA(cudaMemcpyAsync(d_y, h_vec, sizeof(double) * m, cudaMemcpyHostToDevice, s));
+        }
+        dev.assemble(dC, dAs, d_y, dEye, target, ld, hy);
     }
     if (tm) tm->assemble += wall() - t0;
 }
@@ -1001,6 +1006,8 @@ void KKT::init(int m_, cudaStream_t stream, Timers *t, bool denseM) {
     diag_add.assign(m, 0.0);
     for (double **p : {&d_rhs, &d_x, &d_r, &d_t, &d_diag}) HB_CUDA(hb::cmalloc(p, sizeof(double) * m));
     HB_CUDA(hb::cmalloc_host(&h_buf, sizeof(double) * ((size_t) m + 1)));   // and a status word
+    HB_CUDA(hb::cmalloc_host(&h_diag, sizeof(double) * m));
+    diagPending = false;
     if (!h_buf || cudaHostGetDevicePointer((void **) &dm_buf, h_buf, 0) != cudaSuccess) {
         cudaGetLastError();
         dm_buf = nullptr;
@@ -1028,8 +1035,14 @@ void KKT::release() {
     }
     if (h_buf) hb::cache_free_host(h_buf);
     h_buf = dm_buf = nullptr;
+    if (h_diag) hb::cache_free_host(h_diag);
+    h_diag = nullptr;
     if (d_words) hb::cache_free(d_words);
     d_words = nullptr;
+    for (cudaEvent_t &e : phase) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
 }
 
 void KKT::clean(int type) {
@@ -1090,12 +1103,43 @@ hdsdp_retcode KKT::add_sdp(SdpCone &cone, int type) {
     const long ld = cone.ld;
     const double r = cone.dualResidual;
     const double *Wp = nullptr;
+    // The device work is enqueued without a wait in between, the vectors and the trace into the
+    // cone's pinned buffers; finish() waits once, forms the host sums in their order and reads the
+    // phases' times from events on the stream.
+    auto mark = [&](int i) {
+        if (!tm) return;
+        if (!phase[i] && cudaEventCreate(&phase[i]) != cudaSuccess) phase[i] = nullptr;
+        if (phase[i]) HB_CUDA(cudaEventRecord(phase[i], s));
+    };
+    bool vec2 = false, traced = false;
+    auto to_host = [&](double *h, const double *d) {
+        if (cone.m > 0) HB_CUDA(cudaMemcpyAsync(h, d, sizeof(double) * cone.m, cudaMemcpyDeviceToHost, s));
+    };
+    auto finish = [&](int marks) {
+        HB_CUDA(cudaStreamSynchronize(s));
+        auto acc = [&](std::vector<double> &dst, const double *h, double scale) {
+            if (rows)
+                for (int i = 0; i < cone.m; ++i) dst[(*rows)[i]] += scale * h[i];
+            else
+                for (int i = 0; i < cone.m; ++i) dst[i] += scale * h[i];
+        };
+        if (traced) dTraceSinv += cone.h_scal[0];
+        acc(asinv, cone.h_vec, 1.0);
+        if (vec2) acc(asinvrd, cone.h_vec2, r);
+        double *const into[4] = {tm ? &tm->s_inverse : nullptr, tm ? &tm->sch_matrix : nullptr,
+                                 tm ? &tm->sch_inner : nullptr, tm ? &tm->sch_innersq : nullptr};
+        for (int i = 0; tm && i + 1 < marks; ++i) {
+            float ms = 0.f;
+            if (phase[i] && phase[i + 1] && cudaEventElapsedTime(&ms, phase[i], phase[i + 1]) == cudaSuccess)
+                *into[i] += 1e-3 * ms;
+        }
+    };
+    mark(0);
     if (type == KKT_TYPE_PRIMAL) {
         if (!primalX) return HDSDP_RETCODE_FAILED;
         Wp = primalX;
     } else {
         if (cone.hy && !cone.ensure_dense(BUFFER_DUALVAR)) return HDSDP_RETCODE_FAILED;
-        double ti = wall();
         // split precision: W = K^T K on the tensor cores once n makes the product worth it
         bool done = false;
         if (cone.dev.precision == 1 && n >= kSplitInverseMinN) {
@@ -1103,31 +1147,28 @@ hdsdp_retcode KKT::add_sdp(SdpCone &cone, int type) {
             done = cone.dev.split_inverse(cone.Fvar.K, cone.W, ld);
         }
         if (!done) compute_inverse(s, cone.Fvar, cone.W, ld);
-        if (tm) {
-            HB_CUDA(cudaStreamSynchronize(s));
-            tm->s_inverse += wall() - ti;
-        }
         Wp = cone.W;
         cone.pinVar = true;   // the accepted point's factor
     }
+    mark(1);
     SdpDevice &dev = cone.dev;
     if (type == KKT_TYPE_CORRECTOR) {
         dev.inner_all(Wp, ld, cone.d_vec);
-        add_host(asinv, cone.d_vec, h_buf, cone.m, 1.0, s, rows);
+        to_host(cone.h_vec, cone.d_vec);
         if (r != 0.0) {
-            dev.inner_all_sq(Wp, ld, cone.d_vec, false, true);
-            add_host(asinvrd, cone.d_vec, h_buf, cone.m, r, s, rows);
+            dev.inner_all_sq(Wp, ld, cone.d_vec2, false, true);
+            to_host(cone.h_vec2, cone.d_vec2);
+            vec2 = true;
         }
+        finish(2);
         if (tm) tm->schur += wall() - t0;
         return device_error_flag() ? HDSDP_RETCODE_FAILED : HDSDP_RETCODE_OK;
     }
     if (r != 0.0) {
         trace(s, n, Wp, ld, cone.d_scal);
         HB_CUDA(cudaMemcpyAsync(cone.h_scal, cone.d_scal, sizeof(double), cudaMemcpyDeviceToHost, s));
-        HB_CUDA(cudaStreamSynchronize(s));
-        dTraceSinv += cone.h_scal[0];
+        traced = true;
     }
-    double tq = wall();
     if (!rows && !mOpen) {
         // the first contribution, from a cone holding every constraint: written outright
         dev.schur_matrix(Wp, ld, M, ldm, (type == KKT_TYPE_PRIMAL) ? nullptr : cone.Fvar.K);
@@ -1137,6 +1178,7 @@ hdsdp_retcode KKT::add_sdp(SdpCone &cone, int type) {
         const int mk = cone.m;
         const long ldk = pad_ld(mk);
         if (msubCap < (size_t) ldk * mk) {
+            HB_CUDA(cudaStreamSynchronize(s));   // the blocks enqueued so far must have read the old one
             if (Msub) hb::cache_free(Msub);
             msubCap = (size_t) ldk * mk;
             HB_CUDA(hb::cmalloc(&Msub, sizeof(double) * msubCap));
@@ -1150,22 +1192,17 @@ hdsdp_retcode KKT::add_sdp(SdpCone &cone, int type) {
             HB_CUDA(cudaGetLastError());
         }
     }
-    if (tm) {
-        HB_CUDA(cudaStreamSynchronize(s));
-        tm->sch_matrix += wall() - tq;
-        tq = wall();
-    }
+    mark(2);
     dev.inner_all(Wp, ld, cone.d_vec, true);
-    add_host(asinv, cone.d_vec, h_buf, cone.m, 1.0, s, rows);
-    if (tm) {
-        tm->sch_inner += wall() - tq;
-        tq = wall();
-    }
+    to_host(cone.h_vec, cone.d_vec);
+    mark(3);
     if (r != 0.0) {
-        dev.inner_all_sq(Wp, ld, cone.d_vec, true);
-        add_host(asinvrd, cone.d_vec, h_buf, cone.m, r, s, rows);
+        dev.inner_all_sq(Wp, ld, cone.d_vec2, true);
+        to_host(cone.h_vec2, cone.d_vec2);
+        vec2 = true;
     }
-    if (tm) tm->sch_innersq += wall() - tq;
+    mark(4);
+    finish(5);
     if (type == KKT_TYPE_HOMOGENEOUS) {
         // B = W C W; <A_i, B>, <C, W>, <C, B>, r * tr(B)
         gemm(s, n, n, n, 1.0, dev.Cfull, dev.ld, 0, Wp, ld, 0, 0.0, dev.T1, dev.ld, 0);
@@ -1182,7 +1219,6 @@ hdsdp_retcode KKT::add_sdp(SdpCone &cone, int type) {
             dCSinvRdSinv += r * cone.h_scal[0];
         }
     }
-    HB_CUDA(cudaStreamSynchronize(s));
     if (tm) {
         tm->schur += wall() - t0;
         tm->n_schur += 1;
@@ -1365,14 +1401,16 @@ void KKT::add_bound(BoundCone &b, int type) {
         asinv[i] += b.duInv[i];
     }
     if (type == KKT_TYPE_CORRECTOR) return;
-    for (int i = 0; i < b.m; ++i) h_buf[i] = b.dlInv[i] * b.dlInv[i] + b.duInv[i] * b.duInv[i];
+    if (diagPending) HB_CUDA(cudaStreamSynchronize(s));   // h_diag is still being copied
+    diagPending = false;
+    for (int i = 0; i < b.m; ++i) h_diag[i] = b.dlInv[i] * b.dlInv[i] + b.duInv[i] * b.duInv[i];
     if (arrow) {
-        arrow_add_diag(h_buf);
+        arrow_add_diag(h_diag);
     } else {
         open_m();
-        HB_CUDA(cudaMemcpyAsync(d_diag, h_buf, sizeof(double) * m, cudaMemcpyHostToDevice, s));
+        HB_CUDA(cudaMemcpyAsync(d_diag, h_diag, sizeof(double) * m, cudaMemcpyHostToDevice, s));
         add_diag_vec(s, m, M, ldm, d_diag);
-        HB_CUDA(cudaStreamSynchronize(s));
+        diagPending = true;
     }
     if (type == KKT_TYPE_HOMOGENEOUS) {
         for (int i = 0; i < b.m; ++i) {
@@ -1447,6 +1485,7 @@ hdsdp_retcode KKT::factorize() {
     }
     if (ok && F.fuse_k) compute_inverse_factor(s, F);
     HB_CUDA(cudaStreamSynchronize(s));
+    diagPending = false;
     if (tm) tm->schur_factor += wall() - t0;
     return ok && !device_error_flag() ? HDSDP_RETCODE_OK : HDSDP_RETCODE_FAILED;
 }
@@ -1895,6 +1934,11 @@ __global__ void __launch_bounds__(kLzThreads, 1)
     }
 }
 
+// the coefficients of both Ritz vectors (2 (k + 1) of them), passed by value
+struct LzCoef {
+    double v[2 * (kLanczosMaxDim + 1)];
+};
+
 // ---- Lanczos for blocks above the one-CTA kernel up to order kLzClusterMaxN: one cluster of 16
 // CTAs holds the columns of K, K^T and D in its shared memory (as the cooperative variant does
 // over the whole grid) and exchanges the vectors by stores into one another's shared memory. A
@@ -2074,16 +2118,16 @@ __global__ void __launch_bounds__(kLzClThreads, 1)
 }
 
 // The Ritz part of a check: z_q = V y_q and m_q = M z_q for both coefficient vectors (y, then
-// y + kp1), warm = m_0, out[q] = |m_q - lam z_q| (and in the host's mirror hout when set).
+// y + kp1), warm = m_0, out[q] = |m_q - lam z_q|.
 __global__ void __launch_bounds__(kLzClThreads, 1)
     lz_cluster_ritz_kernel(int n, const double *K, const double *KT, long ldk, const double *D, long ldD,
-                           const double *V, long ldv, int kp1, const double *y, double lam, double *warm, double *out,
-                           double *hout) {
+                           const double *V, long ldv, int kp1, const __grid_constant__ LzCoef y, double lam, double *warm,
+                           double *out) {
     LzCluster C;
     C.init(n, K, KT, ldk, D, ldD);
     const int tid = threadIdx.x, lane = C.lane, warp = C.warp;
     double *z = C.vec, *st = z + 2 * n, *part = st + 2 * n, *red = part + 2 * kLzCl, *sy = red + kLzClWarps;
-    if (tid < 2 * kp1) sy[tid] = y[tid];
+    if (tid < 2 * kp1) sy[tid] = y.v[tid];
     __syncthreads();
     for (int i = tid; i < 2 * n; i += kLzClThreads) {
         const int q = i >= n, r = i - q * n;
@@ -2130,7 +2174,6 @@ __global__ void __launch_bounds__(kLzClThreads, 1)
     if (blockIdx.x == 0 && tid < 2) {
         const double r = sqrt(LzCluster::total(part + tid * kLzCl));
         out[tid] = r;
-        if (hout) hout[tid] = r;
     }
 }
 
@@ -2529,14 +2572,18 @@ __device__ void lanczos_small_ritz_body(int n, const double *K, long ldk, const 
 }
 
 __global__ void __launch_bounds__(kSmallLanczosThreads) lanczos_small_kernel(int n, const double *K, long ldk, const double *D, long ldD, const double *a,
-                                     const double *b, double *V, long ldv, double *ab, int maxdim) {
+                                     const double *b, double *V, long ldv, double *ab, int maxdim, double *hab) {
     lanczos_small_body(n, K, ldk, D, ldD, a, b, V, ldv, ab, maxdim);
+    if (hab) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < 2 * maxdim + 2; e += blockDim.x) hab[e] = ab[e];
+    }
 }
 
 __global__ void __launch_bounds__(kSmallRitzThreads) lanczos_small_ritz_kernel(int n, const double *K, long ldk, const double *D, long ldD,
-                                          const double *V, long ldv, int kp1, const double *y, double lam,
+                                          const double *V, long ldv, int kp1, const __grid_constant__ LzCoef y, double lam,
                                           double *warm, double *out) {
-    lanczos_small_ritz_body(n, K, ldk, D, ldD, V, ldv, kp1, y, lam, warm, out);
+    lanczos_small_ritz_body(n, K, ldk, D, ldD, V, ldv, kp1, y.v, lam, warm, out);
 }
 
 // Several cones' small-block runs in one launch, one CTA each.
@@ -2858,9 +2905,10 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
         });
         lanczos_small_kernel<<<hb::counted(1), kSmallLanczosThreads, small_lanczos_smem(n), s>>>(
             n, F.K, F.ld, D, ldD, nComputed == 0 ? nullptr : warm, nComputed == 0 ? init_vec : pert_vec, V, ld, d_ab,
-            maxdim);
+            maxdim, dm_ab);
         HB_CUDA(cudaGetLastError());
-        HB_CUDA(cudaMemcpyAsync(h_ab, d_ab, sizeof(double) * (2 * maxdim + 2), cudaMemcpyDeviceToHost, s));
+        if (!dm_ab)
+            HB_CUDA(cudaMemcpyAsync(h_ab, d_ab, sizeof(double) * (2 * maxdim + 2), cudaMemcpyDeviceToHost, s));
         HB_CUDA(cudaStreamSynchronize(s));
         if (tm) tm->n_lanczos_mv += maxdim;
     } else if (!cluster && !fused) {
@@ -2967,16 +3015,19 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
             yy[kp1 + i] = evec[(size_t) i + (size_t) i2 * kp1];
         }
         lastSteps = kp1;
-        const bool mapped = cluster && dm_yv && dm_scal;   // coefficients and residuals in place
-        if (mapped) std::memcpy(h_yv, yy.data(), sizeof(double) * 2 * kp1);
+        // one launch: the coefficients with its parameters, the residuals into pinned memory
+        const bool mapped = (cluster || small) && dm_scal;
+        LzCoef coef;
+        if (cluster || small) std::copy(yy.begin(), yy.end(), coef.v);
         else HB_CUDA(cudaMemcpyAsync(d_y, yy.data(), sizeof(double) * 2 * kp1, cudaMemcpyHostToDevice, s));
+        double *const res = mapped ? dm_scal : d_scal;
         if (cluster) {
             HB_CUDA(lz_cluster_launch(lz_cluster_ritz_kernel, lz_cl_smem(n), s, n, F.K, F.KT, F.ld, D, ldD, V, ld, kp1,
-                                      mapped ? dm_yv : d_y, eigMin1, warm, d_scal, mapped ? dm_scal : nullptr));
+                                      coef, eigMin1, warm, res));
             if (tm) tm->n_lanczos_mv += 2;
         } else if (small) {
             lanczos_small_ritz_kernel<<<hb::counted(1), kSmallRitzThreads, small_ritz_smem(n), s>>>(
-                n, F.K, F.ld, D, ldD, V, ld, kp1, d_y, eigMin1, warm, d_scal);
+                n, F.K, F.ld, D, ldD, V, ld, kp1, coef, eigMin1, warm, res);
             HB_CUDA(cudaGetLastError());
             if (tm) tm->n_lanczos_mv += 2;
         } else {

@@ -462,6 +462,8 @@ __device__ __forceinline__ void gemm_tile(const GemmP &p, int bx, int by) {
                 double v = p.alpha * acc[i][j][e];
                 if (p.beta != 0.0) v += p.beta * (*cp);
                 *cp = v;
+                // a lane's neighbours hold the mirrored entry's neighbours: whole sectors
+                if ((p.flags & GEMM_C_MIRROR) && row > col) p.C[(size_t) col + (size_t) row * p.ldc] = v;
             }
         }
     }
@@ -1001,8 +1003,7 @@ void compute_inverse_factor(cudaStream_t s, DenseFactor &F) {
 void compute_inverse(cudaStream_t s, DenseFactor &F, double *W, long ldW) {
     compute_inverse_factor(s, F);
     const int n = F.n;
-    gemm(s, n, n, n, 1.0, F.K, F.ld, 1, F.K, F.ld, 0, 0.0, W, ldW, GEMM_C_LOWER | GEMM_A_UPPER | GEMM_B_LOWER);
-    symmetrize_lower(s, n, W, ldW);
+    gemm(s, n, n, n, 1.0, F.K, F.ld, 1, F.K, F.ld, 0, 0.0, W, ldW, GEMM_C_LOWER | GEMM_C_MIRROR | GEMM_A_UPPER | GEMM_B_LOWER);
 }
 
 // ------------------------------------------------------------------------------------

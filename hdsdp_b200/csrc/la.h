@@ -13,6 +13,7 @@ namespace hb {
 
 enum GemmFlags : int {
     GEMM_C_LOWER = 1,      // compute / write only entries with row >= col
+    GEMM_C_MIRROR = 32,    // with GEMM_C_LOWER: store them above the diagonal too
     GEMM_A_LOWER = 2,      // op(A)(i,k) == 0 for k > i  (read as zero)
     GEMM_A_UPPER = 4,      // op(A)(i,k) == 0 for k < i
     GEMM_B_LOWER = 8,      // op(B)(k,j) == 0 for k < j

@@ -180,14 +180,29 @@ __global__ void scatter_sym_kernel(int nnz, const int *r, const int *c, const do
     }
 }
 
-__global__ void s_init_kernel(int n, const double *C, long ldc, double dC, double dEye, double *S, long lds) {
-    const long total = (long) n * n;
-    for (long idx = blockIdx.x * (long) blockDim.x + threadIdx.x; idx < total; idx += (long) gridDim.x * blockDim.x) {
-        int r = (int) (idx % n), c = (int) (idx / n);
+// S = dC C + dEye I, a block 256 rows of a column at a time
+__device__ __forceinline__ void s_init_body(int n, const double *C, long ldc, double dC, double dEye, double *S, long lds) {
+    const int nr = (n + 255) / 256, r = (blockIdx.x % nr) * 256 + threadIdx.x, step = gridDim.x / nr;
+    if (r >= n) return;
+    for (int c = blockIdx.x / nr; c < n; c += step) {
         double v = (dC != 0.0) ? dC * C[(size_t) r + (size_t) c * ldc] : 0.0;
         if (r == c) v += dEye;
         S[(size_t) r + (size_t) c * lds] = v;
     }
+}
+__global__ void s_init_kernel(int n, const double *C, long ldc, double dC, double dEye, double *S, long lds) {
+    s_init_body(n, C, ldc, dC, dEye, S, lds);
+}
+
+// the same, and the coefficients from the launch's parameters into w (a copy and its gap less)
+struct AsmCoef {
+    double v[kAsmParamMax];
+};
+__global__ void s_init_coef_kernel(int n, const double *C, long ldc, double dC, double dEye, double *S, long lds,
+                                   const __grid_constant__ AsmCoef coef, int m, double *w) {
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < m; i += blockDim.x) w[i] = coef.v[i];
+    s_init_body(n, C, ldc, dC, dEye, S, lds);
 }
 
 __global__ void s_gather_kernel(int npos, const int *pr, const int *pc, const int *ptr, const int *ej,
@@ -1005,9 +1020,17 @@ void SdpDevice::release() {
     h_scal = nullptr;
 }
 
-void SdpDevice::assemble(double dC, double dA, const double *d_wvec, double dEye, double *S, long ldS) {
+void SdpDevice::assemble(double dC, double dA, double *d_wvec, double dEye, double *S, long ldS, const double *hw) {
     cudaStream_t s = stream;
-    s_init_kernel<<<hb::counted(grid1((long) n * n)), 256, 0, s>>>(n, Cfull, ld, dC, dEye, S, ldS);
+    // columns in turn over as many blocks as the machine holds at once
+    const int nr = (n + 255) / 256, nb = nr * std::max(1, std::min(n, 148 * 8 / nr));
+    if (hw) {
+        AsmCoef coef;
+        std::copy(hw, hw + m, coef.v);
+        s_init_coef_kernel<<<hb::counted(nb), 256, 0, s>>>(n, Cfull, ld, dC, dEye, S, ldS, coef, m, d_wvec);
+    } else {
+        s_init_kernel<<<hb::counted(nb), 256, 0, s>>>(n, Cfull, ld, dC, dEye, S, ldS);
+    }
     if (dA != 0.0) {
         if (npos > 0)
             s_gather_kernel<<<hb::counted(grid1(npos)), 256, 0, s>>>(npos, pos_r, pos_c, pos_ptr, ent_j, ent_v, d_wvec, dA, S, ldS);

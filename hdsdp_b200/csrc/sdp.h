@@ -40,6 +40,7 @@ struct HostCoeff {
     std::vector<double> packed;
 };
 
+constexpr int kAsmParamMax = 448;   // coefficients that go with a launch's parameters (3.5 of 4 KB)
 struct SdpDevice {
     int n = 0, m = 0;
     long ld = 0;
@@ -124,7 +125,8 @@ struct SdpDevice {
     void release();
 
     // S = dC*C + dA*sum_j w_j A_j + dEye*I (full symmetric), w on device (length m)
-    void assemble(double dC, double dA, const double *d_wvec, double dEye, double *S, long ldS);
+    // with hw set (m <= kAsmParamMax) the coefficients are taken from there and d_wvec is written
+    void assemble(double dC, double dA, double *d_wvec, double dEye, double *S, long ldS, const double *hw = nullptr);
 
     // Schur complement M (m x m, lower triangle written) from symmetric W.
     // With precision 1 and Kinv = L^-1 (W = Kinv^T Kinv) the dense rank-one

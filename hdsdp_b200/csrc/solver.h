@@ -45,8 +45,9 @@ struct Timers {
 };
 
 // Lanczos maximum-step estimator (linalg/hdsdp_lanczos.c:161-292) on the GPU.
+constexpr int kLanczosMaxDim = 30;
 struct Lanczos {
-    int n = 0, maxdim = 30;
+    int n = 0, maxdim = kLanczosMaxDim;
     long ld = 0;
     cudaStream_t s = nullptr;
     double *V = nullptr, *w = nullptr, *z1 = nullptr, *z2 = nullptr, *t1 = nullptr, *u = nullptr, *warm = nullptr;
@@ -297,7 +298,10 @@ struct KKT {
     std::vector<double> asinv, asinvrd, asinvcs;
     double dCSinv = 0, dCSinvCSinv = 0, dCSinvRdSinv = 0, dTraceSinv = 0;
     double *d_rhs = nullptr, *d_x = nullptr, *d_r = nullptr, *d_t = nullptr, *d_diag = nullptr;
+    double *h_diag = nullptr;     // pinned source of d_diag; diagPending: its copy may still run
+    bool diagPending = false;
     double *h_buf = nullptr, *dm_buf = nullptr;   // pinned, and its device address (null where not mapped)
+    cudaEvent_t phase[5] = {};                    // the phases of a cone's Schur build
     double *d_words = nullptr;                    // tagged words of the fused solve, and the last tag used
     unsigned long long wordTag = 0;
     std::vector<double> diag_add;     // bound-cone diagonal accumulated before factorisation
