@@ -413,14 +413,14 @@ def schur_probe(inst, y, resi, precision: int = 0) -> dict:
     Ap, Ai, Ax = _csc(inst)
     y = np.ascontiguousarray(y, dtype=np.float64)
     m = inst.m
-    M = np.zeros(m * m)
+    M = np.empty(m * m)   # written whole: zeros above the diagonal
     asinv, asinvrd = np.zeros(m), np.zeros(m)
     tr = C.c_double()
     r = L.hdsdpb_schur_probe(m, inst.n, _ip(Ap), _ip(Ai), _dp(Ax), _dp(y), float(resi), int(precision),
                              _dp(M), _dp(asinv), _dp(asinvrd), C.byref(tr))
     if r != 0:
         raise RuntimeError("hdsdpb_schur_probe returned %d" % r)
-    return {"M": np.tril(M.reshape(m, m, order="F")), "asinv": asinv, "asinvrd": asinvrd,
+    return {"M": M.reshape(m, m, order="F"), "asinv": asinv, "asinvrd": asinvrd,
             "tracesinv": tr.value}
 
 

@@ -137,17 +137,23 @@ hdsdp_retcode SdpCone::proc_data(int nRow, int nCol, const int *Ap, const int *A
     const long npack = (long) n * (n + 1) / 2;
     auto load = [&](int col, HostCoeff &h, int &type) -> hdsdp_retcode {
         const int s0 = Ap[col], s1 = Ap[col + 1];
-        std::vector<std::pair<long, double>> ent;
-        ent.reserve(s1 - s0);
+        bool sorted = true;
         for (int e = s0; e < s1; ++e) {
             if (Ai[e] < 0 || Ai[e] >= npack) return HDSDP_RETCODE_FAILED;
-            ent.push_back({(long) Ai[e], Ax[e]});
+            sorted = sorted && (e == s0 || Ai[e - 1] <= Ai[e]);
         }
-        auto less = [](const std::pair<long, double> &x, const std::pair<long, double> &y) {
-            return x.first < y.first;
-        };
-        if (!std::is_sorted(ent.begin(), ent.end(), less)) std::stable_sort(ent.begin(), ent.end(), less);
-        const int nnz = (int) ent.size();
+        // entries out of order are sorted in a copy; the usual ones are read in place
+        std::vector<std::pair<long, double>> ent;
+        if (!sorted) {
+            ent.reserve(s1 - s0);
+            for (int e = s0; e < s1; ++e) ent.push_back({(long) Ai[e], Ax[e]});
+            std::stable_sort(ent.begin(), ent.end(), [](const std::pair<long, double> &x, const std::pair<long, double> &y) {
+                return x.first < y.first;
+            });
+        }
+        auto index = [&](int e) { return sorted ? (long) Ai[s0 + e] : ent[e].first; };
+        auto value = [&](int e) { return sorted ? Ax[s0 + e] : ent[e].second; };
+        const int nnz = s1 - s0;
         h.r.resize(nnz);
         h.c.resize(nnz);
         h.v.resize(nnz);
@@ -155,7 +161,7 @@ hdsdp_retcode SdpCone::proc_data(int nRow, int nCol, const int *Ap, const int *A
         int jc = 0;
         long colStart = 0, nextStart = n;
         for (int e = 0; e < nnz; ++e) {
-            const long q = ent[e].first;
+            const long q = index(e);
             if (q >= nextStart) {
                 unpack(n, q, h.r[e], h.c[e]);
                 jc = h.c[e];
@@ -165,7 +171,7 @@ hdsdp_retcode SdpCone::proc_data(int nRow, int nCol, const int *Ap, const int *A
                 h.c[e] = jc;
                 h.r[e] = (int) (q - colStart);
             }
-            h.v[e] = ent[e].second;
+            h.v[e] = value(e);
         }
         // sdpDataMatSetData (linalg/hdsdp_sdpdata.c:2262-2286)
         if (nnz == 0) type = REF_ZERO;
@@ -173,7 +179,7 @@ hdsdp_retcode SdpCone::proc_data(int nRow, int nCol, const int *Ap, const int *A
             type = REF_DENSE;
             h.dense_packed = true;
             h.packed.assign(npack, 0.0);
-            for (auto &p : ent) h.packed[p.first] = p.second;
+            for (int e = 0; e < nnz; ++e) h.packed[index(e)] = value(e);
         } else type = REF_SPARSE;
         return HDSDP_RETCODE_OK;
     };

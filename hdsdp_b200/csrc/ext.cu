@@ -140,10 +140,9 @@ int hdsdpb_schur_probe(int m, int n, const int *Ap, const int *Ai, const double 
         if (k.build(c, KKT_TYPE_INFEASIBLE) != HDSDP_RETCODE_OK) ret = -1;
         if (ret == 0) {
             if (M) {
-                std::vector<double> h((size_t) k.ldm * m);
-                cudaMemcpy(h.data(), k.M, sizeof(double) * k.ldm * m, cudaMemcpyDeviceToHost);
-                for (int j = 0; j < m; ++j)
-                    for (int i = 0; i < m; ++i) M[(size_t) j * m + i] = (i >= j) ? h[(size_t) j * k.ldm + i] : 0.0;
+                cudaMemcpy2D(M, sizeof(double) * m, k.M, sizeof(double) * k.ldm, sizeof(double) * m, m,
+                             cudaMemcpyDeviceToHost);
+                for (int j = 1; j < m; ++j) std::fill(M + (size_t) j * m, M + (size_t) j * m + j, 0.0);
             }
             std::memcpy(asinv, k.asinv.data(), sizeof(double) * m);
             std::memcpy(asinvrd, k.asinvrd.data(), sizeof(double) * m);

@@ -253,6 +253,12 @@ __global__ void s_gather2_long_kernel(int npos, const int *pr, const int *pc, co
     }
 }
 
+// column a of A1 (zero before): the entries ptr[a] .. ptr[a + 1) of the factors' lists
+__global__ void r1d_spread_kernel(const int *ptr, const int *idx, const double *val, double *A1, long ld) {
+    const int a = blockIdx.x;
+    for (int e = ptr[a] + threadIdx.x; e < ptr[a + 1]; e += blockDim.x) A1[idx[e] + (size_t) a * ld] = val[e];
+}
+
 __global__ void r1d_weights_kernel(int k, const int *id, const double *sign, const double *w, double dA, double *d) {
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < k; a += gridDim.x * blockDim.x) d[a] = dA * sign[a] * w[id[a]];
 }
@@ -775,12 +781,27 @@ void SdpDevice::upload(int n_, int m_, const HostCoeff &C, const std::vector<Hos
     r1d_id = upload_vec(r1did, s);
     r1d_sign = upload_vec(r1dsg, s);
     if (nr1d > 0) {
-        std::vector<double> hA1((size_t) ld * nr1d, 0.0);
+        // the factors' entries go over, and are spread on the device: their zeros need not be
+        // written by the host, nor copied
+        std::vector<int> aptr(nr1d + 1, 0), aidx;
+        std::vector<double> aval;
+        for (int a = 0; a < nr1d; ++a) aptr[a + 1] = aptr[a] + (int) A[r1did[a]].aidx.size();
+        aidx.reserve(aptr[nr1d]);
+        aval.reserve(aptr[nr1d]);
         for (int a = 0; a < nr1d; ++a) {
             const HostCoeff &c = A[r1did[a]];
-            for (size_t t = 0; t < c.aidx.size(); ++t) hA1[(size_t) a * ld + c.aidx[t]] = c.aval[t];
+            aidx.insert(aidx.end(), c.aidx.begin(), c.aidx.end());
+            aval.insert(aval.end(), c.aval.begin(), c.aval.end());
         }
-        A1 = upload_vec(hA1, s);
+        int *d_aptr = upload_vec(aptr, s), *d_aidx = upload_vec(aidx, s);
+        double *d_aval = upload_vec(aval, s);
+        HB_CUDA(hb::cmalloc(&A1, sizeof(double) * ld * nr1d));
+        HB_CUDA(cudaMemsetAsync(A1, 0, sizeof(double) * ld * nr1d, s));
+        r1d_spread_kernel<<<hb::counted(nr1d), 128, 0, s>>>(d_aptr, d_aidx, d_aval, A1, ld);
+        HB_CUDA(cudaStreamSynchronize(s));
+        hb::cache_free(d_aptr);
+        hb::cache_free(d_aidx);
+        hb::cache_free(d_aval);
         HB_CUDA(hb::cmalloc(&G, sizeof(double) * pad_ld(nr1d) * nr1d));
         if (precision >= 1) {
             // the factors a_i are fixed: split them once
