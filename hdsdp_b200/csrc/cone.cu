@@ -2391,11 +2391,11 @@ __device__ __forceinline__ void lz_dmma(double (&c)[2], double a, double b) {
 // sum over a warp of three entries a lane
 __device__ __forceinline__ double sum96(const double (&x)[3]) { return warp_sum((x[0] + x[1]) + x[2]); }
 
-// Start vector v0 = normalise(a + b) (a may be null), then maxdim steps of the
-// three-term recurrence as lanczos_orth_kernel takes them; the basis V (all maxdim + 1
-// columns, zero past a breakdown) and alpha / beta go to global memory.
+// Start vector v0 = normalise(a + b) (a may be null), or V's first column as it is (b null), then
+// the first `steps` of maxdim steps of the three-term recurrence as lanczos_orth_kernel takes
+// them; the basis V (steps + 1 columns, zero past a breakdown) and alpha / beta go to global memory.
 __device__ void lanczos_small_body(int n, const double *K, long ldk, const double *D, long ldD, const double *a,
-                                   const double *b, double *V, long ldv, double *ab, int maxdim) {
+                                   const double *b, double *V, long ldv, double *ab, int maxdim, int steps) {
     static_assert(kSmallLanczosN == 96, "three entries a lane, twelve row blocks");
     extern __shared__ double sm[];
     constexpr int P = kSmallPitch;
@@ -2445,10 +2445,10 @@ __device__ void lanczos_small_body(int n, const double *K, long ldk, const doubl
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
             const int i = lane + 32 * m;
-            v[m] = (i < n) ? (a ? a[i] : 0.0) + b[i] : 0.0;
+            v[m] = (i < n) ? (b ? (a ? a[i] : 0.0) + b[i] : V[i]) : 0.0;
             q[m] = v[m] * v[m];
         }
-        const double nrm = sqrt(sum96(q));
+        const double nrm = b ? sqrt(sum96(q)) : 1.0;
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
             const int i = lane + 32 * m;
@@ -2458,7 +2458,7 @@ __device__ void lanczos_small_body(int n, const double *K, long ldk, const doubl
         if (lane < 2) ab[2 * maxdim + lane] = 0.0;
     }
     double betaPrev = 0.0;
-    for (int k = 0; k < maxdim; ++k) {
+    for (int k = 0; k < steps; ++k) {
         __syncthreads();
         if (warp < nb) {
             double p0 = 0.0, p1 = 0.0, p2 = 0.0, p3 = 0.0;
@@ -2578,8 +2578,8 @@ __device__ void lanczos_small_ritz_body(int n, const double *K, long ldk, const 
 }
 
 __global__ void __launch_bounds__(kSmallLanczosThreads) lanczos_small_kernel(int n, const double *K, long ldk, const double *D, long ldD, const double *a,
-                                     const double *b, double *V, long ldv, double *ab, int maxdim, double *hab) {
-    lanczos_small_body(n, K, ldk, D, ldD, a, b, V, ldv, ab, maxdim);
+                                     const double *b, double *V, long ldv, double *ab, int maxdim, int steps, double *hab) {
+    lanczos_small_body(n, K, ldk, D, ldD, a, b, V, ldv, ab, maxdim, steps);
     if (hab) {
         __syncthreads();
         for (int e = threadIdx.x; e < 2 * maxdim + 2; e += blockDim.x) hab[e] = ab[e];
@@ -2618,7 +2618,7 @@ template <class Job> struct LzPack {
     Job job[kLzBatch];
 };
 __device__ void lz_run(const LzStepJob &J) {
-    lanczos_small_body(J.n, J.K, J.ldk, J.D, J.ldD, J.a, J.b, J.V, J.ldv, J.ab, J.maxdim);
+    lanczos_small_body(J.n, J.K, J.ldk, J.D, J.ldD, J.a, J.b, J.V, J.ldv, J.ab, J.maxdim, J.maxdim);
     if (J.hab) {
         __threadfence_block();
         __syncthreads();
@@ -2909,14 +2909,6 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int) small_ritz_smem(kSmallLanczosN)));
         });
-        lanczos_small_kernel<<<hb::counted(1), kSmallLanczosThreads, small_lanczos_smem(n), s>>>(
-            n, F.K, F.ld, D, ldD, nComputed == 0 ? nullptr : warm, nComputed == 0 ? init_vec : pert_vec, V, ld, d_ab,
-            maxdim, dm_ab);
-        HB_CUDA(cudaGetLastError());
-        if (!dm_ab)
-            HB_CUDA(cudaMemcpyAsync(h_ab, d_ab, sizeof(double) * (2 * maxdim + 2), cudaMemcpyDeviceToHost, s));
-        HB_CUDA(cudaStreamSynchronize(s));
-        if (tm) tm->n_lanczos_mv += maxdim;
     } else if (!cluster && !fused) {
         HB_CUDA(cudaMemsetAsync(V, 0, sizeof(double) * ld * (maxdim + 1), s));
         HB_CUDA(cudaMemsetAsync(d_ab, 0, sizeof(double) * (2 * maxdim + 2), s));
@@ -2924,6 +2916,18 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
         else lanczos_start_kernel<<<hb::counted(1), 1024, 0, s>>>(n, warm, pert_vec, V);
     }
     int stepsDone = 0;
+    // the small kernel's first `steps` steps; from V's first column when they are taken again
+    auto run_small = [&](int steps, bool again) {
+        lanczos_small_kernel<<<hb::counted(1), kSmallLanczosThreads, small_lanczos_smem(n), s>>>(
+            n, F.K, F.ld, D, ldD, nComputed == 0 ? nullptr : warm,
+            again ? nullptr : nComputed == 0 ? init_vec : pert_vec, V, ld, d_ab, maxdim, steps, dm_ab);
+        HB_CUDA(cudaGetLastError());
+        if (!dm_ab)
+            HB_CUDA(cudaMemcpyAsync(h_ab, d_ab, sizeof(double) * (2 * maxdim + 2), cudaMemcpyDeviceToHost, s));
+        HB_CUDA(cudaStreamSynchronize(s));
+        if (tm) tm->n_lanczos_mv += steps;
+        stepsDone = steps;
+    };
 
     hdsdp_retcode ret = HDSDP_RETCODE_OK;
     bool done = false;
@@ -2932,6 +2936,12 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
     std::vector<double> T, ev, evec;
     auto scheduled = [&](int k) { return ((k + 1) % freq == 0) || k >= maxdim - 1; };
     for (int k = 0; k < maxdim && !done; ++k) {
+        if (small && k >= stepsDone) {
+            // a check more than the last bound needed (1.2 us a step; all 30 took 36 us of a launch's
+            // 47); in the rare other case all of them, from the same start
+            if (k == 0) run_small(std::min(maxdim, lastSteps + freq), false);
+            else run_small(maxdim, true);
+        }
         if (fused || cluster) {
             if (k >= stepsDone) {
                 // to about where the last bound stopped (the checks below look at every scheduled
