@@ -1945,6 +1945,130 @@ struct LzCoef {
     double v[2 * (kLanczosMaxDim + 1)];
 };
 
+// The Ritz part of a check of the grid kernel's orders: z_q = V y_q and m_q = M z_q for both coefficient
+// vectors (y, then y + kp1), warm = m_0, out[q] = |m_q - lam z_q|, with the same split and exchange; the
+// columns are read from L2 once for both vectors. A bound of order 457 / 1000 / 2000 with the ten launches
+// before it: 161 / 183 / 216 us, with this one 123 / 136 / 158.
+__global__ void __launch_bounds__(kLzThreads, 1)
+    lz_grid_ritz_kernel(int n, const double *K, const double *KT, long ldk, const double *D, long ldD, LzList S,
+                        const double *V, long ldv, int kp1, const __grid_constant__ LzCoef y, double lam, double *warm,
+                        double *out, double *err, LzWord *words, unsigned long long tag) {
+    __shared__ double red[2][kLzWarps];
+    __shared__ int lost;
+    extern __shared__ double sx[];   // two vectors
+    const int G = gridDim.x, cpb = (n + G - 1) / G;
+    const int j0 = min(n, (int) blockIdx.x * cpb), nc = min(n, j0 + cpb) - j0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wpc = min(kLzMaxSegs, kLzWarps / cpb), slot = warp / wpc, seg = warp % wpc;
+    const bool own = warp == 0 && lane < nc, list = S.cnt && *S.flag != S.epoch;
+    if (tid == 0) lost = 0;
+    for (int i = tid; i < n; i += kLzThreads) {
+        double a = 0.0, b = 0.0;
+#pragma unroll 5
+        for (int j = 0; j < kp1; ++j) {
+            const double v = __ldg(V + (size_t) i + (size_t) j * ldv);
+            a += v * y.v[j];
+            b += v * y.v[kp1 + j];
+        }
+        sx[i] = a;
+        sx[n + i] = b;
+    }
+    __syncthreads();
+    double z[2], m[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) z[q] = own ? sx[q * n + j0 + lane] : 0.0;
+    // both vectors' products with the block's columns, to the first warp's threads
+    auto product = [&](const double *A, long ld, int mode) {
+        double p[2][2] = {};
+        if (slot < nc) {
+            const int j = j0 + slot;
+            if (mode == 0 && list) {
+                if (seg == 0) {
+                    p[0][0] = lz_list_dot(S, j, sx);
+                    p[1][0] = lz_list_dot(S, j, sx + n);
+                }
+            } else {
+                const int lo = (mode == 1) ? j : 0, hi = (mode == 2) ? j + 1 : n;
+                const double *col = A + (size_t) j * ld;
+                const int chunk = (((hi - lo + wpc - 1) / wpc) + 31) & ~31;
+                const int e = min(hi, lo + (seg + 1) * chunk);
+                for (int i = lo + seg * chunk + lane; i < e; i += 256) {
+                    double c[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) c[q] = (i + 32 * q < e) ? __ldg(col + i + 32 * q) : 0.0;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (i + 32 * q < e) {
+                            p[0][q & 1] += c[q] * sx[i + 32 * q];
+                            p[1][q & 1] += c[q] * sx[n + i + 32 * q];
+                        }
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const double acc = warp_sum(p[q][0] + p[q][1]);
+            if (lane == 0) red[q][warp] = acc;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            m[q] = 0.0;
+            if (own) {
+#pragma unroll
+                for (int w = 0; w < kLzMaxSegs; ++w)
+                    if (w < wpc) m[q] += red[q][lane * wpc + w];
+            }
+        }
+    };
+    auto get = [&](const LzWord *p, double &x) {
+        for (int it = 0; it < kLzPollLimit; ++it)
+            if (lz_get(p, x, tag)) return;
+        lost = 1;
+        *err = 1.0;
+    };
+    // publishes sign m and brings both vectors in; false when given up
+    auto exchange = [&](int which, double sign) {
+        LzWord *p = words + (size_t) (2 * which) * n;
+        if (own) {
+            lz_put(p + j0 + lane, sign * m[0], tag);
+            lz_put(p + n + j0 + lane, sign * m[1], tag);
+        }
+        for (int i = tid; i < 2 * n; i += kLzThreads) {
+            double x = 0.0;
+            get(p + i, x);
+            sx[i] = x;
+        }
+        __syncthreads();
+        return lost == 0;
+    };
+    product(K, ldk, 1);
+    if (!exchange(0, 1.0)) return;
+    product(D, ldD, 0);
+    if (!exchange(1, -1.0)) return;
+    product(KT, ldk, 2);
+    if (warp > 0) return;
+    LzWord *part = words + 4 * (size_t) n;
+    if (own) warm[j0 + lane] = m[0];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const double r = own ? m[q] - lam * z[q] : 0.0, p = warp_sum(r * r);
+        if (lane == 0) lz_put(part + q * G + blockIdx.x, p, tag);
+    }
+    if (blockIdx.x > 0) return;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        double v = 0.0;
+        for (int b = lane; b < G; b += 32) {
+            double x = 0.0;
+            get(part + q * G + b, x);
+            v += x;
+        }
+        v = warp_sum(v);
+        if (lane == 0) out[q] = sqrt(v);
+    }
+}
+
 // ---- Lanczos for blocks above the one-CTA kernel up to order kLzClusterMaxN: one cluster of 16
 // CTAs holds the columns of K, K^T and D in its shared memory (as the cooperative variant does
 // over the whole grid) and exchanges the vectors by stores into one another's shared memory. A
@@ -2873,12 +2997,12 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
     // in flight than the cooperative grid
     bool fused = !small && !cluster && !hyOp && n <= std::min(kLzFusedMaxN, 32 * device_sm_count());
     if (fused && !d_words) {
-        if (hb::cmalloc(&d_words, sizeof(LzWord) * 3 * n) != cudaSuccess) {
+        if (hb::cmalloc(&d_words, sizeof(LzWord) * (4 * (size_t) n + 2 * kLzFusedMaxN)) != cudaSuccess) {
             cudaGetLastError();
             d_words = nullptr;
             fused = false;
         } else {
-            HB_CUDA(cudaMemsetAsync(d_words, 0, sizeof(LzWord) * 3 * n, s));
+            HB_CUDA(cudaMemsetAsync(d_words, 0, sizeof(LzWord) * (4 * (size_t) n + 2 * kLzFusedMaxN), s));
             wordTag = 0;
         }
     }
@@ -3032,9 +3156,9 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
         }
         lastSteps = kp1;
         // one launch: the coefficients with its parameters, the residuals into pinned memory
-        const bool mapped = (cluster || small) && dm_scal;
+        const bool mapped = (cluster || small || fused) && dm_scal;
         LzCoef coef;
-        if (cluster || small) std::copy(yy.begin(), yy.end(), coef.v);
+        if (cluster || small || fused) std::copy(yy.begin(), yy.end(), coef.v);
         else HB_CUDA(cudaMemcpyAsync(d_y, yy.data(), sizeof(double) * 2 * kp1, cudaMemcpyHostToDevice, s));
         double *const res = mapped ? dm_scal : d_scal;
         if (cluster) {
@@ -3046,6 +3170,17 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
                 n, F.K, F.ld, D, ldD, V, ld, kp1, coef, eigMin1, warm, res);
             HB_CUDA(cudaGetLastError());
             if (tm) tm->n_lanczos_mv += 2;
+        } else if (fused) {
+            int nn = n, kk = kp1;
+            const double *Kp = F.K, *KTp = F.KT, *Dp = D, *Vp = V;
+            long ldk = F.ld, ldd = ldD, ldv = ld;
+            double lam = eigMin1, *wp = warm, *rp = res, *ep = (dm_ab ? dm_ab : d_ab) + 2 * maxdim + 1;
+            LzWord *words = reinterpret_cast<LzWord *>(d_words);
+            unsigned long long tag = ++wordTag;
+            void *args[] = {&nn, &Kp, &KTp, &ldk, &Dp, &ldd, &S, &Vp, &ldv, &kk, &coef, &lam, &wp, &rp, &ep, &words, &tag};
+            HB_CUDA(cudaLaunchCooperativeKernel((const void *) lz_grid_ritz_kernel, hb::counted(lzGrid), kLzThreads, args,
+                                                sizeof(double) * 2 * n, s));
+            if (tm) tm->n_lanczos_mv += 2;
         } else {
             lanczos_combine_kernel<<<hb::counted((n + 255) / 256), 256, 0, s>>>(n, V, ld, kp1, d_y, z1);
             mv(z1, z2);
@@ -3056,7 +3191,14 @@ hdsdp_retcode Lanczos::solve(DenseFactor &F, const double *D, long ldD, double *
             lanczos_resid_kernel<<<hb::counted(1), 1024, 0, s>>>(n, z1, z2, eigMin1, d_scal + 1);
         }
         if (!mapped) HB_CUDA(cudaMemcpyAsync(h_scal, d_scal, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
+        if (fused && !dm_ab)
+            HB_CUDA(cudaMemcpyAsync(h_ab, d_ab, sizeof(double) * (2 * maxdim + 2), cudaMemcpyDeviceToHost, s));
         HB_CUDA(cudaStreamSynchronize(s));
+        if (fused && h_ab[2 * maxdim + 1] != 0.0) {   // a block of the launch gave up waiting
+            device_error_flag() = 1;
+            ret = HDSDP_RETCODE_FAILED;
+            break;
+        }
         const double resiVal1 = h_scal[0], resiVal2 = h_scal[1];
         const double resiDiff = eigMin1 - eigMin2 - resiVal2;
         double valGamma = (resiDiff > 0) ? resiDiff : 1e-16;
