@@ -660,8 +660,13 @@ void coldot(cudaStream_t s, int nrows, int ncols, const double *A, long lda, con
             double *out, double alpha, double beta, int mode) {
     if (ncols <= 0) return;
     if (ncols < 4096 && nrows >= 256) {
-        // few columns: several warps per column keep enough loads in flight
-        if (ncols < 1024)
+        // few columns: several warps per column keep enough loads in flight (a solve with a factor of
+        // order 4,485 / 8,000, whose products are 1,000 columns of up to 7,000 rows, takes 115 / 296 us
+        // with sixteen, 132 / 315 with four; square ones are slower with more: order 2,001 6.4 us with
+        // four, 7.6 with eight)
+        if (ncols < 2048 && nrows > 2048)
+            coldot_seg_kernel<16><<<hb::counted(ncols), 512, 0, s>>>(nrows, A, lda, x, out, alpha, beta, mode);
+        else if (ncols < 1024)
             coldot_seg_kernel<8><<<hb::counted(ncols), 256, 0, s>>>(nrows, A, lda, x, out, alpha, beta, mode);
         else
             coldot_seg_kernel<4><<<hb::counted(ncols), 128, 0, s>>>(nrows, A, lda, x, out, alpha, beta, mode);
