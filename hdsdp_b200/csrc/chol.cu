@@ -1179,22 +1179,21 @@ __global__ void copy_lower_k(int n, const double *S, long lds, double *L, long l
 
 int sm_count() { return device_sm_count(); }
 
-int coop_grid(const void *fn) {
-    // resident cooperative CTAs, per device and kernel (two kernels use this)
-    static std::atomic<int> cached[kMaxDevices][2];
-    const int slot = (fn == (const void *) potrf_coop_kernel) ? 0 : 1;
+// resident CTAs of the cooperative factorisation, per device
+int coop_grid() {
+    static std::atomic<int> cached[kMaxDevices];
     const int dev = current_device();
-    int v = cached[dev][slot].load(std::memory_order_acquire);
+    int v = cached[dev].load(std::memory_order_acquire);
     if (v) return v;
-    static std::atomic<unsigned long long> init[2];
-    once_per_device(init[slot], [&] {
+    static std::atomic<unsigned long long> init;
+    once_per_device(init, [&] {
         const int smem = SM_DOUBLES * (int) sizeof(double);
-        HB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        HB_CUDA(cudaFuncSetAttribute(potrf_coop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         int per = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, COOP_THREADS, smem);
-        cached[dev][slot].store(std::max(1, device_sm_count() * std::max(per, 1)), std::memory_order_release);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, potrf_coop_kernel, COOP_THREADS, smem);
+        cached[dev].store(std::max(1, device_sm_count() * std::max(per, 1)), std::memory_order_release);
     });
-    return cached[dev][slot].load(std::memory_order_acquire);
+    return cached[dev].load(std::memory_order_acquire);
 }
 
 }  // namespace
@@ -1223,7 +1222,7 @@ bool coop_factorize_enqueue(cudaStream_t s, DenseFactor &F, const double *S, lon
     // at most one block per SM, so that the block factoring the diagonal never shares an SM
     // (four quarter tiles a tile where the blocks outnumber the tiles)
     const long want = 1 + 4 * (F.fuse_k ? t0 * (t0 + 1) / 2 + t0 * t0 / 4 : t0 * (t0 + 1) / 2);
-    const int grid = (int) std::max(2L, std::min<long>(std::min(coop_grid(fn), sm_count()), want));
+    const int grid = (int) std::max(2L, std::min<long>(std::min(coop_grid(), sm_count()), want));
     double *Lp = F.L;
     long ld = F.ld;
     int nn = n;
