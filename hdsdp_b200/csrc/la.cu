@@ -325,9 +325,11 @@ struct PCopy {
     }
 };
 
-// 16-byte copies: both operands start on a 16-byte boundary and have an even leading dimension
+// 16-byte copies: both operands start on a 16-byte boundary, have an even leading dimension, and a
+// tile's offsets (below 64 leading dimensions) fit the 32 bits they are kept in
 __host__ __device__ __forceinline__ bool p_pairs(const GemmP &p) {
-    return (((uintptr_t) p.A | (uintptr_t) p.B) % 16 == 0) && ((p.lda | p.ldb) % 2 == 0);
+    return (((uintptr_t) p.A | (uintptr_t) p.B) % 16 == 0) && ((p.lda | p.ldb) % 2 == 0) && p.lda < (1L << 25) &&
+           p.ldb < (1L << 25);
 }
 
 // tile (bx, by) of C
