@@ -2071,12 +2071,14 @@ __global__ void __launch_bounds__(kLzThreads, 1)
 // ---- Lanczos for blocks above the one-CTA kernel up to order kLzClusterMaxN: one cluster of 16
 // CTAs holds the columns of K, K^T and D in its shared memory (as the cooperative variant does
 // over the whole grid) and exchanges the vectors by stores into one another's shared memory. A
-// step is four exchanges, so what a barrier costs sets its time: 0.25 us in a cluster against
-// 1.2 us over the grid. The order limit is what 16 x 227 KB hold. A step bound (12 steps and the
-// Ritz part; order 100 / 200 / 300 / 456): 170 / 174 / 176 / 179 us with the cooperative kernel in
-// launches of three steps and a Ritz part of eleven launches, now 64 / 72 / 89 / 107 in two.
+// step is three exchanges (every CTA holds v_k, v_{k-1} and w whole and forms alpha and beta itself),
+// so what a barrier costs sets its time: 0.25 us in a cluster against 1.2 us over the grid. The order
+// limit is what 16 x 227 KB hold. A step bound (12 steps and the Ritz part; order 100 / 200 / 300 / 456):
+// 170 / 174 / 176 / 179 us with the cooperative kernel in launches of three steps and a Ritz part of
+// eleven launches, now 61 / 70 / 85 / 103 in two (64 / 70 / 89 / 107 with two more exchanges a step).
 constexpr int kLzCl = 16, kLzClThreads = 512, kLzClWarps = kLzClThreads / 32;
 constexpr int kLzClusterMaxN = 456;
+static_assert(kLzClusterMaxN <= kLzClThreads, "an entry a thread");
 
 __host__ __device__ inline int lz_cl_cpb(int n) { return (n + kLzCl - 1) / kLzCl; }
 inline size_t lz_cl_smem(int n) {
@@ -2169,79 +2171,62 @@ __global__ void __launch_bounds__(kLzClThreads, 1)
                             int k0, int k1) {
     LzCluster C;
     C.init(n, K, KT, ldk, D, ldD);
-    const int tid = threadIdx.x, warp = C.warp;
-    double *v = C.vec, *vp = v + n, *st = vp + n, *su = st + n, *sw = su + n, *part = sw + n, *qpart = part + kLzCl,
-           *red = qpart + kLzCl;
+    const int tid = threadIdx.x, lane = C.lane, warp = C.warp;
+    double *sv = C.vec, *st = sv + n, *su = st + n, *sw = su + n;
+    __shared__ double red[2][kLzClWarps];
     const bool first = blockIdx.x == 0;
-    double betaPrev = 0.0;
+    // the block's sum of x, by the same additions in every CTA; calls alternate between the halves of red
+    auto block_sum = [&](double x, int half) {
+        x = warp_sum(x);
+        if (lane == 0) red[half][warp] = x;
+        __syncthreads();
+        return warp_sum(lane < kLzClWarps ? red[half][lane] : 0.0);
+    };
+    double vk = 0.0, vp = 0.0, beta = 0.0;   // entry tid of v_k and v_{k-1} (n <= kLzClThreads)
     if (k0 == 0) {
-        double acc = 0.0;
-        for (int i = tid; i < n; i += kLzClThreads) {
-            const double x = (a ? a[i] : 0.0) + b[i];
-            v[i] = x;
-            acc += x * x;
-        }
-        const double nrm = sqrt(bsum(acc));
-        for (int i = tid; i < n; i += kLzClThreads) {
-            v[i] = (nrm > 0.0) ? v[i] / nrm : 0.0;
-            if (first) V[i] = v[i];
-        }
+        if (tid < n) vk = (a ? a[tid] : 0.0) + b[tid];
+        const double nrm = sqrt(block_sum(vk * vk, 0));
+        vk = (nrm > 0.0) ? vk / nrm : 0.0;
+        if (first && tid < n) V[tid] = vk;
     } else {
-        for (int i = tid; i < n; i += kLzClThreads) {
-            v[i] = V[(size_t) k0 * ldv + i];
-            vp[i] = V[(size_t) (k0 - 1) * ldv + i];
+        if (tid < n) {
+            vk = V[(size_t) k0 * ldv + tid];
+            vp = V[(size_t) (k0 - 1) * ldv + tid];
         }
-        betaPrev = ab[maxdim + k0 - 1];
+        beta = ab[maxdim + k0 - 1];
     }
+    if (tid < n) sv[tid] = vk;
     lz_cl_sync();   // every CTA is there, its vector and columns in place
     for (int k = k0; k < k1; ++k) {
         for (int c = warp; c < C.nc; c += kLzClWarps)       // t = K^T v
-            C.share(C.dot(C.colK(c), v, C.j0 + c, n), st + C.j0 + c);
+            C.share(C.dot(C.colK(c), sv, C.j0 + c, n), st + C.j0 + c);
         lz_cl_sync();
         for (int c = warp; c < C.nc; c += kLzClWarps)       // u = -D t
             C.share(-C.dot(C.sD + (long) c * n, st, 0, n), su + C.j0 + c);
         lz_cl_sync();
-        double w[2] = {}, p = 0.0;
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {                       // w = K u - beta v_{k-1}
-            const int c = warp + m * kLzClWarps, j = C.j0 + c;
-            if (c >= C.nc) break;
-            w[m] = C.dot(C.colKT(c), su, 0, j + 1);
-            if (k > 0) w[m] -= betaPrev * vp[j];
-            p += w[m] * v[j];
-        }
-        C.share_sum(p, red, part);
+        for (int c = warp; c < C.nc; c += kLzClWarps)       // w = K u
+            C.share(C.dot(C.colKT(c), su, 0, C.j0 + c + 1), sw + C.j0 + c);
         lz_cl_sync();
-        const double alp = LzCluster::total(part);
-        p = 0.0;
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const int c = warp + m * kLzClWarps, j = C.j0 + c;
-            if (c >= C.nc) break;
-            w[m] -= alp * v[j];
-            p += w[m] * w[m];
-            C.share(w[m], sw + j);
-        }
-        C.share_sum(p, red, qpart);
-        lz_cl_sync();
-        const double nrm = sqrt(LzCluster::total(qpart));
-        betaPrev = (nrm > 0.0) ? nrm : 0.0;
-        for (int i = tid; i < n; i += kLzClThreads) {
-            const double x = (nrm > 0.0) ? sw[i] / nrm : 0.0;
-            vp[i] = x;
-            if (first) V[(size_t) (k + 1) * ldv + i] = x;
+        double w = (tid < n) ? sw[tid] : 0.0;
+        if (k > 0) w -= beta * vp;
+        const double alp = block_sum(w * vk, 0);
+        w -= alp * vk;
+        const double nrm = sqrt(block_sum(w * w, 1));
+        beta = (nrm > 0.0) ? nrm : 0.0;
+        vp = vk;
+        vk = (nrm > 0.0) ? w / nrm : 0.0;
+        if (tid < n) {
+            sv[tid] = vk;
+            if (first) V[(size_t) (k + 1) * ldv + tid] = vk;
         }
         if (first && tid == 0) {
             ab[k] = alp;
-            ab[maxdim + k] = betaPrev;
+            ab[maxdim + k] = beta;
             if (hab) {
                 hab[k] = alp;
-                hab[maxdim + k] = betaPrev;
+                hab[maxdim + k] = beta;
             }
         }
-        double *const x = v;
-        v = vp;
-        vp = x;
         __syncthreads();
     }
 }
