@@ -322,6 +322,8 @@ __device__ __forceinline__ bool potf2_dev(double *L, long ld, int j0, int nb, do
             const double *Us = U + (s & 1) * 8 * PU;
             asm volatile("bar.sync 1, 256;" ::: "memory");
             const double2 u = *reinterpret_cast<const double2 *>(Us + 2 * fc + fr * PU);
+            // warp 0 may be a sweep further on by now and have failed there: that one's verdict is
+            // for the next sweep, which all of these warps reach together
             const int failed = *(volatile int *) &fail;
             const bool low = j > s;
             // the tile of column s times E_ss
@@ -330,7 +332,7 @@ __device__ __forceinline__ bool potf2_dev(double *L, long ld, int j0, int nb, do
             dmma_c(f[0], f[1], acc[0][1], u.y);
             c[0] += f[0];
             c[1] += f[1];
-            if (failed) break;
+            if (failed && failed <= 8 * (s + 1)) break;
             if (live && (low || j - 1 < s)) {
                 if (low) {
                     if (j == s + 1) {
