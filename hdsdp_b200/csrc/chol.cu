@@ -363,7 +363,10 @@ __device__ __forceinline__ bool potf2_dev(double *L, long ld, int j0, int nb, do
                 }
             }
             asm volatile("bar.sync 2, 224;" ::: "memory");
-            if (j == 2 && s == max(0, nq - 2) && lane == 0) mid();
+            if (j == 2 && s == max(0, nq - 2)) {
+                if (lane == 0) mid();
+                __syncwarp();   // the products below are the whole warp's
+            }
             if (live) {
                 if (j == s + 1) {
                     // from here on row block s of E: E_ss, and -E_ss T(q, s)^T to its right
