@@ -5,9 +5,9 @@
 // trailing lower triangle tile by tile on the DMMA path. Block 0's chain (its first rows of the
 // panel, the next diagonal block) sets the time; the blocks signal one another through counters
 // and wait only for what they read. A failed pivot (non-positive or NaN, the dpotrf test used by
-// the reference's positive-definiteness checks, linalg/hdsdp_linsolver.c:521-553) is published
-// in *info and every block leaves at its next wait for a diagonal block. The status and
-// sum log L_ii go to the host from the same launch.
+// the reference's positive-definiteness checks, linalg/hdsdp_linsolver.c:521-553) is stored
+// in *info and published with the diagonal block's signal, at which every block leaves. The status
+// and sum log L_ii go to the host from the same launch.
 //
 // Measured (factor only / with K = L^-1, ms, copy and status included): order 64 0.038 / 0.048
 // -> 0.017 / 0.021, 200 0.111 / 0.123 -> 0.049 / 0.061, 500 0.205 / 0.222 -> 0.105 / 0.115,
@@ -238,8 +238,9 @@ __device__ __forceinline__ double *region(int r) { return dyn_smem + r * 64 * TP
 // Factor the nb x nb diagonal block at (j0, j0) and write its inverse to Dinv (lower part; the
 // rest of Dinv is zero from the allocation on). With `staged` the block and the previous
 // panel's 64 rows P are in regions 3 and 2 (copies possibly still in flight) and the block is
-// first updated, A_jj -= P P^T. Executed by one block of 256 threads. Returns false (and sets
-// *info) on a failed pivot. The strictly upper part of the diagonal block in L holds zeros
+// first updated, A_jj -= P P^T. Executed by one block of 256 threads. Returns false, to every
+// thread alike, on a failed pivot (then *info is set, ahead of whatever the block releases next)
+// or when mid() gave up. The strictly upper part of the diagonal block in L holds zeros
 // (copy_lower_k and every later write keep it so), which lets whole column segments be staged.
 //
 // Sweep s turns column block s. Warp 0 factors the pivot block and publishes E_ss = L_ss^-T
@@ -247,7 +248,8 @@ __device__ __forceinline__ double *region(int r) { return dyn_smem + r * 64 * TP
 // as operands (barrier 2, without warp 0), and each row block is updated with them. The owner
 // of row s + 1 updates the next pivot block before all else and hands it to warp 0 (barrier 3).
 //
-// mid() is called by one thread of warp 2 near the end, where that warp has time to spare.
+// mid() is called by one thread of warp 2 near the end, where that warp has time to spare; false
+// means that it gave up (and has set *info).
 template <class Mid>
 __device__ __forceinline__ bool potf2_dev(double *L, long ld, int j0, int nb, double *Dinv, long ldd, int *info,
                                           bool staged, Mid mid) {
@@ -258,14 +260,14 @@ __device__ __forceinline__ bool potf2_dev(double *L, long ld, int j0, int nb, do
     // pitches keep the reads of the other operand free of bank conflicts in that order.
     constexpr int PU = 72, PB = 66;
     double *U = region(R_X), *Ls = U + 16 * PU, *B = U + 32 * PU;
-    __shared__ int fail;
+    __shared__ int fail, lost;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double *Ljj = L + (size_t) j0 + (size_t) j0 * ld;
     double *Dj = Dinv + j0;
     const bool vec = ((((size_t) Dj) & 15) == 0) && ((ldd & 1) == 0);   // two rows of Dinv a store
     if (!staged) stage_tile(T, Ljj, ld, nb, nb, 64, true);
     cpa_wait_all();
-    if (tid == 0) fail = 0;
+    if (tid == 0) fail = lost = 0;
     for (int r = nb + tid; r < 64; r += blockDim.x) T[r + r * TP] = 1.0;  // pad with the identity
     __syncthreads();
     const int sb = 4096 + (j0 / 64) * 32;
@@ -364,7 +366,7 @@ __device__ __forceinline__ bool potf2_dev(double *L, long ld, int j0, int nb, do
             }
             asm volatile("bar.sync 2, 224;" ::: "memory");
             if (j == 2 && s == max(0, nq - 2)) {
-                if (lane == 0) mid();
+                if (lane == 0 && !mid()) lost = 1;
                 __syncwarp();   // the products below are the whole warp's
             }
             if (live) {
@@ -413,11 +415,11 @@ __device__ __forceinline__ bool potf2_dev(double *L, long ld, int j0, int nb, do
     }
     __syncthreads();
     CHOL_STAMP(sb + 11);
-    if (fail) {
-        if (tid == 0) *info = j0 + fail;
-        return false;
-    }
-    return true;
+    const int failed = fail, gaveUp = lost;
+    if (!failed && !gaveUp) return true;
+    if (tid == 0 && !gaveUp) *info = j0 + failed;
+    __syncthreads();
+    return false;
 }
 
 // Tile product on the DMMA path over K = nb <= 64:
@@ -678,6 +680,11 @@ __device__ __forceinline__ void k_final_tile(const double *Dinv, long ldd, doubl
 // Block 0 is the chain that sets the time, so it waits for the others only where it must: it
 // needs the last panel's updates (which are done long before it has finished the diagonal block
 // it is in), and the others need its diagonal blocks and its rows of the panel.
+//
+// Whether to go on is decided once per block and never from *info, which others may be writing:
+// block 0 by what potf2_dev returns to all of its threads, the others by what their waits return.
+// After a failure in diagonal block q every other block still takes part in panel q and leaves at
+// its wait for diagonal block q, whenever it gets there, so no arrival that others count on is lost.
 template <bool ONE, class Sync>
 __device__ __forceinline__ void potrf_body(double *L, long ld, int n, double *Dinv, long ldd, int *info, double *K,
                                            double *KT, int bid, int ngrid, Sync &sync) {
@@ -692,7 +699,7 @@ __device__ __forceinline__ void potrf_body(double *L, long ld, int n, double *Di
         const long nx = (K && bj >= 1) ? (long) (nblk - bj) * bj : 0;
         if ((ONE || bid > 0) && nx > 0) {
             auto kjob = [&](long u) { return k_update_job(L, ld, K, n, bj + (int) (u / bj), (int) (u % bj), bj - 1); };
-            if (!ONE) sync.update_wait_all(bj);
+            if (!sync.update_wait_all(bj)) return;
             if (2 * nx <= nworker) {
                 // half the blocks would stay idle: quarter tiles
                 for (long t = wid; t < 4 * nx; t += nworker) {
@@ -703,11 +710,7 @@ __device__ __forceinline__ void potrf_body(double *L, long ld, int n, double *Di
                 tile_stream([&](long u, TileJob &J) { J = kjob(u); }, wid, nx, nworker);
             }
         }
-        if (!ONE && !first && bid > 0) sync.diag_wait(jn / NB);
-        if (!first && *(volatile int *) info) {
-            if (bid == 0) sync.diag_release(jn / NB);   // the others wait for it before they look
-            return;
-        }
+        if (!first && bid > 0 && !sync.diag_wait(jn / NB)) return;
         const int j0 = jn - NB, rows = n - jn, nchunk = (rows + 63) / 64, nbn = min(NB, rows);
         double *P = L + (size_t) jn + (size_t) j0 * ld, *A22 = L + (size_t) jn + (size_t) jn * ld;
         const int pb = bj * 16 + (bid == 1 ? 8 : 0);
@@ -727,11 +730,15 @@ __device__ __forceinline__ void potrf_body(double *L, long ld, int n, double *Di
                 if (!ONE) sync.panel_arrive();
                 if (bid <= 1) CHOL_STAMP(pb + 2);
             }
-            potf2_dev(L, ld, jn, nbn, Dinv, ldd, info, !first, [&]() {
+            const bool good = potf2_dev(L, ld, jn, nbn, Dinv, ldd, info, !first, [&]() {
                 // the panel's updates by the other blocks, before the next panel
-                if (!ONE && !first) sync.update_wait(jn / NB);
+                return first || sync.update_wait(jn / NB);
             });
             if (!first && bid <= 1) CHOL_STAMP(pb + 4);
+            if (!good) {
+                sync.diag_failed(jn / NB);
+                return;
+            }
         }
         if (!first && (ONE || bid > 0)) {
             // the rest of the panel, by half chunks where the blocks outnumber them
@@ -750,7 +757,7 @@ __device__ __forceinline__ void potrf_body(double *L, long ld, int n, double *Di
             }
             if (bid == 1) CHOL_STAMP(pb + 1);
             if (!ONE) sync.panel_arrive();
-            sync.panel_wait(jn / NB);
+            if (!sync.panel_wait(jn / NB)) return;
             if (bid == 1) CHOL_STAMP(pb + 2);
             // the trailing matrix (tile 0 is the next diagonal block) and K's block row bj
             const long ntile = (long) nchunk * (nchunk + 1) / 2, nk = K ? bj + 1 : 0;
@@ -782,9 +789,9 @@ __device__ __forceinline__ void potrf_body(double *L, long ld, int n, double *Di
         }
         if (!first && bid <= 1) CHOL_STAMP(pb + 5);
     }
-    if (bid > 0) sync.diag_wait(nblk);
-    else sync.diag_release(nblk);
-    if (!K || *(volatile int *) info) return;
+    if (bid == 0) sync.diag_release(nblk);
+    else if (!sync.diag_wait(nblk)) return;
+    if (!K) return;
     // the last block row of K: its update by block row nblk - 2, then its final form
     const int bj = nblk - 1;
     if (2 * bj <= ngrid) {
@@ -792,72 +799,92 @@ __device__ __forceinline__ void potrf_body(double *L, long ld, int n, double *Di
             TileJob J = k_update_job(L, ld, K, n, bj, t >> 2, bj - 1);
             if (sub_job(J, 32, 32, 32 * (t & 1), 32 * ((t >> 1) & 1))) Tile<32, 32>::run(J);
         }
-        if (bj >= 1) sync.all();
+        if (bj >= 1 && !sync.all()) return;
         for (int t = bid; t < 2 * (bj + 1); t += ngrid) k_final_tile(Dinv, ldd, K, KT, ld, n, bj, t >> 1, t & 1, 2);
         return;
     }
     for (int c = bid; c < bj; c += ngrid) Tile64::run(k_update_job(L, ld, K, n, bj, c, bj - 1));
-    if (bj >= 1) sync.all();
+    if (bj >= 1 && !sync.all()) return;
     for (int c = bid; c <= bj; c += ngrid) k_final_tile(Dinv, ldd, K, KT, ld, n, bj, c, 0, 1);
 }
 
-// The signals between the blocks of a cooperative launch: counters in global memory that start
-// at zero and only grow. One thread of a block (of warp 3, which has time to spare in the
-// diagonal blocks) signals and waits for all of it. Waits are bounded; a wait that gives up
-// sets *info, which every block checks after its waits.
+// The signals between the blocks of a cooperative launch: words in global memory that start at zero
+// and only grow. One thread of a block signals and polls for all of it: thread kThread (of warp 3,
+// which has time to spare in the diagonal blocks), or in block 0's update_wait() the thread that
+// calls it. Waits are bounded and return the same to every thread of the block: false when the wait
+// gave up, which sets *info to -1, or, for a diagonal block, when it failed.
 struct GridSync {
-    unsigned *c;    // 0: all(), 1: panel, 2: updates, 3: diagonal blocks done
+    unsigned *c;    // 0: all(), 1: panel, 2: updates, 3: diagonal blocks done (and kFailed)
     int *info;
     unsigned nall = 0;
     static constexpr int kThread = 96;
+    static constexpr unsigned kFailed = 1u << 31;   // the last one counted by word 3 has failed
     __device__ __forceinline__ void add(int k) {
         __syncthreads();
         if (threadIdx.x == kThread) {
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(c + k) : "memory");
         }
     }
-    __device__ __forceinline__ void poll(int k, unsigned target) {   // one thread
-        unsigned v = 0;
-        long it = 0;
-        do {
+    // one thread: the word once it has reached the target (but for kFailed); false on giving up
+    __device__ __forceinline__ bool poll(int k, unsigned target, unsigned &v) {
+        for (long it = 0; it < (1L << 22); ++it) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(c + k) : "memory");
-        } while ((int) (v - target) < 0 && ++it < (1L << 22));
-        if ((int) (v - target) < 0) *(volatile int *) info = -1;
+            if ((v & ~kFailed) >= target) return true;
+        }
+        *(volatile int *) info = -1;
+        return false;
     }
-    __device__ __forceinline__ void wait(int k, unsigned target) {
-        if (threadIdx.x == kThread) poll(k, target);
-        __syncthreads();
+    __device__ __forceinline__ bool wait(int k, unsigned target) {
+        unsigned v;
+        return !__syncthreads_or(threadIdx.x == kThread && !poll(k, target, v));
     }
     // every block has finished its part of panel p (block 0 its chunk 0)
     __device__ __forceinline__ void panel_arrive() { add(1); }
-    __device__ __forceinline__ void panel_wait(int p) { wait(1, (unsigned) p * gridDim.x); }
+    __device__ __forceinline__ bool panel_wait(int p) { return wait(1, (unsigned) p * gridDim.x); }
     // the blocks beside block 0 have finished their updates by panel p (awaited by one thread of block 0)
     __device__ __forceinline__ void update_arrive() { add(2); }
-    __device__ __forceinline__ void update_wait(int p) { poll(2, (unsigned) p * (gridDim.x - 1)); }
-    __device__ __forceinline__ void update_wait_all(int p) { wait(2, (unsigned) p * (gridDim.x - 1)); }
+    __device__ __forceinline__ bool update_wait(int p) {
+        unsigned v;
+        return poll(2, (unsigned) p * (gridDim.x - 1), v);
+    }
+    __device__ __forceinline__ bool update_wait_all(int p) { return wait(2, (unsigned) p * (gridDim.x - 1)); }
     // block 0 has finished d diagonal blocks (and seen the updates before the last of them)
-    __device__ __forceinline__ void diag_release(int d) {   // after a block barrier
+    __device__ __forceinline__ void diag_release(unsigned d) {   // after a block barrier
         if (threadIdx.x == kThread) {
             asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(c + 3), "r"(d) : "memory");
         }
     }
-    __device__ __forceinline__ void diag_wait(int d) { wait(3, (unsigned) d); }
-    __device__ __forceinline__ void all() {
+    // diagonal block q has failed, those before it are done
+    __device__ __forceinline__ void diag_failed(int q) { diag_release((unsigned) (q + 1) | kFailed); }
+    // d diagonal blocks done; false when the d-th of them failed
+    __device__ __forceinline__ bool diag_wait(int d) {
+        unsigned v;
+        return !__syncthreads_or(threadIdx.x == kThread &&
+                                 (!poll(3, (unsigned) d, v) || v == ((unsigned) d | kFailed)));
+    }
+    __device__ __forceinline__ bool all() {
         add(0);
-        wait(0, ++nall * gridDim.x);
+        return wait(0, ++nall * gridDim.x);
     }
 };
 
 // the same for a grid of one block
 struct BlockSync {
     __device__ __forceinline__ void panel_arrive() {}
-    __device__ __forceinline__ void panel_wait(int) { __syncthreads(); }
+    __device__ __forceinline__ bool panel_wait(int) {
+        __syncthreads();
+        return true;
+    }
     __device__ __forceinline__ void update_arrive() { __syncthreads(); }
-    __device__ __forceinline__ void update_wait(int) {}
-    __device__ __forceinline__ void update_wait_all(int) {}
-    __device__ __forceinline__ void diag_release(int) {}
-    __device__ __forceinline__ void diag_wait(int) {}
-    __device__ __forceinline__ void all() { __syncthreads(); }
+    __device__ __forceinline__ bool update_wait(int) { return true; }
+    __device__ __forceinline__ bool update_wait_all(int) { return true; }
+    __device__ __forceinline__ void diag_release(unsigned) {}
+    __device__ __forceinline__ void diag_failed(int) {}
+    __device__ __forceinline__ bool diag_wait(int) { return true; }
+    __device__ __forceinline__ bool all() {
+        __syncthreads();
+        return true;
+    }
 };
 
 // sum_i log L_ii summed as the log-diagonal kernel sums it with its 1024 threads (terms v,
@@ -907,7 +934,8 @@ __global__ void __launch_bounds__(COOP_THREADS, 1)
                       double *hinfo, int logdet) {
     GridSync sync{reinterpret_cast<unsigned *>(info) + kInfoCounters, info};
     potrf_body<false>(L, ld, n, Dinv, ldd, info, K, KT, (int) blockIdx.x, (int) gridDim.x, sync);
-    // block 0 has the last word on *info: the others' waits end before its own work does
+    // block 0 has the last word on *info: the others' waits end before its own work does, and blocks
+    // still on their way out after a failed pivot leave it alone
     if (blockIdx.x == 0 && (logdet || hinfo)) write_status(n, L, ld, info, hinfo, logdet);
 }
 
