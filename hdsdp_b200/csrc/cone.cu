@@ -574,10 +574,11 @@ void assemble_buffers(const std::vector<SdpCone *> &cones, double dC, double dAs
     if (tm) tm->assemble += wall() - t0;
 }
 
-static void copy_factor(cudaStream_t s, DenseFactor &dst, const DenseFactor &src) {
+void copy_factor(cudaStream_t s, DenseFactor &dst, const DenseFactor &src) {
     HB_CUDA(cudaMemcpyAsync(dst.L, src.L, sizeof(double) * src.ld * src.n, cudaMemcpyDeviceToDevice, s));
     HB_CUDA(cudaMemcpyAsync(dst.Dinv, src.Dinv, sizeof(double) * src.ld * 64, cudaMemcpyDeviceToDevice, s));
     dst.k_valid = false;
+    dst.rec_strips = false;   // dst's strips are those of another factor: solves go by Dinv
     if (src.k_valid && src.K && src.KT) {
         if (!dst.K) HB_CUDA(hb::cmalloc(&dst.K, sizeof(double) * dst.ld * dst.n));
         if (!dst.KT) HB_CUDA(hb::cmalloc(&dst.KT, sizeof(double) * dst.ld * dst.n));

@@ -465,6 +465,37 @@ int hdsdpb_cholesky_solve(int n, const double *S, const double *b, double *x) {
     return ret;
 }
 
+int hdsdpb_cholesky_copy_solve(int n, const double *S0, const double *S, const double *b, double *x) {
+    if (n <= 0 || !S0 || !S || !b || !x) return -1;
+    cudaStream_t s;
+    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return -1;
+    const long ld = pad_ld(n);
+    double *dS = nullptr, *dx = nullptr;
+    hb::cmalloc(&dS, sizeof(double) * ld * n);
+    hb::cmalloc(&dx, sizeof(double) * n);
+    cudaMemcpy(dx, b, sizeof(double) * n, cudaMemcpyHostToDevice);
+    DenseFactor F[2];
+    bool ok = true;
+    for (int q = 0; q < 2; ++q) {
+        cudaMemcpy2D(dS, sizeof(double) * ld, q ? S : S0, sizeof(double) * n, sizeof(double) * n, n, cudaMemcpyHostToDevice);
+        F[q].alloc(n, 0);   // ends in a fence
+        ok = factorize(s, F[q], dS, ld) && ok;
+    }
+    int ret = ok ? 0 : 1;
+    if (ok) {
+        copy_factor(s, F[0], F[1]);
+        if (!chol_solve(s, F[0], dx, dx)) ret = -1;
+        cudaMemcpyAsync(x, dx, sizeof(double) * n, cudaMemcpyDeviceToHost, s);
+    }
+    cudaStreamSynchronize(s);
+    if (ok && chol_solve_error()) ret = -1;
+    for (DenseFactor &G : F) G.release();
+    hb::cache_free(dS);
+    hb::cache_free(dx);
+    cudaStreamDestroy(s);
+    return device_error_flag() ? -1 : ret;
+}
+
 int hdsdpb_inverse(int n, const double *S, double *Sinv) {
     if (n < 0 || (n > 0 && (!S || !Sinv))) return -1;
     if (n == 0) return 0;

@@ -147,6 +147,8 @@ struct DenseFactor {
 // device vectors of length n and may alias. Returns false if the launch failed or a
 // bounded wait inside it gave up.
 bool chol_solve(cudaStream_t s, DenseFactor &F, const double *b, double *x);
+// dst = src, two factors of the same order (K and KT only where src's are valid).
+void copy_factor(cudaStream_t s, DenseFactor &dst, const DenseFactor &src);
 // Reads and clears the flag raised when a wait inside chol_solve gave up (synchronising).
 int chol_solve_error();
 

@@ -171,6 +171,11 @@ extern int hdsdpb_cholesky_batch( int count, int n, int mode, const double *S, d
    not positive definite, -1 on error. */
 extern int hdsdpb_cholesky_solve( int n, const double *S, const double *b, double *x );
 
+/* The same with a copied factor, as a cone copies one whose slack matrix it meets again: S0 is
+   factored in one object and S in another, the second factor is copied over the first, and the
+   first solves S x = b. */
+extern int hdsdpb_cholesky_copy_solve( int n, const double *S0, const double *S, const double *b, double *x );
+
 /* Solution of S x = b for a symmetric, possibly indefinite S (n x n, column-major, only
    its lower triangle read) through P S P^T = L D L^T with Bunch-Kaufman pivoting (the
    reference's dsytrf / dsytrs use, linalg/hdsdp_linsolver.c:1118-1190). out (may be NULL):
