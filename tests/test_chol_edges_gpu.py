@@ -86,3 +86,22 @@ def test_batch_is_the_grid_factor(gpu_lib):
             got.append((L, K, ld))
         for a, b in zip(*got):
             assert np.array_equal(a, b)
+
+
+def test_reciprocal_square_root_of_a_pivot(gpu_lib):
+    """Diagonal matrices over the range of pivots that the straight-line reciprocal square root takes
+    (2^-500 to 2^500), all mantissas and their ends: L^-1 holds it in the first column of each pair of
+    columns, and in the second the square roots of the determinant and of the first pivot times it."""
+    n, u = 1024, 2.0 ** -53
+    rng = np.random.default_rng(0)
+    edge = np.array([1.0, 1.0 + 2 * u, 1.5, 2.0 - 2 * u, 2.0, 2.0 + 4 * u, 3.0, 4.0 - 4 * u])
+    sets = [rng.uniform(1.0, 4.0, n), np.tile(edge, n // edge.size), rng.uniform(1.0, 4.0, n) * 2.0 ** rng.integers(-498, 498, n),
+            np.tile(edge, n // edge.size) * 2.0 ** (2 * rng.integers(-249, 249, n))]
+    for d in sets:
+        _, K = _factor_and_inverse(np.diag(d))
+        exact = 1.0 / np.sqrt(d.astype(np.longdouble))
+        err = np.abs((np.diag(K) - exact) / exact).astype(float) / u
+        # 1.5 u of roundings and a margin for the iteration's own error; a second column has two of
+        # these, the determinant's half rounding and two products
+        assert err[0::2].max() <= 2.0
+        assert err[1::2].max() <= 2 * 2.0 + 0.5 + 2.0
