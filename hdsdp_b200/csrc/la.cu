@@ -476,10 +476,11 @@ constexpr int kPBytes = P_ST * (kPStage<BM_, !TA> + kPStage<BN_, TB != 0>) * (in
 
 // GEMM z = blockIdx.z of a strided group (one product: z = 0): operands at A + z sa, B + z sb,
 // C + z sc; with kstep set, the K range [z kstep, (z + 1) kstep) of one product (sa and sb then
-// move along K); the group's last product has mLast rows and kLast of K when these are set
+// move along K); the group's last product has mLast rows and kLast of K when these are set. The
+// launch's first column tile is y0.
 template <int BM_, int BN_, int P_ST, int MINB, int TA, int TB>
 __global__ void __launch_bounds__(P_T, MINB) gemm_kernel(GemmP p, long sa, long sb, long sc, int kstep, int mLast,
-                                                             int kLast) {
+                                                             int kLast, int y0) {
     const int z = blockIdx.z;
     p.A += z * sa;
     p.B += z * sb;
@@ -490,7 +491,7 @@ __global__ void __launch_bounds__(P_T, MINB) gemm_kernel(GemmP p, long sa, long 
         p.K = kLast;
         if ((int) blockIdx.x * BM_ >= mLast) return;
     }
-    gemm_tile<BM_, BN_, P_ST, TA, TB>(p, blockIdx.x, blockIdx.y);
+    gemm_tile<BM_, BN_, P_ST, TA, TB>(p, blockIdx.x, y0 + blockIdx.y);
 }
 
 // Tile sizes, by measurement (us for C = A B of order n, the 64 x 64 tile against the 32 x 32 one):
@@ -499,6 +500,7 @@ __global__ void __launch_bounds__(P_T, MINB) gemm_kernel(GemmP p, long sa, long 
 // entries of C. The small tile's copies run five stages ahead because its DMMAs take only 256
 // cycles a k-tile.
 constexpr long kGemmLargeMN = 3072L * 3072L;
+constexpr int kGridYMax = 65535;   // blocks of a grid in y (and z); more columns take several launches
 constexpr int kGemmSt32 = 5, kGemmBlk32 = 4, kGemmSt64 = 3, kGemmBlk64 = 3;
 
 template <int BM_, int BN_, int P_ST, int MINB, int TA, int TB>
@@ -510,9 +512,13 @@ void launch_tiles(const GemmP &p, long sa, long sb, long sc, int count, int kste
         HB_CUDA(cudaFuncSetAttribute(gemm_kernel<BM_, BN_, P_ST, MINB, TA, TB>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     });
-    dim3 grid((p.M + BM_ - 1) / BM_, (p.N + BN_ - 1) / BN_, count);
-    gemm_kernel<BM_, BN_, P_ST, MINB, TA, TB><<<hb::counted(grid), P_T, bytes, s>>>(p, sa, sb, sc, kstep, mLast, kLast);
-    HB_CUDA(cudaGetLastError());
+    const int ny = (p.N + BN_ - 1) / BN_;
+    for (int y0 = 0; y0 < ny; y0 += kGridYMax) {
+        dim3 grid((p.M + BM_ - 1) / BM_, std::min(kGridYMax, ny - y0), count);
+        gemm_kernel<BM_, BN_, P_ST, MINB, TA, TB><<<hb::counted(grid), P_T, bytes, s>>>(p, sa, sb, sc, kstep, mLast, kLast,
+                                                                                       y0);
+        HB_CUDA(cudaGetLastError());
+    }
 }
 
 template <int TA, int TB>
@@ -533,28 +539,29 @@ void launch_gemm(const GemmP &p, long sa, long sb, long sc, int count, int kstep
 }
 
 // one GEMM of a group per blockIdx.z (tiles beyond its own M x N exit)
-__global__ void __launch_bounds__(P_T, kGemmBlk32) gemm_grouped_kernel(const GemmP *__restrict__ ps) {
+__global__ void __launch_bounds__(P_T, kGemmBlk32) gemm_grouped_kernel(const GemmP *__restrict__ ps, int y0) {
     const GemmP p = ps[blockIdx.z];
-    if ((int) blockIdx.x * 32 >= p.M || (int) blockIdx.y * 32 >= p.N) return;
+    const int bx = blockIdx.x, by = y0 + blockIdx.y;
+    if (bx * 32 >= p.M || by * 32 >= p.N) return;
     if (p.ta) {
-        if (p.tb) gemm_tile<32, 32, kGemmSt32, 1, 1>(p, blockIdx.x, blockIdx.y);
-        else gemm_tile<32, 32, kGemmSt32, 1, 0>(p, blockIdx.x, blockIdx.y);
+        if (p.tb) gemm_tile<32, 32, kGemmSt32, 1, 1>(p, bx, by);
+        else gemm_tile<32, 32, kGemmSt32, 1, 0>(p, bx, by);
     } else {
-        if (p.tb) gemm_tile<32, 32, kGemmSt32, 0, 1>(p, blockIdx.x, blockIdx.y);
-        else gemm_tile<32, 32, kGemmSt32, 0, 0>(p, blockIdx.x, blockIdx.y);
+        if (p.tb) gemm_tile<32, 32, kGemmSt32, 0, 1>(p, bx, by);
+        else gemm_tile<32, 32, kGemmSt32, 0, 0>(p, bx, by);
     }
 }
 }  // namespace
 
 void gemm_strided(cudaStream_t s, const GemmDesc &d, long sa, long sb, long sc, int count, int kstep) {
     if (count <= 0 || d.M <= 0 || d.N <= 0) return;
-    for (int z0 = 0; z0 < count; z0 += 65535) {
+    for (int z0 = 0; z0 < count; z0 += kGridYMax) {
         GemmP p = d;
         p.A += z0 * sa;
         p.B += z0 * sb;
         p.C += z0 * sc;
         if (kstep > 0) p.K -= z0 * kstep;
-        launch_gemm(p, sa, sb, sc, std::min(65535, count - z0), kstep, 0, 0, s);
+        launch_gemm(p, sa, sb, sc, std::min(kGridYMax, count - z0), kstep, 0, 0, s);
     }
 }
 
@@ -566,11 +573,13 @@ void gemm_grouped(cudaStream_t s, const GemmDesc *d_desc, int count, int maxM, i
     once_per_device(init, [] {
         HB_CUDA(cudaFuncSetAttribute(gemm_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     });
-    for (int z0 = 0; z0 < count; z0 += 65535) {
-        dim3 grid((maxM + 31) / 32, (maxN + 31) / 32, std::min(65535, count - z0));
-        gemm_grouped_kernel<<<hb::counted(grid), P_T, bytes, s>>>(d_desc + z0);
-        HB_CUDA(cudaGetLastError());
-    }
+    const int ny = (maxN + 31) / 32;
+    for (int z0 = 0; z0 < count; z0 += kGridYMax)
+        for (int y0 = 0; y0 < ny; y0 += kGridYMax) {
+            dim3 grid((maxM + 31) / 32, std::min(kGridYMax, ny - y0), std::min(kGridYMax, count - z0));
+            gemm_grouped_kernel<<<hb::counted(grid), P_T, bytes, s>>>(d_desc + z0, y0);
+            HB_CUDA(cudaGetLastError());
+        }
 }
 
 void gemm(cudaStream_t s, int M, int N, int K, double alpha, const double *A, long lda, int transA,

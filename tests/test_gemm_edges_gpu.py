@@ -47,3 +47,20 @@ def test_gemm_edges(m, n, k, pad, ta, tb):
     assert lib.hdsdpb_gemm(m, n, k, 0.75, _ptr(abuf), lda, ta, _ptr(bbuf), ldb, tb, -0.5, _ptr(cbuf), ldc) == 0
     assert (np.abs(c - want) <= bound).all()
     assert np.isnan(cbuf[:, m:]).all()
+
+
+@pytest.mark.parametrize("tb", [0, 1])
+def test_more_column_tiles_than_a_grid_has(tb):
+    """65,535 tiles of 32 columns and one more column, which takes a second launch."""
+    lib = _lib.load()
+    m, n, k = 3, 65535 * 32 + 1, 2
+    rng = np.random.default_rng(tb)
+    a = np.asfortranarray(rng.standard_normal((m, k)))
+    b = rng.standard_normal((n, k)) if tb else rng.standard_normal((k, n))
+    b = np.asfortranarray(b)
+    c = np.zeros((m, n), order="F")
+    lib.hdsdpb_gemm.argtypes = [C.c_int] * 3 + [C.c_double, C.POINTER(C.c_double), C.c_int, C.c_int, C.POINTER(C.c_double),
+                                                C.c_int, C.c_int, C.c_double, C.POINTER(C.c_double), C.c_int]
+    assert lib.hdsdpb_gemm(m, n, k, 1.0, _ptr(a), m, 0, _ptr(b), n if tb else k, tb, 0.0, _ptr(c), m) == 0
+    op = b.T if tb else b
+    assert (np.abs(c - a @ op) <= 4 * (k + 4) * 2.0 ** -53 * (np.abs(a) @ np.abs(op))).all()
