@@ -309,16 +309,17 @@ __global__ void dr_axpy_kernel(int n, int ndr, const int *__restrict__ id, const
     }
 }
 
-// part[j gridDim.x + b] = block b's share of <A_j, Z> (columns b, b + gridDim.x, ...), or the
-// whole of it into out[id[j]] when one block takes a matrix
+// matrix j = blockIdx.x (there may be more of them than a grid has blocks in y): part[j gridDim.y + b]
+// = block b's share of <A_j, Z> (columns b, b + gridDim.y, ...), or the whole of it into out[id[j]]
+// when one block takes a matrix
 __global__ void dr_inner_kernel(int n, const int *__restrict__ id, const double *__restrict__ A, long lda,
                                 const double *__restrict__ Z, long ldz, double *part, double *out) {
     __shared__ double red[32];
-    const int j = blockIdx.y;
+    const int j = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const double *a = A + (size_t) j * lda * n;
     double acc = 0.0;
-    for (int c = blockIdx.x * nw + warp; c < n; c += gridDim.x * nw) {
+    for (int c = blockIdx.y * nw + warp; c < n; c += gridDim.y * nw) {
         const double *ac = a + (size_t) c * lda, *zc = Z + (size_t) c * ldz;
         for (int r = lane; r < n; r += 32) acc += ac[r] * zc[r];
     }
@@ -329,8 +330,8 @@ __global__ void dr_inner_kernel(int n, const int *__restrict__ id, const double 
     if (threadIdx.x == 0) {
         double t = 0.0;
         for (int q = 0; q < nw; ++q) t += red[q];
-        if (gridDim.x == 1) out[id[j]] = t;
-        else part[(size_t) j * gridDim.x + blockIdx.x] = t;
+        if (gridDim.y == 1) out[id[j]] = t;
+        else part[(size_t) j * gridDim.y + blockIdx.y] = t;
     }
 }
 
@@ -862,7 +863,8 @@ void SdpDevice::upload(int n_, int m_, const HostCoeff &C, const std::vector<Hos
         }
         // as many products at a time as fit kDrScratch; the inner products split along the
         // entries until their 64 x 64 tiles give the SMs two blocks each (at least 128 entries)
-        dr_chunk = (int) std::max<size_t>(1, std::min<size_t>(ndr, kDrScratch / (sizeof(double) * mat)));
+        // (and no more than a grid has blocks in y)
+        dr_chunk = (int) std::max<size_t>(1, std::min<size_t>(std::min(ndr, 65535), kDrScratch / (sizeof(double) * mat)));
         const long tiles = (long) ((ndr + 63) / 64) * ((dr_chunk + 63) / 64);
         const long want = std::max(1L, 296 / tiles);
         const long entries = ld * n;
@@ -1199,7 +1201,7 @@ void SdpDevice::schur_matrix(const double *W, long ldW, double *M, long ldM, con
 
 void SdpDevice::dr_inner(const double *Z, long ldZ, double *out) {
     if (ndr == 0) return;
-    const dim3 grid(dr_dsplit, ndr);
+    const dim3 grid(ndr, dr_dsplit);
     dr_inner_kernel<<<hb::counted(grid), 256, 0, stream>>>(n, dr_id, dr_slab, ld, Z, ldZ, dr_part, out);
     if (dr_dsplit > 1)
         dr_sum_kernel<<<hb::counted((ndr + 63) / 64), 64, 0, stream>>>(ndr, dr_dsplit, dr_id, dr_part, out);

@@ -4,10 +4,12 @@ alone and mixed with sparse and rank-one coefficients. Bar: 1e-11 relative, the 
 parity tests."""
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from hdsdp_b200 import api, instances
+from hdsdp_b200 import _lib, api, instances
 from oracle import kernels_ref as K
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +56,31 @@ def test_dense_class_primal_dual(gpu_lib):
     _, logdet = api.ratio_probe(inst, y, 0.0, 0.1 * y, 0.0)
     S = K.dual_slack(mats[0], mats[1:], y)
     assert logdet == pytest.approx(np.linalg.slogdet(S)[1], rel=1e-12, abs=1e-11)
+
+
+def test_more_matrices_than_a_grid_has_rows(gpu_lib):
+    """<A_i, X> over 65,537 dense 3 x 3 matrices of one cone."""
+    n, m = 3, 65537
+    rng = np.random.default_rng(4)
+    R = rng.standard_normal((m + 1, n, n))
+    A = (R + R.transpose(0, 2, 1)) / 2.0
+    c, r = np.triu_indices(n)   # column by column of the lower triangle
+    pos = instances.pack_idx(n, r, c)
+    Ap = np.ascontiguousarray(pos.size * np.arange(m + 2), np.int32)
+    Ai = np.ascontiguousarray(np.tile(pos, m + 1), np.int32)
+    Ax = np.ascontiguousarray(A[:, r, c]).ravel()
+    X = R[0] @ R[0].T
+    L, ip = _lib.load(), C.POINTER(C.c_int)
+    user, cone, out = C.c_void_p(), C.c_void_p(), np.zeros(m)
+    assert L.HUserDataCreate(C.byref(user)) == 0
+    L.HUserDataSetConeData(user, 4, m, n, Ap.ctypes.data_as(ip), Ai.ctypes.data_as(ip), api._dp(Ax))
+    assert L.HConeCreate(C.byref(cone)) == 0 and L.HConeSetData(cone, user) == 0
+    try:
+        assert L.HConeProcData(cone) == 0 and L.HConePresolveData(cone) == 0
+        L.HConeComputeATimesX(cone, api._dp(X), api._dp(out))
+    finally:
+        L.HConeDestroy(C.byref(cone))
+        L.HUserDataDestroy(C.byref(user))
+        L.hdsdpb_release_cached_memory()
+    want = np.einsum("kij,ij->k", A[1:], X)
+    assert np.abs(out - want).max() <= 1e-11 * np.abs(want).max()
