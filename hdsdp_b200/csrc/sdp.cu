@@ -34,7 +34,8 @@ T *upload_vec(const std::vector<T> &h, cudaStream_t s) {
 // of rows r and c. Launched on a grid of (row blocks, columns c); rows below c return.
 __device__ __forceinline__ long long r1map_pos(int n, int r, int c) { return (long long) (2LL * n - c - 1) * c / 2 + r; }
 
-// Scratch for the products with the dense coefficient matrices (bytes for each of the two sets).
+// Scratch for the products with the dense coefficient matrices (bytes for each of the two sets, and
+// for one range of the entries of their inner products with the class).
 constexpr size_t kDrScratch = 256u << 20;
 
 // Lists longer than this leave the sliced layout for the warp-per-position one.
@@ -864,7 +865,8 @@ void SdpDevice::upload(int n_, int m_, const HostCoeff &C, const std::vector<Hos
         // as many products at a time as fit kDrScratch; the inner products split along the
         // entries until their 64 x 64 tiles give the SMs two blocks each (at least 128 entries)
         // (and no more than a grid has blocks in y)
-        dr_chunk = (int) std::max<size_t>(1, std::min<size_t>(std::min(ndr, 65535), kDrScratch / (sizeof(double) * mat)));
+        const size_t fit = std::min(kDrScratch / (sizeof(double) * mat), kDrScratch / (sizeof(double) * ndr));
+        dr_chunk = (int) std::max<size_t>(1, std::min<size_t>(std::min(ndr, 65535), fit));
         const long tiles = (long) ((ndr + 63) / 64) * ((dr_chunk + 63) / 64);
         const long want = std::max(1L, 296 / tiles);
         const long entries = ld * n;

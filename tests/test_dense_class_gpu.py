@@ -59,7 +59,11 @@ def test_dense_class_primal_dual(gpu_lib):
 
 
 def test_more_matrices_than_a_grid_has_rows(gpu_lib):
-    """<A_i, X> over 65,537 dense 3 x 3 matrices of one cone."""
+    """<A_i, X> over 65,537 dense 3 x 3 matrices of one cone, whose scratch stays in proportion: below
+    2 GB (a set of 256 MB for each product and each part of their inner products), where every pair of
+    matrices would take 34 GB."""
+    import torch
+
     n, m = 3, 65537
     rng = np.random.default_rng(4)
     R = rng.standard_normal((m + 1, n, n))
@@ -75,9 +79,12 @@ def test_more_matrices_than_a_grid_has_rows(gpu_lib):
     assert L.HUserDataCreate(C.byref(user)) == 0
     L.HUserDataSetConeData(user, 4, m, n, Ap.ctypes.data_as(ip), Ai.ctypes.data_as(ip), api._dp(Ax))
     assert L.HConeCreate(C.byref(cone)) == 0 and L.HConeSetData(cone, user) == 0
+    L.hdsdpb_release_cached_memory()
+    before = torch.cuda.mem_get_info()[0]
     try:
         assert L.HConeProcData(cone) == 0 and L.HConePresolveData(cone) == 0
         L.HConeComputeATimesX(cone, api._dp(X), api._dp(out))
+        assert before - torch.cuda.mem_get_info()[0] < 2 << 30
     finally:
         L.HConeDestroy(C.byref(cone))
         L.HUserDataDestroy(C.byref(user))
