@@ -40,3 +40,9 @@ def test_step_bound(gpu_lib, n, kind):
     step, logdet = api.ratio_probe(inst, y, 0.0, dy, 0.0)
     assert step == pytest.approx(lanczos_step(S, dS), rel=1e-8)
     assert logdet == pytest.approx(np.linalg.slogdet(S)[1], rel=1e-12, abs=1e-11)
+
+
+@pytest.mark.parametrize("n,kind", [(3000, "hub"), (3000, "dense"), (4097, "diag"), (4097, "hub")])
+def test_step_bound_product_by_product(gpu_lib, n, kind):
+    """Where each product is a launch: four warps a column below order 4096, one above."""
+    test_step_bound(gpu_lib, n, kind)
