@@ -1,4 +1,4 @@
-// Persistent cooperative Cholesky factorisation and triangular inverse.
+// Persistent cooperative Cholesky factorisation, and the inverse of the factor alongside.
 //
 // One cooperative launch covers the whole factorisation: for every 64-column panel, block 0
 // factors the diagonal block (and inverts it), all blocks solve the panel rows, then update the
@@ -14,8 +14,8 @@
 // 1000 0.394 / 0.408 -> 0.209 / 0.226, 2000 0.782 / 0.957 -> 0.529 / 0.754 (before: shuffled
 // 16-column sweeps, two grid barriers a panel, five launches a factorisation).
 //
-// The triangular inverse K = L^-1 uses the same structure on block rows:
-// X_i <- Dinv_i X_i, then X_below -= L_below,i X_i.
+// K = L^-1, where it is wanted, is formed by block rows one panel behind: K_i = Dinv_i X_i, then
+// X_below -= L_below,i K_i.
 #include "la.h"
 #include <cooperative_groups.h>
 #include <mutex>

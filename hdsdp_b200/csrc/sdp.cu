@@ -293,7 +293,8 @@ __global__ void r1d_weights_kernel(int k, const int *id, const double *sign, con
 // ---- dense coefficient matrices (class DR): all of them in one launch each --------------
 // These kernels stream the slab of ndr matrices (8 ld n ndr bytes) once. One launch per matrix
 // and per inner product was bound by launches: order 80 with 40 matrices took 7,600 of them and
-// 35.2 ms for two dual-scaling iterations, now about 240 and 3.4 ms.
+// 35.2 ms for two dual-scaling iterations, 3.4 ms with these kernels and 1.5 ms with what the
+// factorisations, bounds and solves around them have gained since.
 
 // S += dA sum_i w[id[i]] A_i, in the order of i; one thread per entry, so the loads of a warp
 // are contiguous in every matrix

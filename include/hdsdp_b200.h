@@ -167,7 +167,8 @@ extern int hdsdpb_cholesky_batch( int count, int n, int mode, const double *S, d
 
 /* Solution of S x = b through the Cholesky factor of S by blocked forward and backward
    substitution with L (the reference's dpotrs use, linalg/hdsdp_linsolver.c:607-633; the
-   solver uses it for Schur systems of order >= 6000). Returns 0 on success, 1 if S is
+   solver uses it for Schur systems of order >= 4096). Above order 3584, where the factor is
+   made recursively, the substitution goes by that recursion's blocks. Returns 0 on success, 1 if S is
    not positive definite, -1 on error. */
 extern int hdsdpb_cholesky_solve( int n, const double *S, const double *b, double *x );
 
@@ -204,8 +205,8 @@ extern int hdsdpb_cholesky_noalloc( int n, const double *S, double *L, double *l
 extern int hdsdpb_inverse( int n, const double *S, double *Sinv );
 
 /* The Cholesky factor L of a symmetric positive definite n x n matrix together with its
-   inverse K = L^-1, as the solver forms them for its Schur matrix below 6000 rows (K in the
-   factorisation's own launch; above order 3840 the recursive blocked form). Column-major
+   inverse K = L^-1, as the solver forms them for its Schur matrix below 4096 rows (K in the
+   factorisation's own launch; above order 2048 the recursive blocked form). Column-major
    host buffers; L and K are written with zeros above the diagonal. Returns 0 on success, 1
    if not positive definite, -1 on error. */
 extern int hdsdpb_cholesky_inverse_factor( int n, const double *S, double *L, double *K );
@@ -229,8 +230,8 @@ extern int hdsdpb_split_gemm( int M, int N, int K, const double *A, int lda, int
    5 Lanczos step bound, 6 rank-64 SYRK update, 7 Cholesky that also forms L^-1,
    8 Cholesky without it, 9 solve with the factor (forward and backward substitution),
    10 as 7 on the one-launch kernel at every order (7 takes the recursive blocked form
-   above order 3840), 11 as 8 on the one-launch kernel at every order (8 takes the
-   recursive form above order 8192). Writes milliseconds per call. */
+   above order 2048), 11 as 8 on the one-launch kernel at every order (8 takes the
+   recursive form above order 3584). Writes milliseconds per call. */
 extern int hdsdpb_kernel_timing( int which, int n, int reps, double *ms );
 
 /* Host only (no device work): the ordering of the sparse factorisation of S for the
